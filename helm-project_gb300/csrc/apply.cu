@@ -22,6 +22,7 @@
 // between neighbouring slices. The tile width and the number of fields per
 // thread iteration are the tuning knobs (see the autotuner in api.cpp).
 #include <algorithm>
+#include <type_traits>
 
 #include "fp32x2.cuh"
 #include "internal.hpp"
@@ -293,7 +294,7 @@ __global__ void __launch_bounds__(256) k_f64(SellArgs a, const double *__restric
 //   k_split_long: rows of more than 32 entries, one warp per (row, F
 //                 fields), lane = leaf of the order in fp32x2.cuh, the F
 //                 fields carried side by side, entries read row-contiguous
-//                 (Sell::lcol/lhi/llo), shuffle butterfly at the end.
+//                 (Sell::lcol/lhi/llo), shuffle tree at the end.
 // Entry k of row p of slice sid sits at base[sid] + 32k + p.
 __device__ __forceinline__ bool row_item(const SellArgs &a, i64 nrhs, i64 &row, int &sid, int &p, i64 &f) {
     const int lane = threadIdx.x & 31;
@@ -358,32 +359,72 @@ struct LongRows {
 };
 constexpr int kLongF = 8;  // fields per warp in the long-row kernels
 constexpr int kLongQ1 = 8;  // entries a lane loads ahead in a single-field long row
+constexpr int kLongQ = 4;   // the same with several fields
 constexpr int kBatchLongF = 4;  // fields per long-row item of the persistent batch kernel (k_batch<true>)
 
-// Warp w: long row w % n, fields [F*(w / n), ...). Lane j sums entries
-// j, j+32, ... of the row for each of the F fields (leaves), then a
-// butterfly over lane offsets 1..16 combines the leaves; lane f stores
-// field f.
+// In-order pairwise tree over the 32 leaves (lane = leaf) for F values a
+// lane, F a power of two up to 32. While a lane holds more than one value,
+// the two lanes of a pair split them: each sends the half it gives up and
+// combines the half it keeps, so the five levels cost F/2 + F/4 + ... + 1
+// combinations (and one more a level once a single value is left) instead of
+// 5 F. combine() is the same in either operand order. Afterwards lane l
+// holds the root of value tree_value<F>(l) in v[0], the lanes that agree in
+// their low log2(F) bits the same one.
+template <int F, class V, class X, class C>
+__device__ __forceinline__ void tree_combine(V (&v)[F], X shfl, C combine) {
+    const int lane = threadIdx.x & 31;
+    int n = F;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        if (n > 1) {
+            n >>= 1;
+            const bool up = (lane & off) != 0;
+#pragma unroll
+            for (int i = 0; i < F / 2; ++i)
+                if (i < n) {
+                    const V keep = up ? v[i + n] : v[i], give = up ? v[i] : v[i + n];
+                    v[i] = combine(keep, shfl(give, off));
+                }
+        } else {
+            v[0] = combine(v[0], shfl(v[0], off));
+        }
+    }
+}
+template <int F>
+__device__ __forceinline__ int tree_value(int lane) {
+    int f = 0;
+#pragma unroll
+    for (int h = F / 2, b = 1; h > 0; h >>= 1, b <<= 1)
+        if (lane & b) f += h;
+    return f;
+}
+
+struct Leaf {
+    float s, c;
+};
+
+// One warp: long row i, fields [F*fc, ...). Lane j sums entries
+// j, j+32, ... of the row for each of the F fields (leaves), two fields at a
+// time in packed arithmetic, then the leaves go through tree_combine.
+// Bound by instruction issue (0.25 deg -> C48, 45 fields, rows of 110 entries
+// on average). Fields the call does not have (f >= nf) are summed as zeros
+// and not stored.
 template <int F = kLongF>
-__device__ __forceinline__ void split_long_row(const LongRows &L, i64 w, const float *x, i64 ldx, float *y,
+__device__ __forceinline__ void split_long_row(const LongRows &L, i64 i, i64 fc, const float *x, i64 ldx, float *y,
                                                i64 ldy, i64 nrhs) {
     const int lane = threadIdx.x & 31;
-    const i64 i = w % L.n, fc = w / L.n;
     const i64 row = L.row[i];
     const int b = L.ptr[i], n = L.ptr[i + 1] - b;
     const i64 f0 = fc * F;
     const int nf = static_cast<int>(nrhs - f0 < F ? nrhs - f0 : F);
-    float s[F], c[F];
-#pragma unroll
-    for (int f = 0; f < F; ++f) {
-        s[f] = 0.f;
-        c[f] = 0.f;
-    }
-    // four of the leaf's entries per step (kLongQ1 for a single field): their
-    // loads are issued together (memory-level parallelism for rows of
-    // hundreds of entries), then summed in order, as one entry per step would
+    x += f0 * ldx;
+    Leaf v[F];
     int k = lane;
-    if (nf == 1) {  // warp-uniform
+    if constexpr (F == 1) {
+        // kLongQ1 of the leaf's entries per step: their loads are issued
+        // together (memory-level parallelism for rows of hundreds of
+        // entries), then summed in order, as one entry per step would
+        v[0] = {0.f, 0.f};
         for (; k + 32 * (kLongQ1 - 1) < n; k += 32 * kLongQ1) {
             int cq[kLongQ1];
             float hq[kLongQ1], lq[kLongQ1], xq[kLongQ1];
@@ -394,69 +435,92 @@ __device__ __forceinline__ void split_long_row(const LongRows &L, i64 w, const f
                 lq[q] = L.lo[b + k + 32 * q];
             }
 #pragma unroll
-            for (int q = 0; q < kLongQ1; ++q) xq[q] = ldg_f(x + f0 * ldx + cq[q]);
+            for (int q = 0; q < kLongQ1; ++q) xq[q] = ldg_f(x + cq[q]);
 #pragma unroll
-            for (int q = 0; q < kLongQ1; ++q) csum1(s[0], c[0], hq[q], lq[q], xq[q]);
+            for (int q = 0; q < kLongQ1; ++q) csum1(v[0].s, v[0].c, hq[q], lq[q], xq[q]);
         }
-    }
-    for (; k + 96 < n; k += 128) {
-        int cq[4];
-        float hq[4], lq[4], xq[4][F];
+        for (; k < n; k += 32) csum1(v[0].s, v[0].c, L.hi[b + k], L.lo[b + k], ldg_f(x + L.col[b + k]));
+    } else {
+        F2 s[F / 2], c[F / 2];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            cq[q] = L.col[b + k + 32 * q];
-            hq[q] = L.hi[b + k + 32 * q];
-            lq[q] = L.lo[b + k + 32 * q];
-        }
+        for (int f = 0; f < F / 2; ++f) s[f] = c[f] = pk(0.f, 0.f);
+        // Q rounds of 32 entries, their loads issued together; only the last
+        // round of a row is partial (its missing entries are steps of weight
+        // 0 on 0, which leave both sums as they are)
+        auto rounds = [&](auto q_tag, bool partial) {
+            constexpr int Q = decltype(q_tag)::value;
+            int cq[Q];
+            float hq[Q], lq[Q], xq[Q][F];
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-            for (int f = 0; f < F; ++f) xq[q][f] = f < nf ? ldg_f(x + (f0 + f) * ldx + cq[q]) : 0.f;
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-            for (int f = 0; f < F; ++f)
-                if (f < nf) csum1(s[f], c[f], hq[q], lq[q], xq[q][f]);
-    }
-    for (; k < n; k += 32) {
-        const int col = L.col[b + k];
-        const float h = L.hi[b + k], l = L.lo[b + k];
-#pragma unroll
-        for (int f = 0; f < F; ++f)
-            if (f < nf) csum1(s[f], c[f], h, l, ldg_f(x + (f0 + f) * ldx + col));
-    }
-#pragma unroll
-    for (int f = 0; f < F; ++f) {
-        if (f < nf) {  // warp-uniform
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const float s2 = __shfl_xor_sync(0xffffffffu, s[f], off);
-                const float c2 = __shfl_xor_sync(0xffffffffu, c[f], off);
-                lcombine(s[f], c[f], s2, c2);
+            for (int q = 0; q < Q; ++q) {
+                const bool on = q < Q - 1 || !partial || k + 32 * q < n;
+                cq[q] = on ? L.col[b + k + 32 * q] : -1;
+                hq[q] = on ? L.hi[b + k + 32 * q] : 0.f;
+                lq[q] = on ? L.lo[b + k + 32 * q] : 0.f;
             }
-            if (lane == f) {
-                const float r = __fadd_rn(s[f], c[f]);
-                y[(f0 + f) * ldy + row] = r;
-                if (L.ylo) L.ylo[(f0 + f) * L.ldylo + row] = sum_err(s[f], c[f], r);
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+#pragma unroll
+                for (int f = 0; f < F; ++f) xq[q][f] = f < nf && cq[q] >= 0 ? ldg_f(x + f * ldx + cq[q]) : 0.f;
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const F2 hp = pk(hq[q], hq[q]), lp = pk(lq[q], lq[q]);
+#pragma unroll
+                for (int f = 0; f < F / 2; ++f) csum2(s[f], c[f], hq[q], hp, lp, xq[q][2 * f], xq[q][2 * f + 1]);
             }
+            k += 32 * Q;
+        };
+        int left = n;  // warp-uniform
+        for (; left >= 32 * kLongQ; left -= 32 * kLongQ) rounds(std::integral_constant<int, kLongQ>{}, false);
+        if (left > 96)
+            rounds(std::integral_constant<int, 4>{}, true);
+        else if (left > 64)
+            rounds(std::integral_constant<int, 3>{}, true);
+        else if (left > 32)
+            rounds(std::integral_constant<int, 2>{}, true);
+        else if (left > 0)
+            rounds(std::integral_constant<int, 1>{}, true);
+#pragma unroll
+        for (int f = 0; f < F / 2; ++f) {
+            upk(s[f], v[2 * f].s, v[2 * f + 1].s);
+            upk(c[f], v[2 * f].c, v[2 * f + 1].c);
         }
+    }
+    __syncwarp();
+    tree_combine<F>(
+        v,
+        [](Leaf a, int off) {
+            return Leaf{__shfl_xor_sync(0xffffffffu, a.s, off), __shfl_xor_sync(0xffffffffu, a.c, off)};
+        },
+        [](Leaf a, Leaf o) {
+            lcombine(a.s, a.c, o.s, o.c);
+            return a;
+        });
+    const int f = tree_value<F>(lane);
+    if (lane < F && f < nf) {
+        const float r = __fadd_rn(v[0].s, v[0].c);
+        y[(f0 + f) * ldy + row] = r;
+        if (L.ylo) L.ylo[(f0 + f) * L.ldylo + row] = sum_err(v[0].s, v[0].c, r);
     }
 }
 
-__global__ void __launch_bounds__(256) k_split_long(LongRows L, const float *__restrict__ x, i64 ldx,
+// Three blocks an SM (80 registers): 128 us for 45 fields of 0.25 deg -> C48,
+// against 170 us at two blocks (92 registers, what the compiler takes by
+// itself), 158 us at four (64), and 140 us at four with two rounds a step.
+// 292 us with every lane combining every field's tree.
+__global__ void __launch_bounds__(256, 3) k_split_long(LongRows L, const float *__restrict__ x, i64 ldx,
                                                     float *__restrict__ y, i64 ldy, i64 nrhs) {
-    const i64 w = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    if (w >= L.n * ((nrhs + kLongF - 1) / kLongF)) return;
-    split_long_row(L, w, x, ldx, y, ldy, nrhs);
+    const i64 i = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    if (i >= L.n) return;
+    for (i64 fc = blockIdx.y; fc * kLongF < nrhs; fc += gridDim.y) split_long_row(L, i, fc, x, ldx, y, ldy, nrhs);
 }
 
 // FP64 form of split_long_row: leaves summed with fma in entry order, then
-// the butterfly with plain additions.
+// tree_combine with plain additions.
 template <int F = kLongF>
-__device__ __forceinline__ void f64_long_row(const LongRows &L, i64 w, const double *x, i64 ldx, double *y,
+__device__ __forceinline__ void f64_long_row(const LongRows &L, i64 i, i64 fc, const double *x, i64 ldx, double *y,
                                              i64 ldy, i64 nrhs) {
     const int lane = threadIdx.x & 31;
-    const i64 i = w % L.n, fc = w / L.n;
     const i64 row = L.row[i];
     const int b = L.ptr[i], n = L.ptr[i + 1] - b;
     const i64 f0 = fc * F;
@@ -465,7 +529,7 @@ __device__ __forceinline__ void f64_long_row(const LongRows &L, i64 w, const dou
 #pragma unroll
     for (int f = 0; f < F; ++f) s[f] = 0.0;
     int k = lane;
-    if (nf == 1) {  // kLongQ1 entries' loads in flight for a single field, as split_long_row
+    if constexpr (F == 1) {  // kLongQ1 entries' loads in flight for a single field, as split_long_row
         for (; k + 32 * (kLongQ1 - 1) < n; k += 32 * kLongQ1) {
             int cq[kLongQ1];
             double wq[kLongQ1], xq[kLongQ1];
@@ -480,7 +544,7 @@ __device__ __forceinline__ void f64_long_row(const LongRows &L, i64 w, const dou
             for (int q = 0; q < kLongQ1; ++q) s[0] = fma(wq[q], xq[q], s[0]);
         }
     }
-    for (; k + 96 < n; k += 128) {  // four entries' loads in flight, summed in order
+    for (; F > 1 && k + 96 < n; k += 128) {  // four entries' loads in flight, summed in order
         int cq[4];
         double wq[4], xq[4][F];
 #pragma unroll
@@ -505,21 +569,19 @@ __device__ __forceinline__ void f64_long_row(const LongRows &L, i64 w, const dou
         for (int f = 0; f < F; ++f)
             if (f < nf) s[f] = fma(wv, __ldg(x + (f0 + f) * ldx + col), s[f]);
     }
-#pragma unroll
-    for (int f = 0; f < F; ++f) {
-        if (f < nf) {
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) s[f] = s[f] + __shfl_xor_sync(0xffffffffu, s[f], off);
-            if (lane == f) y[(f0 + f) * ldy + row] = s[f];
-        }
-    }
+    __syncwarp();
+    tree_combine<F>(
+        s, [](double a, int off) { return __shfl_xor_sync(0xffffffffu, a, off); },
+        [](double a, double o) { return a + o; });
+    const int f = tree_value<F>(lane);
+    if (lane < F && f < nf) y[(f0 + f) * ldy + row] = s[0];
 }
 
 __global__ void __launch_bounds__(256) k_f64_long(LongRows L, const double *__restrict__ x, i64 ldx,
                                                   double *__restrict__ y, i64 ldy, i64 nrhs) {
-    const i64 w = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    if (w >= L.n * ((nrhs + kLongF - 1) / kLongF)) return;
-    f64_long_row(L, w, x, ldx, y, ldy, nrhs);
+    const i64 i = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    if (i >= L.n) return;
+    for (i64 fc = blockIdx.y; fc * kLongF < nrhs; fc += gridDim.y) f64_long_row(L, i, fc, x, ldx, y, ldy, nrhs);
 }
 
 // ─── few fields: one launch over the whole matrix ────────────────────────
@@ -541,7 +603,7 @@ __global__ void __launch_bounds__(256, F <= 2 ? 4 : 2) k_split_fused(SellArgs a,
     // dependent loads, and starting them with the first wave overlaps them
     // with the short rows instead of leaving them as the tail
     if (wg < L.n) {
-        for (i64 fc = 0; fc * F < nrhs; ++fc) split_long_row<F>(L, fc * L.n + wg, x, ldx, y, ldy, nrhs);
+        for (i64 fc = 0; fc * F < nrhs; ++fc) split_long_row<F>(L, wg, fc, x, ldx, y, ldy, nrhs);
         return;
     }
     const i64 w = wg - L.n;
@@ -589,7 +651,7 @@ __global__ void __launch_bounds__(256, F <= 2 ? 4 : 2) k_f64_fused(SellArgs a, L
     const int lane = threadIdx.x & 31;
     const i64 wg = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     if (wg < L.n) {  // long rows first, as k_split_fused
-        for (i64 fc = 0; fc * F < nrhs; ++fc) f64_long_row<F>(L, fc * L.n + wg, x, ldx, y, ldy, nrhs);
+        for (i64 fc = 0; fc * F < nrhs; ++fc) f64_long_row<F>(L, wg, fc, x, ldx, y, ldy, nrhs);
         return;
     }
     const i64 w = wg - L.n;
@@ -832,6 +894,13 @@ LongRows long_rows(const Sell &S) {
     return L;
 }
 
+// Grid of the long-row kernels: a warp per row along x, chunks of kLongF
+// fields along y (all rows of one chunk of fields are in flight together, so
+// the chunk's source values stay in L2).
+dim3 long_grid(i64 rows, i64 nrhs) {
+    return dim3(nblk(rows * 32, 256), static_cast<unsigned>(std::min<i64>(65535, (nrhs + kLongF - 1) / kLongF)));
+}
+
 // Slices of the long classes: their short rows (k_*_rows), then every row
 // of more than 32 entries (k_*_long).
 void launch_split_rows(const SellArgs &a, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, cudaStream_t s) {
@@ -842,11 +911,10 @@ void launch_split_rows(const SellArgs &a, const float *x, i64 ldx, float *y, i64
 void launch_split_long(const Sell &S, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, cudaStream_t s,
                        float *ylo = nullptr, i64 ldylo = 0) {
     if (S.n_lrows == 0 || nrhs == 0) return;
-    const i64 warps = S.n_lrows * ((nrhs + kLongF - 1) / kLongF);
     LongRows L = long_rows(S);
     L.ylo = ylo;
     L.ldylo = ldylo;
-    k_split_long<<<nblk(warps * 32, 256), 256, 0, s>>>(L, x, ldx, y, ldy, nrhs);
+    k_split_long<<<long_grid(L.n, nrhs), 256, 0, s>>>(L, x, ldx, y, ldy, nrhs);
 }
 void launch_f64_rows(const SellArgs &a, const double *x, i64 ldx, double *y, i64 ldy, i64 nrhs, cudaStream_t s) {
     if (a.n_ids == 0 || nrhs == 0) return;
@@ -855,8 +923,7 @@ void launch_f64_rows(const SellArgs &a, const double *x, i64 ldx, double *y, i64
 }
 void launch_f64_long(const Sell &S, const double *x, i64 ldx, double *y, i64 ldy, i64 nrhs, cudaStream_t s) {
     if (S.n_lrows == 0 || nrhs == 0) return;
-    const i64 warps = S.n_lrows * ((nrhs + kLongF - 1) / kLongF);
-    k_f64_long<<<nblk(warps * 32, 256), 256, 0, s>>>(long_rows(S), x, ldx, y, ldy, nrhs);
+    k_f64_long<<<long_grid(S.n_lrows, nrhs), 256, 0, s>>>(long_rows(S), x, ldx, y, ldy, nrhs);
 }
 }  // namespace
 
@@ -874,8 +941,7 @@ void launch_long_rows(const int *row, const int *ptr, const int *col, const floa
     L.n = n;
     L.ylo = ylo;
     L.ldylo = ldylo;
-    const i64 warps = n * ((nrhs + kLongF - 1) / kLongF);
-    k_split_long<<<nblk(warps * 32, 256), 256, 0, s>>>(L, x, ldx, y, ldy, nrhs);
+    k_split_long<<<long_grid(n, nrhs), 256, 0, s>>>(L, x, ldx, y, ldy, nrhs);
 }
 
 namespace {
@@ -1222,7 +1288,7 @@ __global__ void __launch_bounds__(256, ROWS ? 4 : 2) k_batch(const Batch::Desc *
             L.lo = d.llo;
             L.w64 = nullptr;
             L.n = d.n_ids;
-            split_long_row<kBatchLongF>(L, local, d.x, d.ldx, d.y, d.ldy, d.nrhs);
+            split_long_row<kBatchLongF>(L, local % L.n, local / L.n, d.x, d.ldx, d.y, d.ldy, d.nrhs);
             continue;
         }
         if (d.mode == 1) {  // short rows of long-class slices: lane = field

@@ -1,0 +1,99 @@
+"""Applies on row lengths, field counts and alignments at the edges of the
+kernels' tiles, on matrices built from given rows. Every split kernel has to
+give the same bits, and each result is checked against the oracle's
+compensated FP64 sums.
+
+Tolerances: a split output is the compensated sum rounded once to FP32, so it
+is within half an ulp (2^-24 of its value) plus the sum's own error, at most
+n 2^-46 <= 1e-10 of the row's condition sum |w x| for the rows used here; an
+FP64 output carries n rounding errors of 2^-53 of the condition (n <= 4300:
+5e-13, 1e-12 allowed)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows_matrix(gpu, lens, n_src, seed):
+    """Rows of the given lengths: ascending columns in runs with gaps, as the
+    rows of a finer source have, weights uniform in (0, 1] over the length."""
+    rng = np.random.default_rng(seed)
+    rp = np.concatenate([[0], np.cumsum(lens)])
+    col = np.empty(rp[-1], np.int64)
+    for r, n in enumerate(lens):
+        span = min(n_src, n + n // 3 + 2)
+        start = rng.integers(0, n_src - span + 1)
+        col[rp[r]:rp[r + 1]] = start + np.sort(rng.choice(span, n, replace=False))
+    val = rng.uniform(1e-3, 1.0, rp[-1]) / np.maximum(1, np.repeat(lens, lens))
+    return gpu.Matrix.from_csr(n_src, len(lens), rp, col, val)
+
+
+def _reference(M, oracle, X):
+    """Compensated FP64 sums and the condition of every output."""
+    from oracle import Weights
+    c = M.to_csr()
+    row = np.repeat(np.arange(M.n_dst), np.diff(c["row_ptr"])).astype(np.int64)
+    w = Weights(M.n_src, M.n_dst, row, c["col"].astype(np.int64), c["val"], c["frac_a"], c["frac_b"], c["area_a"],
+                c["area_b"])
+    x = X.astype(np.float64)
+    return oracle.apply_csr(w, x, compensated=True), oracle.apply_csr(w, np.abs(x), compensated=True)
+
+
+def _check_split(y, ref, cond):
+    assert np.all(np.abs(y.astype(np.float64) - ref) <= 1.0001 * 2.0**-24 * np.abs(ref) + 1e-10 * cond)
+
+
+def _check_f64(y, ref, cond):
+    assert np.all(np.abs(y - ref) <= 1e-12 * cond)
+
+
+LONG = [33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 159, 160, 161, 192, 255, 256, 257, 1000]
+SHORT = [0, 1, 2, 3, 4, 5, 7, 8, 9, 12, 13, 16, 17, 31, 32]
+
+
+def _mixed_lens(seed):
+    rng = np.random.default_rng(seed)
+    mixed = np.array((LONG + SHORT) * 12)
+    rng.shuffle(mixed)
+    # whole slices of long rows, an empty slice, short slices, and a ragged end
+    return np.concatenate([mixed, [40] * 160, [0] * 64, rng.choice(SHORT, 300), [70] * 3, [3] * 2]).astype(np.int64)
+
+
+@pytest.mark.parametrize("nf", [1, 2, 3, 4, 5, 7, 8, 9, 17, 33])
+def test_mixed_row_lengths(gpu, oracle, nf):
+    """Rows longer than 32 entries among short ones: the long rows' tree for
+    every count of fields a warp carries, blocks staged without their long
+    rows, and blocks of nothing else."""
+    import torch
+    M = _rows_matrix(gpu, _mixed_lens(1), 4000, 2)
+    X = np.random.default_rng(3).standard_normal((nf, M.n_src)).astype(np.float32)
+    ref, cond = _reference(M, oracle, X)
+    xs = torch.tensor(X, device="cuda")
+    y = gpu.apply_f32split(M, xs).cpu().numpy()
+    _check_split(y, ref, cond)
+    forms = [(0, 0, 1), (0, 0, 4), (1, 0, 4), (1, 8, 8), (2, 0, 4), (3, 0, 4), (3, 8, 4), (4, 0, 1), (5, 0, 32)]
+    for v, fpp, u in forms:
+        assert np.array_equal(gpu.apply_f32split(M, xs, fields_per_pass=fpp, unroll=u, variant=v).cpu().numpy(), y), v
+    assert M.device_status() == 0
+    for f in {0, nf - 1}:
+        assert np.array_equal(gpu.apply_f32split(M, xs[f:f + 1]).cpu().numpy()[0], y[f])
+    B = gpu.Batch([M, M], [nf, 1])
+    ys = [torch.empty((n, M.n_dst), dtype=torch.float32, device="cuda") for n in (nf, 1)]
+    B.apply([xs, xs[nf - 1:]], ys)
+    assert np.array_equal(ys[0].cpu().numpy(), y) and np.array_equal(ys[1].cpu().numpy()[0], y[nf - 1])
+    d = gpu.apply_f64(M, xs.double()).cpu().numpy()
+    _check_f64(d, ref, cond)
+    assert np.array_equal(gpu.apply_f64(M, xs[:1].double()).cpu().numpy()[0], d[0])
+
+
+@pytest.mark.parametrize("nf,rows", [(8, 31), (40, 129), (129, 1000), (500, 260), (200, 5000)])
+def test_fields_per_work_item(gpu, oracle, nf, rows):
+    """The default split of the fields over work items, which depends on the
+    matrix's size, against one work item for all fields."""
+    import torch
+    M = _rows_matrix(gpu, np.random.default_rng(4).choice(SHORT, rows), 900, 5)
+    X = np.random.default_rng(6).standard_normal((nf, M.n_src)).astype(np.float32)
+    xs = torch.tensor(X, device="cuda")
+    y = gpu.apply_f32split(M, xs).cpu().numpy()
+    assert np.array_equal(gpu.apply_f32split(M, xs, fields_per_pass=0, unroll=4, variant=3).cpu().numpy(), y)
+    _check_split(y, *_reference(M, oracle, X))

@@ -7,6 +7,10 @@
 //     generate_weights), slices are visited in 3-D Morton order and each
 //     block takes the 3 nearest unused slices among the next ones in that
 //     order; without a hint, 4 consecutive slices;
+//   * rows of more than 32 entries are left out (a warp each, k_split_long);
+//     the block keeps its other rows. (Leaving out a whole block with a long
+//     row sent C384 -> 1 deg, rows of 24 entries and up to 43, to the lane =
+//     field gathers of k_split_rows: a 32-byte sector for every 4-byte value.)
 //   * inside a block the rows are sorted by entry count (longest first), so
 //     warp w holds rows of similar length and loops only to its own maximum;
 //   * the block's distinct source columns are rounded out to 16-byte chunks;
@@ -703,9 +707,8 @@ struct HostBlock {
 // Padding reads the zero run (up to kZeroRun zero floats after the chunks,
 // one a bank). A padding step of a row is exact (weight 0 on a +0 value
 // leaves both sums unchanged), so every split-FP32 layout computes the same
-// bits from perm. Blocks the staged kernels do not take (rows longer than
-// kMaxL, or more staging than kMaxUS) keep each row's CSR order (schedule =
-// false).
+// bits from perm. Blocks the staged kernels do not take (more staging than
+// kMaxUS) keep each row's CSR order (schedule = false).
 void order_entries(const HostBlock &H, const std::vector<int> &rp, const std::vector<int> &col,
                    const std::vector<int> &cols, std::vector<int> &perm, std::vector<int> &q_out,
                    std::vector<int> &e_out, WarpSchedule &S, bool schedule) {
@@ -824,8 +827,12 @@ void build_blocked(Matrix &m, cudaStream_t s) {
             rl.clear();
             for (int g : groups[b])
                 if (g >= 0)
-                    for (i64 r = static_cast<i64>(g) * 32; r < std::min<i64>(n, static_cast<i64>(g) * 32 + 32); ++r)
-                        rl.push_back({-(rp[r + 1] - rp[r]), static_cast<int>(r)});
+                    for (i64 r = static_cast<i64>(g) * 32; r < std::min<i64>(n, static_cast<i64>(g) * 32 + 32); ++r) {
+                        if (rp[r + 1] - rp[r] <= kMaxL)
+                            rl.push_back({-(rp[r + 1] - rp[r]), static_cast<int>(r)});
+                        else  // a long row: not staged, entries in CSR order
+                            for (int k = rp[r]; k < rp[r + 1]; ++k) perm[k] = k;
+                    }
             std::stable_sort(rl.begin(), rl.end());
             for (int t = 0; t < kRows; ++t) H.rows[t] = t < static_cast<int>(rl.size()) ? rl[t].second : -1;
             cols.clear();
@@ -862,7 +869,7 @@ void build_blocked(Matrix &m, cudaStream_t s) {
                 maxlen = std::max(maxlen, mx);
             }
             H.L = std::max(4, (maxlen + 3) / 4 * 4);
-            H.staged = maxlen <= kMaxL && H.us <= kMaxUS;
+            H.staged = H.us <= kMaxUS;
             order_entries(H, rp, col, cols, perm, sq, se, scratch, H.staged);
             if (!H.staged)  // no entries stored: the direct kernels take these slices
                 for (int w = 0; w < kWarps; ++w) H.wlen[w] = 0;
@@ -905,6 +912,7 @@ void build_blocked(Matrix &m, cudaStream_t s) {
         lidx.insert(lidx.end(), H.lidx.begin(), H.lidx.end());
         hi.insert(hi.end(), H.hi.begin(), H.hi.end());
         lo.insert(lo.end(), H.lo.begin(), H.lo.end());
+        if (H.rows[0] < 0) continue;  // long rows only
         if (H.staged) {
             int ub = 0;
             while (kUsBuckets[ub] < H.us) ++ub;

@@ -365,15 +365,24 @@ void host_batch(Matrix &m, const T *src, T *dst, int64_t n_vars, F apply_fn) {
     AXGB_CUDA(cudaStreamSynchronize(st.d2h));
 }
 
-SplitParams default_split_params(i64 nrhs);
+SplitParams default_split_params(const Matrix &m, i64 nrhs);
 SplitParams pick_params(Matrix &m, i64 nrhs) {
     std::lock_guard<std::mutex> lk(m.mu);
     auto it = m.tuned.find(nrhs);
     if (it != m.tuned.end()) return it->second;
-    return default_split_params(nrhs);
+    return default_split_params(m, nrhs);
 }
 
-SplitParams default_split_params(i64 nrhs) {
+// Fields per work item of the staged kernels: 128 where that leaves about
+// two waves of work items (a block of 128 rows and the item's fields; four to
+// six CTAs fit an SM), fewer on smaller matrices, down to four tiles of four.
+int default_item_fields(const Matrix &m, i64 nrhs) {
+    const i64 blocks = std::max<i64>(1, (m.n_dst + 127) / 128), items = 152 * 6 * 2;
+    const i64 f = (blocks * nrhs / items + 3) / 4 * 4;
+    return static_cast<int>(std::min<i64>(128, std::max<i64>(16, f)));
+}
+
+SplitParams default_split_params(const Matrix &m, i64 nrhs) {
     SplitParams p;
     if (nrhs <= 2) {  // one fused launch
         p.variant = 4;
@@ -384,7 +393,7 @@ SplitParams default_split_params(i64 nrhs) {
     }
     if (nrhs >= 8) {  // producer-warp staged kernel, ring depth per row-length class
         p.variant = 3;
-        p.fields_per_pass = 128;
+        p.fields_per_pass = default_item_fields(m, nrhs);
         p.stages = 0;
         p.unroll = 4;
         return p;
@@ -1008,7 +1017,7 @@ int axgb_get_kernel_choice(int h, int64_t nrhs, int32_t *choice, int32_t *cached
     AXGB_TRY({
         auto m = Registry::get().find(Registry::get().mats, h, "matrix");
         AXGB_REQUIRE(choice && nrhs > 0, "get_kernel_choice: NULL choice or nrhs <= 0");
-        SplitParams p = default_split_params(nrhs);
+        SplitParams p = default_split_params(*m, nrhs);
         int32_t c = 0;
         {
             std::lock_guard<std::mutex> lk(m->mu);
@@ -1049,7 +1058,7 @@ int axgb_apply_f32split(int h, const float *x, int64_t ldx, float *y, int64_t ld
                 m->tuned[nrhs] = p;
                 have = true;
             }
-            if (!have) p = default_split_params(nrhs);
+            if (!have) p = default_split_params(*m, nrhs);
             apply_split(*m, x, ldx, y, ldy, nrhs, p, s);
         }
     });

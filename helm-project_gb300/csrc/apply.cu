@@ -225,66 +225,6 @@ __global__ void __launch_bounds__(256) k_split(SellArgs a, const float *__restri
     }
 }
 
-// ─── FP64 kernel ───────────────────────────────────────────────────────────
-// Lane per row, slices of rows with at most L <= 32 entries (longer rows:
-// k_f64_rows); s = fma(w, x, s) in entry order.
-template <int L, int U>
-__global__ void __launch_bounds__(256) k_f64(SellArgs a, const double *__restrict__ x, i64 ldx, double *__restrict__ y,
-                                             i64 ldy, i64 nrhs, i64 tile) {
-    const int lane = threadIdx.x & 31;
-    const i64 item = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const i64 n_tiles = (nrhs + tile - 1) / tile;
-    if (item >= n_tiles * a.n_ids) return;
-    const i64 t = item / a.n_ids;
-    const int sid = a.ids[item - t * a.n_ids];
-    const i64 row = static_cast<i64>(sid) * 32 + lane;
-    const int base = a.base[sid];
-    const int rl = a.rlen[static_cast<i64>(sid) * 32 + lane];
-    const i64 f0 = t * tile, f1 = min(f0 + tile, nrhs);
-    const bool store = row < a.n_rows;
-    static_assert(L > 0 && L <= 32, "lane-per-row kernels cache at most 32 entries");
-    {
-        int c[L];
-        double w[L];
-#pragma unroll
-        for (int k = 0; k < L; ++k) {
-            if (k < rl) {
-                int e = base + k * 32 + lane;
-                c[k] = a.col[e];
-                w[k] = a.w64[e];
-            } else {
-                c[k] = 0;
-                w[k] = 0.0;
-            }
-        }
-        i64 f = f0;
-        for (; f + U <= f1; f += U) {
-            double s[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) s[u] = 0.0;
-            const double *xf = x + f * ldx;
-#pragma unroll
-            for (int k = 0; k < L; ++k)
-                if (k < rl) {
-#pragma unroll
-                    for (int u = 0; u < U; ++u) s[u] = fma(w[k], __ldg(xf + u * ldx + c[k]), s[u]);
-                }
-            if (store) {
-#pragma unroll
-                for (int u = 0; u < U; ++u) y[(f + u) * ldy + row] = s[u];
-            }
-        }
-        for (; f < f1; ++f) {
-            double s = 0.0;
-            const double *xf = x + f * ldx;
-#pragma unroll
-            for (int k = 0; k < L; ++k)
-                if (k < rl) s = fma(w[k], __ldg(xf + c[k]), s);
-            if (store) y[f * ldy + row] = s;
-        }
-    }
-}
-
 // ─── long rows ─────────────────────────────────────────────────────────────
 // Slices in the long classes (some row has more than 32 entries; coarse
 // destination cells over a fine source, e.g. polar cells over a lat-lon
@@ -329,25 +269,9 @@ __global__ void __launch_bounds__(256) k_split_rows(SellArgs a, const float *__r
     if (a.ylo) a.ylo[f * a.ldylo + row] = sum_err(s, c, r);
 }
 
-__global__ void __launch_bounds__(256) k_f64_rows(SellArgs a, const double *__restrict__ x, i64 ldx,
-                                                  double *__restrict__ y, i64 ldy, i64 nrhs) {
-    i64 row, f;
-    int sid, p;
-    if (!row_item(a, nrhs, row, sid, p, f)) return;
-    const int n = a.rlen[row];
-    if (n > 32) return;  // k_f64_long
-    const int e0 = a.base[sid] + p;
-    const double *xf = x + f * ldx;
-    double s = 0.0;
-    for (int k = 0; k < n; ++k) {
-        const int e = e0 + 32 * k;
-        s = fma(a.w64[e], __ldg(xf + a.col[e]), s);
-    }
-    y[f * ldy + row] = s;
-}
-
-constexpr i64 kFusedMaxF64 = 2;  // FP64 applies of at most this many fields take the fused kernel
+constexpr int kF64F = 4;          // fields an FP64 row carries side by side
 constexpr int kFusedK = 4;        // entries a row of the fused kernels loads before gathering
+constexpr int kF64K = 2;          // the same of the FP64 kernel from three fields up
 
 struct LongRows {
     const int *row, *ptr, *col;
@@ -525,63 +449,54 @@ __device__ __forceinline__ void f64_long_row(const LongRows &L, i64 i, i64 fc, c
     const int b = L.ptr[i], n = L.ptr[i + 1] - b;
     const i64 f0 = fc * F;
     const int nf = static_cast<int>(nrhs - f0 < F ? nrhs - f0 : F);
+    x += f0 * ldx;
     double s[F];
 #pragma unroll
     for (int f = 0; f < F; ++f) s[f] = 0.0;
     int k = lane;
-    if constexpr (F == 1) {  // kLongQ1 entries' loads in flight for a single field, as split_long_row
-        for (; k + 32 * (kLongQ1 - 1) < n; k += 32 * kLongQ1) {
-            int cq[kLongQ1];
-            double wq[kLongQ1], xq[kLongQ1];
+    // Q rounds, as split_long_row (a missing entry is an FMA of 0 and 0)
+    auto rounds = [&](auto q_tag, bool partial) {
+        constexpr int Q = decltype(q_tag)::value;
+        int cq[Q];
+        double wq[Q], xq[Q][F];
 #pragma unroll
-            for (int q = 0; q < kLongQ1; ++q) {
-                cq[q] = L.col[b + k + 32 * q];
-                wq[q] = L.w64[b + k + 32 * q];
-            }
-#pragma unroll
-            for (int q = 0; q < kLongQ1; ++q) xq[q] = __ldg(x + f0 * ldx + cq[q]);
-#pragma unroll
-            for (int q = 0; q < kLongQ1; ++q) s[0] = fma(wq[q], xq[q], s[0]);
-        }
-    }
-    for (; F > 1 && k + 96 < n; k += 128) {  // four entries' loads in flight, summed in order
-        int cq[4];
-        double wq[4], xq[4][F];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            cq[q] = L.col[b + k + 32 * q];
-            wq[q] = L.w64[b + k + 32 * q];
+        for (int q = 0; q < Q; ++q) {
+            const bool on = q < Q - 1 || !partial || k + 32 * q < n;
+            cq[q] = on ? L.col[b + k + 32 * q] : -1;
+            wq[q] = on ? L.w64[b + k + 32 * q] : 0.0;
         }
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int q = 0; q < Q; ++q)
 #pragma unroll
-            for (int f = 0; f < F; ++f) xq[q][f] = f < nf ? __ldg(x + (f0 + f) * ldx + cq[q]) : 0.0;
+            for (int f = 0; f < F; ++f) xq[q][f] = f < nf && cq[q] >= 0 ? __ldg(x + f * ldx + cq[q]) : 0.0;
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int q = 0; q < Q; ++q)
 #pragma unroll
             for (int f = 0; f < F; ++f)
                 if (f < nf) s[f] = fma(wq[q], xq[q][f], s[f]);
+        k += 32 * Q;
+    };
+    constexpr int kQ = F == 1 ? kLongQ1 : kLongQ;
+    int left = n;  // warp-uniform
+    for (; left >= 32 * kQ; left -= 32 * kQ) rounds(std::integral_constant<int, kQ>{}, false);
+    if (kQ > 4 && left >= 128) {
+        rounds(std::integral_constant<int, 4>{}, false);
+        left -= 128;
     }
-    for (; k < n; k += 32) {
-        const int col = L.col[b + k];
-        const double wv = L.w64[b + k];
-#pragma unroll
-        for (int f = 0; f < F; ++f)
-            if (f < nf) s[f] = fma(wv, __ldg(x + (f0 + f) * ldx + col), s[f]);
-    }
+    if (left > 96)
+        rounds(std::integral_constant<int, 4>{}, true);
+    else if (left > 64)
+        rounds(std::integral_constant<int, 3>{}, true);
+    else if (left > 32)
+        rounds(std::integral_constant<int, 2>{}, true);
+    else if (left > 0)
+        rounds(std::integral_constant<int, 1>{}, true);
     __syncwarp();
     tree_combine<F>(
         s, [](double a, int off) { return __shfl_xor_sync(0xffffffffu, a, off); },
         [](double a, double o) { return a + o; });
     const int f = tree_value<F>(lane);
     if (lane < F && f < nf) y[(f0 + f) * ldy + row] = s[0];
-}
-
-__global__ void __launch_bounds__(256) k_f64_long(LongRows L, const double *__restrict__ x, i64 ldx,
-                                                  double *__restrict__ y, i64 ldy, i64 nrhs) {
-    const i64 i = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    if (i >= L.n) return;
-    for (i64 fc = blockIdx.y; fc * kLongF < nrhs; fc += gridDim.y) f64_long_row(L, i, fc, x, ldx, y, ldy, nrhs);
 }
 
 // ─── few fields: one launch over the whole matrix ────────────────────────
@@ -644,45 +559,71 @@ __global__ void __launch_bounds__(256, F <= 2 ? 4 : 2) k_split_fused(SellArgs a,
     }
 }
 
+// FP64 apply in one launch. Warps [0, L.n * ceil(nrhs / F)): a long row and F
+// fields; the others: lane per row (rows of at most 32 entries, in the order
+// of Sell::ord from three fields up) and a tile of fields, F side by side,
+// kFusedK entries at a time (their loads, then their gathers, then the FMAs
+// in entry order). The entries are read again for the next F fields (from
+// L1), so rows of every length run in one launch without a register array
+// for the longest. The bound is the FP64 pipe (half a lane an SM
+// sub-partition and cycle). 64 fields of C192 -> 0.5 deg: 169 us, against
+// 297 us for one launch per length class with the entries in registers, the
+// last launches on a few blocks (three blocks an SM and four entries ahead:
+// 210 us; eight fields side by side: 223).
 template <int F>
-__global__ void __launch_bounds__(256, F <= 2 ? 4 : 2) k_f64_fused(SellArgs a, LongRows L, i64 n_slices,
-                                                                 const double *__restrict__ x, i64 ldx,
-                                                                 double *__restrict__ y, i64 ldy, i64 nrhs) {
+__global__ void __launch_bounds__(256, 4) k_f64_fused(SellArgs a, LongRows L, const int *__restrict__ ord,
+                                                                 i64 n_slices, const double *__restrict__ x, i64 ldx,
+                                                                 double *__restrict__ y, i64 ldy, i64 nrhs, i64 tile) {
     const int lane = threadIdx.x & 31;
-    const i64 wg = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    if (wg < L.n) {  // long rows first, as k_split_fused
-        for (i64 fc = 0; fc * F < nrhs; ++fc) f64_long_row<F>(L, wg, fc, x, ldx, y, ldy, nrhs);
+    i64 w = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    // the long rows' warps come first in the grid, as in k_split_fused
+    const i64 n_long = L.n * ((nrhs + F - 1) / F);
+    if (w < n_long) {
+        f64_long_row<F>(L, w % L.n, w / L.n, x, ldx, y, ldy, nrhs);
         return;
     }
-    const i64 w = wg - L.n;
-    if (w < n_slices) {
-        const i64 row = w * 32 + lane;
-        if (row >= a.n_rows) return;
-        const int n = a.rlen[row];
-        if (n > 32) return;
-        const int e0 = a.base[w] + lane;
-        for (i64 f = 0; f < nrhs; ++f) {
-            const double *xf = x + f * ldx;
-            double s = 0.0;
-            for (int k0 = 0; k0 < n; k0 += kFusedK) {  // as k_split_fused
-                int cl[kFusedK];
-                double wv[kFusedK], xv[kFusedK];
+    w -= n_long;
+    const i64 t = w / n_slices, pos = (w - t * n_slices) * 32 + lane;
+    const i64 fa = t * tile, fb = min(fa + tile, nrhs);
+    if (fa >= nrhs) return;
+    const i64 row = F > 2 ? ord[pos] : pos;
+    if (row >= a.n_rows) return;
+    const int n = a.rlen[row];
+    if (n > 32) return;
+    constexpr int K = F <= 2 ? kFusedK : kF64K;
+    const int e0 = a.base[row >> 5] + static_cast<int>(row & 31);
+    for (i64 f = fa; f < fb; f += F) {
+        const int nf = static_cast<int>(min(static_cast<i64>(F), fb - f));
+        const double *xf = x + f * ldx;
+        double s[F];
 #pragma unroll
-                for (int j = 0; j < kFusedK; ++j)
-                    if (k0 + j < n) {
-                        const int e = e0 + 32 * (k0 + j);
-                        cl[j] = a.col[e];
-                        wv[j] = a.w64[e];
-                    }
+        for (int u = 0; u < F; ++u) s[u] = 0.0;
+        for (int k0 = 0; k0 < n; k0 += K) {
+            int cl[K];
+            double wv[K], xv[K][F];
 #pragma unroll
-                for (int j = 0; j < kFusedK; ++j)
-                    if (k0 + j < n) xv[j] = __ldg(xf + cl[j]);
+            for (int j = 0; j < K; ++j)
+                if (k0 + j < n) {
+                    const int e = e0 + 32 * (k0 + j);
+                    cl[j] = a.col[e];
+                    wv[j] = a.w64[e];
+                }
 #pragma unroll
-                for (int j = 0; j < kFusedK; ++j)
-                    if (k0 + j < n) s = fma(wv[j], xv[j], s);
-            }
-            y[f * ldy + row] = s;
+            for (int j = 0; j < K; ++j)
+#pragma unroll
+                for (int u = 0; u < F; ++u)
+                    if (k0 + j < n && u < nf) xv[j][u] = __ldg(xf + u * ldx + cl[j]);
+#pragma unroll
+            for (int j = 0; j < K; ++j)
+                if (k0 + j < n) {
+#pragma unroll
+                    for (int u = 0; u < F; ++u)
+                        if (u < nf) s[u] = fma(wv[j], xv[j][u], s[u]);
+                }
         }
+#pragma unroll
+        for (int u = 0; u < F; ++u)
+            if (u < nf) y[(f + u) * ldy + row] = s[u];
     }
 }
 
@@ -758,6 +699,31 @@ __global__ void k_sell_fill(const int *rp, const int *ccol, const double *val, c
     }
 }
 
+// Rows of every 128 consecutive ones, longest first, rows of more than 32
+// entries (which have their own kernels) as if empty; positions past n_rows
+// keep themselves. The FP64 kernels take a lane's row from here: a warp's
+// FP64 instructions cost the same with any number of lanes active, and
+// consecutive rows differ enough in length (C192 -> 0.5 deg: 3 to 9 entries)
+// to leave a quarter of the lanes idle. Groups of 128 measured best or within
+// 1% of 256 (16 NaN fields of 0.25 deg -> C384 651 / 646 us, 20 FP64 fields of
+// C384 -> 1 deg 121 / 125, 300 of C384 -> 0.25 deg 2836 / 2867); 64 is slower
+// on the first (665).
+std::vector<int> rows_by_length(const std::vector<int> &rp, i64 n_rows, i64 n_pos) {
+    std::vector<int> ord(n_pos);
+    for (i64 g = 0; g < n_pos; g += 128) {
+        const i64 e = std::min<i64>(n_pos, g + 128);
+        auto len = [&](i64 r) {
+            const int n = r < n_rows ? rp[r + 1] - rp[r] : 0;
+            return n > 32 ? 0 : n;
+        };
+        int at[34] = {};  // at[32 - n + 1]: rows of length n, then their first position
+        for (i64 r = g; r < e; ++r) ++at[33 - len(r)];
+        for (int k = 1; k < 34; ++k) at[k] += at[k - 1];
+        for (i64 r = g; r < e; ++r) ord[g + at[32 - len(r)]++] = static_cast<int>(r);
+    }
+    return ord;
+}
+
 void build_sell(Matrix &m, int fmt, cudaStream_t s) {
     Sell &S = fmt == 0 ? m.sell64 : m.sell32;
     if (S.built) return;
@@ -822,6 +788,7 @@ void build_sell(Matrix &m, int fmt, cudaStream_t s) {
                 lrow.push_back(static_cast<int>(r));
                 lptr.push_back(lptr.back() + rp[r + 1] - rp[r]);
             }
+        if (fmt == 0) S.ord.upload_vec(rows_by_length(rp, n_rows, n_slices * 32), s);
         S.n_lrows = static_cast<i64>(lrow.size());
         S.lrow.upload_vec(lrow, s);
         S.lptr.upload_vec(lptr, s);
@@ -916,15 +883,6 @@ void launch_split_long(const Sell &S, const float *x, i64 ldx, float *y, i64 ldy
     L.ldylo = ldylo;
     k_split_long<<<long_grid(L.n, nrhs), 256, 0, s>>>(L, x, ldx, y, ldy, nrhs);
 }
-void launch_f64_rows(const SellArgs &a, const double *x, i64 ldx, double *y, i64 ldy, i64 nrhs, cudaStream_t s) {
-    if (a.n_ids == 0 || nrhs == 0) return;
-    const i64 warps = a.n_ids * 32 * ((nrhs + 31) / 32);
-    k_f64_rows<<<nblk(warps * 32, 256), 256, 0, s>>>(a, x, ldx, y, ldy, nrhs);
-}
-void launch_f64_long(const Sell &S, const double *x, i64 ldx, double *y, i64 ldy, i64 nrhs, cudaStream_t s) {
-    if (S.n_lrows == 0 || nrhs == 0) return;
-    k_f64_long<<<long_grid(S.n_lrows, nrhs), 256, 0, s>>>(long_rows(S), x, ldx, y, ldy, nrhs);
-}
 }  // namespace
 
 // Rows of more than 32 entries given row-contiguous (the segmented layout's
@@ -971,26 +929,22 @@ void launch_f64_fused(const Matrix &m, const Sell &S, const double *x, i64 ldx, 
     if (warps == 0 || nrhs == 0) return;
     const SellArgs a = sell_args(m, S, 0);
     const LongRows L = long_rows(S);
-    const unsigned g = nblk(warps * 32, 256);
+    // Fields of a short row's warp: up to 64, so that its entries are read once
+    // from L2 and the tile's other passes find them in L1; fewer, down to 8,
+    // where that would leave less than about four waves of warps. 300 fields of
+    // C384 -> 0.25 deg: 3.58 ms with 64, 3.91 with 16, 4.70 with all; 20 fields
+    // of C384 -> 1 deg: 148 us with 8, 191 with 16.
+    const i64 fit = S.n_slices * nrhs / (152 * 24 * 4) / kF64F * kF64F;
+    const i64 tile = std::min<i64>(64, std::max<i64>(8, fit));
+    auto grid = [&](int F) {
+        return nblk((L.n * ((nrhs + F - 1) / F) + S.n_slices * ((nrhs + tile - 1) / tile)) * 32, 256);
+    };
     if (nrhs == 1)
-        k_f64_fused<1><<<g, 256, 0, s>>>(a, L, S.n_slices, x, ldx, y, ldy, nrhs);
+        k_f64_fused<1><<<grid(1), 256, 0, s>>>(a, L, S.ord.p, S.n_slices, x, ldx, y, ldy, nrhs, tile);
     else if (nrhs == 2)
-        k_f64_fused<2><<<g, 256, 0, s>>>(a, L, S.n_slices, x, ldx, y, ldy, nrhs);
+        k_f64_fused<2><<<grid(2), 256, 0, s>>>(a, L, S.ord.p, S.n_slices, x, ldx, y, ldy, nrhs, tile);
     else
-        k_f64_fused<kLongF><<<g, 256, 0, s>>>(a, L, S.n_slices, x, ldx, y, ldy, nrhs);
-}
-
-template <int L>
-void launch_f64(const SellArgs &a, const double *x, i64 ldx, double *y, i64 ldy, i64 nrhs, i64 tile, cudaStream_t s) {
-    i64 items = ((nrhs + tile - 1) / tile) * a.n_ids;
-    if (items == 0) return;
-    unsigned blocks = nblk(items * 32, 256);
-    if (nrhs >= 4)  // four independent FMA chains and their gathers in flight a thread (eight measured slower)
-        k_f64<L, 4><<<blocks, 256, 0, s>>>(a, x, ldx, y, ldy, nrhs, tile);
-    else if (nrhs >= 2)
-        k_f64<L, 2><<<blocks, 256, 0, s>>>(a, x, ldx, y, ldy, nrhs, tile);
-    else
-        k_f64<L, 1><<<blocks, 256, 0, s>>>(a, x, ldx, y, ldy, nrhs, tile);
+        k_f64_fused<kF64F><<<grid(kF64F), 256, 0, s>>>(a, L, S.ord.p, S.n_slices, x, ldx, y, ldy, nrhs, tile);
 }
 
 // ─── NaN-aware and masked FP64 applies ────────────────────────────────────
@@ -1474,19 +1428,8 @@ void apply_split_layouts(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, 
 void apply_f64(Matrix &m, const double *x, i64 ldx, double *y, i64 ldy, i64 nrhs, cudaStream_t s) {
     if (!m.sell64.built) matrix_prepare(m, 0, s);
     const Sell &S = m.sell64;
-    i64 tile = nrhs;
-    if (tile <= 0) return;
-    if (nrhs <= kFusedMaxF64) {  // one launch; same bits as the class kernels
-        launch_f64_fused(m, S, x, ldx, y, ldy, nrhs, s);
-        AXGB_CUDA(cudaGetLastError());
-        return;
-    }
-    launch_f64<8>(sell_args(m, S, 0), x, ldx, y, ldy, nrhs, tile, s);
-    launch_f64<16>(sell_args(m, S, 1), x, ldx, y, ldy, nrhs, tile, s);
-    launch_f64<32>(sell_args(m, S, 2), x, ldx, y, ldy, nrhs, tile, s);
-    launch_f64_rows(sell_args(m, S, 3), x, ldx, y, ldy, nrhs, s);
-    launch_f64_rows(sell_args(m, S, 4), x, ldx, y, ldy, nrhs, s);
-    launch_f64_long(S, x, ldx, y, ldy, nrhs, s);
+    if (nrhs <= 0) return;
+    launch_f64_fused(m, S, x, ldx, y, ldy, nrhs, s);
     AXGB_CUDA(cudaGetLastError());
 }
 

@@ -151,6 +151,7 @@ struct Sell {
     DBuf<int> base, len, col;
     DBuf<float> hi, lo;     // split weights (format 1)
     DBuf<double> w64;       // FP64 weights (format 0)
+    DBuf<int> ord;          // rows of every 128 by length, longest first (format 0)
     // slice ids grouped by length class: <=8, <=16, <=32, <=64, >64
     std::vector<i64> class_begin;  // 6 entries into class_ids
     DBuf<int> class_ids;

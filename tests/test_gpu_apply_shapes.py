@@ -97,3 +97,16 @@ def test_fields_per_work_item(gpu, oracle, nf, rows):
     y = gpu.apply_f32split(M, xs).cpu().numpy()
     assert np.array_equal(gpu.apply_f32split(M, xs, fields_per_pass=0, unroll=4, variant=3).cpu().numpy(), y)
     _check_split(y, *_reference(M, oracle, X))
+
+
+@pytest.mark.parametrize("nf,rows", [(65, 300), (130, 64000)])
+def test_f64_field_tiles(gpu, oracle, nf, rows):
+    """FP64 applies whose warps take 8 and 16 fields, the last tile in part."""
+    import torch
+    M = _rows_matrix(gpu, np.random.default_rng(14).choice(SHORT + [40], rows), 900, 15)
+    X = np.random.default_rng(16).standard_normal((nf, M.n_src))
+    xs = torch.tensor(X, device="cuda")
+    d = gpu.apply_f64(M, xs).cpu().numpy()
+    _check_f64(d, *_reference(M, oracle, X))
+    for f in (0, 8, nf - 1):
+        assert np.array_equal(gpu.apply_f64(M, xs[f:f + 1]).cpu().numpy()[0], d[f])

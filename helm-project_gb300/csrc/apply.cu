@@ -662,7 +662,7 @@ __global__ void k_slice_len(const int *rp, i64 n_rows, i64 n_slices, int *len) {
 // perm (optional): CSR index of the k-th entry of each row (split layouts).
 __global__ void k_sell_fill(const int *rp, const int *ccol, const double *val, const int *perm, i64 n_rows,
                             i64 n_slices, const int *base, const int *slen32, int *rlen, int *col, float *hi,
-                            float *lo, double *w64) {
+                            float *lo, double *w64, double *total) {
     i64 r = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (r >= n_slices * 32) return;
     i64 s = r >> 5;
@@ -676,11 +676,13 @@ __global__ void k_sell_fill(const int *rp, const int *ccol, const double *val, c
     }
     rlen[r] = n;
     int last = n > 0 ? ccol[r0 + n - 1] : 0;
+    double tot = 0.0;
     for (int k = 0; k < L; ++k) {
         int e = b + k * 32 + lane;
         if (k < n) {
             const int src = perm ? perm[r0 + k] : r0 + k;
             double w = val[src];
+            tot = __dadd_rn(tot, w);
             col[e] = ccol[src];
             if (hi) {
                 float h = __double2float_rn(w);
@@ -697,6 +699,7 @@ __global__ void k_sell_fill(const int *rp, const int *ccol, const double *val, c
             if (w64) w64[e] = 0.0;
         }
     }
+    if (total && r < n_rows) total[r] = tot;
 }
 
 // Rows of every 128 consecutive ones, longest first, rows of more than 32
@@ -748,6 +751,7 @@ void build_sell(Matrix &m, int fmt, cudaStream_t s) {
         S.lo.alloc(total);
     } else {
         S.w64.alloc(total);
+        S.total.alloc(n_rows);
     }
     if (n_slices > 0) {
         const int *perm = (fmt == 1 && m.split_perm.p) ? m.split_perm.p : nullptr;
@@ -755,7 +759,7 @@ void build_sell(Matrix &m, int fmt, cudaStream_t s) {
         k_sell_fill<<<nblk(n_slices * 32, 256), 256, 0, s>>>(m.row_ptr.p, ccol, m.val.p, perm, n_rows, n_slices,
                                                             S.base.p, slen32.p, rlen.p, S.col.p,
                                                             fmt == 1 ? S.hi.p : nullptr, fmt == 1 ? S.lo.p : nullptr,
-                                                            fmt == 0 ? S.w64.p : nullptr);
+                                                            fmt == 0 ? S.w64.p : nullptr, fmt == 0 ? S.total.p : nullptr);
         AXGB_CUDA(cudaGetLastError());
     }
     // length classes on the host
@@ -949,82 +953,223 @@ void launch_f64_fused(const Matrix &m, const Sell &S, const double *x, i64 ldx, 
 
 // ─── NaN-aware and masked FP64 applies ────────────────────────────────────
 // nan_batch_apply of include/axis/solver/apply.hpp:359-437 on the FP64
-// sliced-ELL layout (each row's entries in CSR order), lane per row: per row
-// the total weight, per field the weighted sum and the valid weight, with
+// layout (each row's entries in CSR order): per row the total weight
+// (Sell::total), per field the weighted sum and the valid weight, with
 // unfused multiply and add in entry order, so the NaN decisions and the
-// values match the reference loop bit for bit. 0 < L <= 32: entries cached
-// in registers; L == 0: rows of any length, entries re-read per field.
-__device__ __forceinline__ double nan_result(double total, double wsum, double valid, double na_thres) {
-    if (valid == 0.0 || total == 0.0) return __longlong_as_double(0x7ff8000000000000ll);
-    const double frac = __ddiv_rn(valid, total);
-    return frac < __dsub_rn(__dsub_rn(1.0, na_thres), 1e-6) ? __longlong_as_double(0x7ff8000000000000ll)
-                                                            : __ddiv_rn(wsum, valid);
+// values match the reference loop bit for bit.
+//
+// The bound is the FP64 pipe (half a lane an SM sub-partition and cycle), so
+// FP64 work is what is left out: NaN is tested on the bits, the valid weight
+// is summed only in rows that have a NaN (else it is the total, the same
+// additions), and the divisions are shortened (NanRow). 16 fields of 0.25 deg -> C384 with a third of the cells missing:
+// 651 us, against 2485 us with three FP64 operations an entry, two
+// divisions an output, and a lane walking each long row.
+constexpr int kNanG = 16;  // fields a warp
+constexpr int kNanU = 4;   // fields of a short row carried side by side
+constexpr int kNanK = 4;   // entries loaded ahead in a short row
+
+__device__ __forceinline__ bool nan_bits(double x) {
+    return (static_cast<unsigned long long>(__double_as_longlong(x)) & 0x7fffffffffffffffull) > 0x7ff0000000000000ull;
 }
 
-template <int L>
-__global__ void __launch_bounds__(256) k_nan_sell(SellArgs a, const double *__restrict__ x, i64 ldx,
-                                                  double *__restrict__ y, i64 ldy, i64 nrhs, double na_thres) {
-    const int lane = threadIdx.x & 31;
-    const i64 item = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    if (item >= a.n_ids) return;
-    const int sid = a.ids[item];
-    const i64 row = static_cast<i64>(sid) * 32 + lane;
-    if (row >= a.n_rows) return;
-    const int base = a.base[sid] + lane, rl = a.rlen[row];
-    if constexpr (L > 0) {
-        int c[L];
-        double w[L];
-        double total = 0.0;
-#pragma unroll
-        for (int k = 0; k < L; ++k) {
-            if (k < rl) {
-                c[k] = a.col[base + 32 * k];
-                w[k] = a.w64[base + 32 * k];
-                total = __dadd_rn(total, w[k]);
-            }
+__device__ __forceinline__ double nan_result(double total, double wsum, double valid, double thres) {
+    if (valid == 0.0 || total == 0.0) return __longlong_as_double(0x7ff8000000000000ll);
+    return __ddiv_rn(valid, total) < thres ? __longlong_as_double(0x7ff8000000000000ll) : __ddiv_rn(wsum, valid);
+}
+
+// What the outputs of one row share. A row without a NaN has valid = total,
+// its fraction total / total is 1 unless total is not finite, and its outputs
+// are quotients by one divisor: from the correctly rounded reciprocal y,
+// Markstein's two corrections with exact FMA residuals (IBM J. Res. Dev. 34,
+// 1990) give the correctly rounded quotient in five operations, where
+// __ddiv_rn takes about 25. It holds away from over- and underflow: operands
+// outside 2^+-500 take __ddiv_rn.
+struct NanRow {
+    double total, thres, p, y;  // p = thres * total
+    bool none;  // every output without a NaN is NaN
+    bool safe;  // total within 2^+-500
+    static __device__ __forceinline__ bool mid(double v) {
+        return static_cast<unsigned>(((__double2hiint(v) >> 20) & 0x7ff) - 523) <= 1000u;
+    }
+    __device__ __forceinline__ NanRow(double t, double th) : total(t), thres(th) {
+        none = t == 0.0 || (1.0 < th && fabs(t) <= 1.7976931348623157e308);
+        p = __dmul_rn(th, t);
+        safe = mid(t);
+        y = safe ? __drcp_rn(t) : 0.0;
+    }
+    __device__ __forceinline__ double all(double wsum) const {
+        if (none) return __longlong_as_double(0x7ff8000000000000ll);
+        if (!safe || !mid(wsum)) return __ddiv_rn(wsum, total);
+        const double q0 = __dmul_rn(wsum, y);
+        const double q1 = __fma_rn(__fma_rn(-total, q0, wsum), y, q0);
+        return __fma_rn(__fma_rn(-total, q1, wsum), y, q1);
+    }
+    // Some sources NaN, valid weight above 0 possible. The fraction is divided
+    // out only where it lies within 2^-48 of the threshold: the rounded product
+    // and quotient are off by 2^-52 at most. Positive doubles order as integers.
+    __device__ __forceinline__ double some(double wsum, double valid) const {
+        if (safe && mid(p) && mid(valid) && (__double2hiint(total) | __double2hiint(p) | __double2hiint(valid)) >= 0) {
+            const long long v = __double_as_longlong(valid), q = __double_as_longlong(p);
+            if (v < q - 32) return __longlong_as_double(0x7ff8000000000000ll);
+            if (v > q + 32) return __ddiv_rn(wsum, valid);
         }
-        for (i64 v = 0; v < nrhs; ++v) {
-            const double *xv = x + v * ldx;
-            double wsum = 0.0, valid = 0.0;
+        return nan_result(total, wsum, valid, thres);
+    }
+};
+
+// Warps [0, L.n): one row of more than 32 entries each. The lanes multiply 32
+// entries of each field side by side; then lane f < 16 adds the products of
+// field f in entry order and lane 16 + f the valid weights. Warps from L.n
+// on: lane per row (Sell::ord). blockIdx.y: 16 fields. The long rows come
+// first in the grid: their additions are chains of up to some thousand. The
+// outputs of short rows with some sources NaN need a second sum and a
+// division of their own; a warp with a coast has a few such lanes for every
+// field, so they are put aside and worked off 32 at a time, a lane each.
+struct NanItem {
+    double wsum;
+    unsigned mask;  // entries of the row whose source is NaN
+    unsigned short lane, field;
+};
+constexpr int kNanPs = 33;  // products a field (32, and one against bank conflicts)
+static_assert(sizeof(NanItem) * (31 + 32 * kNanU) <= sizeof(double) * kNanG * kNanPs, "items put aside fit a warp's ps");
+__global__ void __launch_bounds__(256) k_nan(SellArgs a, LongRows L, const double *__restrict__ totals,
+                                             const int *__restrict__ ord, i64 n_slices, const double *__restrict__ x,
+                                             i64 ldx, double *__restrict__ y, i64 ldy, i64 nrhs, double na_thres) {
+    __shared__ double ps[8][kNanG][kNanPs];
+    __shared__ double wsh[8][32];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const i64 wg = static_cast<i64>(blockIdx.x) * 8 + wp;
+    const double thres = __dsub_rn(__dsub_rn(1.0, na_thres), 1e-6);
+    if (wg < L.n) {
+        const i64 row = L.row[wg];
+        const int b = L.ptr[wg], n = L.ptr[wg + 1] - b;
+        const double total = totals[row];
+        {
+            const i64 f0 = static_cast<i64>(blockIdx.y) * kNanG;
+            const int nf = static_cast<int>(min(static_cast<i64>(kNanG), nrhs - f0));
+            const double *xf = x + f0 * ldx;
+            double acc = 0.0;  // lanes 0..15: weighted sum of field lane; lanes 16..31: its valid weight
+            for (int k0 = 0; k0 < n; k0 += 32) {
+                const bool on = k0 + lane < n;
+                const int c = on ? L.col[b + k0 + lane] : 0;
+                const double w = on ? L.w64[b + k0 + lane] : 0.0;
+                double xv[kNanG];
 #pragma unroll
-            for (int k = 0; k < L; ++k) {
-                if (k < rl) {
-                    const double xk = __ldg(xv + c[k]);
-                    if (!isnan(xk)) {
-                        wsum = __dadd_rn(wsum, __dmul_rn(w[k], xk));
-                        valid = __dadd_rn(valid, w[k]);
-                    }
+                for (int f = 0; f < kNanG; ++f) xv[f] = on && f < nf ? __ldg(xf + f * ldx + c) : 0.0;
+                unsigned skip = 0;
+                wsh[wp][lane] = w;
+#pragma unroll
+                for (int f = 0; f < kNanG; ++f) {
+                    const unsigned nan_mask = __ballot_sync(0xffffffffu, nan_bits(xv[f]));
+                    if ((lane & 15) == f) skip = nan_mask;
+                    ps[wp][f][lane] = __dmul_rn(w, xv[f]);
                 }
+                __syncwarp();
+                const int m = min(32, n - k0);
+                const double *src = lane < kNanG ? ps[wp][lane] : wsh[wp];
+#pragma unroll 8
+                for (int k = 0; k < m; ++k) {
+                    const double t = __dadd_rn(acc, src[k]);
+                    if (!((skip >> k) & 1u)) acc = t;
+                }
+                __syncwarp();
             }
-            y[v * ldy + row] = nan_result(total, wsum, valid, na_thres);
+            const double valid = __shfl_down_sync(0xffffffffu, acc, 16);
+            if (lane < nf) y[(f0 + lane) * ldy + row] = nan_result(total, acc, valid, thres);
         }
-    } else {
-        // rows of any length (the long classes): fields over gridDim.y, the
-        // loads of 8 entries issued ahead of their in-order accumulation
-        double total = 0.0;
-        for (int k = 0; k < rl; ++k) total = __dadd_rn(total, a.w64[base + 32 * k]);
-        for (i64 v = blockIdx.y; v < nrhs; v += gridDim.y) {
-            const double *xv = x + v * ldx;
-            double wsum = 0.0, valid = 0.0;
-            for (int k0 = 0; k0 < rl; k0 += 8) {
-                double wk[8], xk[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    if (k0 + u < rl) {
-                        wk[u] = a.w64[base + 32 * (k0 + u)];
-                        xk[u] = __ldg(xv + a.col[base + 32 * (k0 + u)]);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    if (k0 + u < rl && !isnan(xk[u])) {
-                        wsum = __dadd_rn(wsum, __dmul_rn(wk[u], xk[u]));
-                        valid = __dadd_rn(valid, wk[u]);
-                    }
-                }
+        return;
+    }
+    const i64 sid = wg - L.n;
+    if (sid >= n_slices) return;
+    const i64 row = ord[sid * 32 + lane];
+    const bool live = row < a.n_rows && a.rlen[row] <= 32;
+    const int n = live ? a.rlen[row] : 0;
+    const int base = a.base[row >> 5] + static_cast<int>(row & 31);
+    const NanRow R(live ? totals[row] : 0.0, thres);
+    const unsigned full = n == 32 ? 0xffffffffu : (1u << n) - 1u;
+    // outputs of rows with some sources NaN, put aside
+    NanItem *list = reinterpret_cast<NanItem *>(&ps[wp][0][0]);
+    int held = 0;  // warp-uniform
+    auto drain = [&](int at_least) {
+        while (held >= at_least && held > 0) {
+            const int take = min(held, 32);
+            __syncwarp();
+            const int i = held - take + lane;
+            NanItem it{0.0, 0, 0, 0};
+            if (lane < take) it = list[i];
+            held -= take;
+            // the row's constants by its lane
+            NanRow Q = R;
+            Q.total = __shfl_sync(0xffffffffu, R.total, it.lane);
+            Q.p = __shfl_sync(0xffffffffu, R.p, it.lane);
+            Q.safe = __shfl_sync(0xffffffffu, static_cast<int>(R.safe), it.lane) != 0;
+            const int qn = __shfl_sync(0xffffffffu, n, it.lane), qb = __shfl_sync(0xffffffffu, base, it.lane);
+            const i64 qrow = __shfl_sync(0xffffffffu, row, it.lane);
+            if (lane < take) {
+                double valid = 0.0;
+                for (int k = 0; k < qn; ++k)
+                    if (!((it.mask >> k) & 1u)) valid = __dadd_rn(valid, a.w64[qb + 32 * k]);
+                y[(static_cast<i64>(blockIdx.y) * kNanG + it.field) * ldy + qrow] = Q.some(it.wsum, valid);
             }
-            y[v * ldy + row] = nan_result(total, wsum, valid, na_thres);
+            __syncwarp();
         }
+    };
+    {
+        const i64 f0 = static_cast<i64>(blockIdx.y) * kNanG;
+        const int nf = static_cast<int>(min(static_cast<i64>(kNanG), nrhs - f0));
+        for (int g = 0; g < nf; g += kNanU) {
+            const double *xf = x + (f0 + g) * ldx;
+            double ws[kNanU];
+            unsigned nm[kNanU];  // the row's entries whose source is NaN
+#pragma unroll
+            for (int u = 0; u < kNanU; ++u) {
+                ws[u] = 0.0;
+                nm[u] = 0;
+            }
+            for (int k0 = 0; k0 < n; k0 += kNanK) {
+                int c[kNanK];
+                double w[kNanK], xv[kNanK][kNanU];
+#pragma unroll
+                for (int j = 0; j < kNanK; ++j)
+                    if (k0 + j < n) {
+                        c[j] = a.col[base + 32 * (k0 + j)];
+                        w[j] = a.w64[base + 32 * (k0 + j)];
+                    }
+#pragma unroll
+                for (int j = 0; j < kNanK; ++j)
+#pragma unroll
+                    for (int u = 0; u < kNanU; ++u)
+                        if (k0 + j < n && g + u < nf) xv[j][u] = __ldg(xf + u * ldx + c[j]);
+#pragma unroll
+                for (int j = 0; j < kNanK; ++j)
+                    if (k0 + j < n) {
+#pragma unroll
+                        for (int u = 0; u < kNanU; ++u)
+                            if (g + u < nf) {
+                                const bool bad = nan_bits(xv[j][u]);
+                                const double t = __dadd_rn(ws[u], __dmul_rn(w[j], xv[j][u]));
+                                ws[u] = bad ? ws[u] : t;
+                                nm[u] |= static_cast<unsigned>(bad) << (k0 + j);
+                            }
+                    }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < kNanU; ++u) {
+                if (g + u >= nf) break;
+                const bool aside = live && nm[u] != 0 && nm[u] != full;
+                const unsigned who = __ballot_sync(0xffffffffu, aside);
+                if (aside)
+                    list[held + __popc(who & ((1u << lane) - 1u))] =
+                        NanItem{ws[u], nm[u], static_cast<unsigned short>(lane), static_cast<unsigned short>(g + u)};
+                else if (live)
+                    y[(f0 + g + u) * ldy + row] =
+                        nm[u] == 0 ? R.all(ws[u]) : __longlong_as_double(0x7ff8000000000000ll);
+                held += __popc(who);
+            }
+            drain(32);
+        }
+        drain(1);
     }
 }
 
@@ -1482,16 +1627,13 @@ void nan_batch_apply_f64(Matrix &m, const double *x, i64 ldx, double *y, i64 ldy
     if (nrhs <= 0 || m.n_dst == 0) return;
     if (!m.sell64.built) matrix_prepare(m, 0, s);
     const Sell &S = m.sell64;
-    auto launch = [&](auto kernel, int cls, unsigned gy) {
-        const SellArgs a = sell_args(m, S, cls);
-        if (a.n_ids > 0) kernel<<<dim3(nblk(a.n_ids * 32, 256), gy), 256, 0, s>>>(a, x, ldx, y, ldy, nrhs, na_thres);
-    };
-    const unsigned fy = static_cast<unsigned>(std::min<i64>(nrhs, 65535));
-    launch(k_nan_sell<8>, 0, 1);
-    launch(k_nan_sell<16>, 1, 1);
-    launch(k_nan_sell<32>, 2, 1);
-    launch(k_nan_sell<0>, 3, fy);
-    launch(k_nan_sell<0>, 4, fy);
+    const i64 warps = S.n_lrows + S.n_slices;
+    for (i64 f = 0; f < nrhs; f += 65535 * kNanG) {
+        const i64 nf = std::min<i64>(nrhs - f, 65535 * kNanG);
+        const dim3 grid(nblk(warps, 8), nblk(nf, kNanG));
+        k_nan<<<grid, 256, 0, s>>>(sell_args(m, S, 0), long_rows(S), S.total.p, S.ord.p, S.n_slices, x + f * ldx, ldx,
+                                   y + f * ldy, ldy, nf, na_thres);
+    }
     AXGB_CUDA(cudaGetLastError());
 }
 

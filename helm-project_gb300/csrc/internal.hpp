@@ -151,6 +151,7 @@ struct Sell {
     DBuf<int> base, len, col;
     DBuf<float> hi, lo;     // split weights (format 1)
     DBuf<double> w64;       // FP64 weights (format 0)
+    DBuf<double> total;     // sum of each row's weights in CSR order (format 0; NaN-aware apply)
     DBuf<int> ord;          // rows of every 128 by length, longest first (format 0)
     // slice ids grouped by length class: <=8, <=16, <=32, <=64, >64
     std::vector<i64> class_begin;  // 6 entries into class_ids

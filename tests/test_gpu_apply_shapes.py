@@ -110,3 +110,38 @@ def test_f64_field_tiles(gpu, oracle, nf, rows):
     _check_f64(d, *_reference(M, oracle, X))
     for f in (0, 8, nf - 1):
         assert np.array_equal(gpu.apply_f64(M, xs[f:f + 1]).cpu().numpy()[0], d[f])
+
+
+@pytest.mark.parametrize("nf", [1, 3, 16, 17, 37])
+@pytest.mark.parametrize("weights,na_thres", [("positive", 0.5), ("positive", 0.0), ("positive", 1.0), ("signed", 0.5),
+                                              ("positive", -1.0), ("tiny", 0.3)])
+def test_nan_apply_row_shapes(gpu, oracle, nf, weights, na_thres):
+    """NaN-aware apply, bit for bit, on rows without NaN, with some and with
+    nothing else; weights whose sums cancel or lie outside the range of the
+    shortened division, infinite and zero fields, and a threshold above 1."""
+    import torch
+    M = _rows_matrix(gpu, _mixed_lens(21), 4000, 22)
+    c = M.to_csr()
+    rng = np.random.default_rng(23)
+    if weights == "signed":
+        c["val"] = c["val"] * rng.choice([-1.0, 1.0], M.nnz)
+    if weights == "tiny":
+        c["val"] = c["val"] * 2.0**-700
+    if weights != "positive":
+        M = gpu.Matrix.from_csr(M.n_src, M.n_dst, c["row_ptr"], c["col"], c["val"])
+    X = rng.standard_normal((nf, M.n_src)) * np.array([1.0, 2.0**400, 2.0**-600])[np.arange(nf) % 3][:, None]
+    X[:, 500:900] = np.nan  # land
+    X[rng.random((nf, M.n_src)) < 0.02] = np.nan
+    X[nf - 1, ::7] = np.inf
+    X[0, 2000:2400] = 0.0
+    if nf > 2:
+        X[1] = np.nan
+        X[2] = np.where(np.isnan(X[2]), 1.0, X[2])
+    from oracle import Weights
+    row = np.repeat(np.arange(M.n_dst), np.diff(c["row_ptr"])).astype(np.int64)
+    w = Weights(M.n_src, M.n_dst, row, c["col"].astype(np.int64), c["val"], c["frac_a"], c["frac_b"], c["area_a"],
+                c["area_b"])
+    ref = oracle.nan_batch_apply(w, X, na_thres)
+    y = gpu.nan_apply_f64(M, torch.tensor(X, device="cuda"), na_thres).cpu().numpy()
+    assert np.array_equal(np.isnan(y), np.isnan(ref))
+    assert np.array_equal(y[~np.isnan(y)], ref[~np.isnan(ref)])

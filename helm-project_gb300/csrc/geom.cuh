@@ -89,6 +89,34 @@ __device__ __forceinline__ DV3 d_arc_cross(const DV3 &v1, const DV3 &v2, const D
     return c;
 }
 
+// The same point, with the two square roots and reciprocals of the midpoint
+// test left out where its sign is beyond doubt: |c| = 1 and the midpoint of
+// an arc between unit vectors has length at most 2, so the dot products with
+// the midpoint and with the normalised midpoint differ from their exact
+// values by less than 1e-14, and above 1e-3 they have the same sign.
+__device__ __forceinline__ DV3 d_arc_cross_fast(const DV3 &v1, const DV3 &v2, const DV3 &n1) {
+    DV3 n2 = d_cross(v1, v2);
+    DV3 d = d_cross(n1, n2);
+    if (d_lensq(d) < 1.0e-30) return d_normalize(d_add(v1, v2));
+    DV3 c = d_normalize(d);
+    DV3 mid = d_add(v1, v2);
+    double side = d_dot(c, mid);
+    if (fabs(side) <= 1.0e-3) side = d_dot(c, d_normalize(mid));
+    if (side < 0.0) c = {-c.x, -c.y, -c.z};
+    return c;
+}
+
+// 2 atan2(num, den) for the small triangles that cells are cut into: up to
+// num / den = 2^-7 by Gregory's series to the ninth power (the next term is
+// below 2^-73 of the first), so the error is the quotient's rounding and the
+// last addition's. Larger ones by atan2.
+__device__ __forceinline__ double d_twice_atan(double num, double den) {
+    if (!(fabs(num) <= 0.0078125 * den)) return 2.0 * atan2(num, den);
+    const double t = num / den, q = t * t;
+    const double r = __fma_rn(q, __fma_rn(q, __fma_rn(q, 1.0 / 9.0, -1.0 / 7.0), 1.0 / 5.0), -1.0 / 3.0);
+    return 2.0 * __fma_rn(t * q, r, t);
+}
+
 // Clip `subject` by every edge of `clip` (Sutherland-Hodgman on great
 // circles, inclusive eps = -1e-14, edges with |a x b|^2 < 1e-30 skipped;
 // spherical_clipper.hpp:181-229 and :301-335). Returns the overlap area;

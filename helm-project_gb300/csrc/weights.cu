@@ -204,25 +204,143 @@ __device__ __forceinline__ void load_poly(const MeshView &m, i64 c, DPoly<CAP> &
     }
 }
 
+// The first 32 vertices of a cell, as load_poly has them.
+struct CellRef {
+    int n, b;  // vertices; first connectivity entry (regular: unused)
+    int i, j;  // regular grids: column and row
+    __device__ __forceinline__ CellRef(const MeshView &m, int c) : n(4), b(0), i(0), j(0) {
+        if (m.regular) {
+            j = c / m.ni;
+            i = c - j * m.ni;
+        } else {
+            b = m.off[c];
+            n = min(32, m.off[c + 1] - b);
+        }
+    }
+    __device__ __forceinline__ DV3 at(const MeshView &m, int k) const {
+        if (m.regular) {
+            const int ci = i + (k == 1 || k == 2 ? 1 : 0), cj = j + (k >= 2 ? 1 : 0);
+            const double *slon = m.trig, *clon = slon + (m.ni + 1), *slat = clon + (m.ni + 1), *clat = slat + (m.nj + 1);
+            const double cl = clat[cj];
+            return {cl * clon[ci], cl * slon[ci], slat[cj]};
+        }
+        const double *q = m.xyz + 3 * static_cast<i64>(m.idx[b + k]);
+        return {q[0], q[1], q[2]};
+    }
+};
+
+// Overlap areas of candidate pairs, a thread each: d_overlap_area for convex
+// cells. A half space cuts a convex polygon in at most one run of vertices,
+// so an edge of the clip cell has at most one crossing into and one out of
+// it: the side tests come first, then both crossings in straight-line code,
+// once an edge for the whole warp. (In the vertex loop of d_overlap_area some
+// lane of a warp has a crossing at nearly every vertex, and all of them pay.)
+// The polygon stays in shared memory, a column a thread: a lane's vertex index
+// does not change its bank. Pairs with more crossings or more than kClipCap
+// vertices go to the general kernel through over_list.
+// Bound by the FP64 pipe. 0.25 deg -> C384, 6.9 M candidates: 10.3 ms, against
+// 24.2 ms with the loop, its polygons in local memory, normalised midpoints
+// and atan2.
+constexpr int kClipCap = 12, kClipT = 128;
+__global__ void __launch_bounds__(kClipT) k_clip_convex(MeshView S, MeshView D, const int *__restrict__ cs,
+                                                        const int *__restrict__ cd, i64 n, double *ov, int *over_list,
+                                                        int *n_over) {
+    __shared__ double P[3 * kClipCap][kClipT];
+    const int tid = threadIdx.x;
+    const i64 k = static_cast<i64>(blockIdx.x) * kClipT + tid;
+    if (k >= n) return;
+    const CellRef C(S, cs[k]), E(D, cd[k]);
+    auto get = [&](int i) { return DV3{P[3 * i][tid], P[3 * i + 1][tid], P[3 * i + 2][tid]}; };
+    auto put = [&](int i, const DV3 &v) {
+        P[3 * i][tid] = v.x;
+        P[3 * i + 1][tid] = v.y;
+        P[3 * i + 2][tid] = v.z;
+    };
+    bool over = C.n > kClipCap;
+    int m = over || C.n < 3 || E.n < 3 ? 0 : C.n;
+    for (int i = 0; i < m; ++i) put(i, C.at(S, i));
+    if (m > 0) {
+        constexpr double eps = -1.0e-14;
+        const DV3 first = E.at(D, 0);
+        DV3 ea = first;
+        for (int ci = 0; ci < E.n; ++ci) {
+            const DV3 eb = ci + 1 == E.n ? first : E.at(D, ci + 1);
+            const DV3 nrm = d_cross(ea, eb);
+            ea = eb;
+            if (d_lensq(nrm) < 1.0e-30) continue;
+            unsigned in = 0;
+            for (int i = 0; i < m; ++i)
+                if (d_dot(nrm, get(i)) >= eps) in |= 1u << i;
+            const unsigned all = (1u << m) - 1u;
+            if (in == all) continue;
+            if (in == 0) {
+                m = 0;
+                break;
+            }
+            const unsigned prev = ((in << 1) | (in >> (m - 1))) & all;  // bit i: vertex before i inside
+            const unsigned enter = in & ~prev, leave = ~in & prev;
+            const int kept = __popc(in);
+            if (__popc(enter) > 1 || kept + 2 > kClipCap) {
+                over = true;
+                break;
+            }
+            const int a = __ffs(enter) - 1, b = __ffs(leave) - 1;
+            const DV3 xa = d_arc_cross_fast(get(a == 0 ? m - 1 : a - 1), get(a), nrm);
+            const DV3 xb = d_arc_cross_fast(get(b == 0 ? m - 1 : b - 1), get(b), nrm);
+            // in vertex order: xa before vertex a, xb in place of vertex b
+            if (a < b) {  // xa, [a, b), xb
+                if (a == 0)
+                    for (int i = kept - 1; i >= 0; --i) put(i + 1, get(i));
+                else if (a > 1)
+                    for (int i = 0; i < kept; ++i) put(i + 1, get(a + i));
+                put(0, xa);
+                put(kept + 1, xb);
+            } else {  // the run passes the end: [0, b), xb, xa, [a, m)
+                const int tail = m - a;
+                if (a < b + 2)
+                    for (int i = tail - 1; i >= 0; --i) put(b + 2 + i, get(a + i));
+                else if (a > b + 2)
+                    for (int i = 0; i < tail; ++i) put(b + 2 + i, get(a + i));
+                put(b, xb);
+                put(b + 1, xa);
+            }
+            m = kept + 2;
+        }
+    }
+    if (over) {
+        over_list[atomicAdd(n_over, 1)] = static_cast<int>(k);
+        ov[k] = 0.0;
+        return;
+    }
+    // fan from vertex 0, as d_poly_area
+    double total = 0.0;
+    if (m >= 3) {
+        const DV3 a = get(0);
+        DV3 b = get(1);
+        double ab = d_dot(a, b);
+        for (int i = 2; i < m; ++i) {
+            const DV3 q = get(i);
+            const double aq = d_dot(a, q), bq = d_dot(b, q);
+            total += d_twice_atan(d_dot(a, d_cross(b, q)), 1.0 + ab + aq + bq);
+            b = q;
+            ab = aq;
+        }
+    }
+    ov[k] = fabs(total);
+}
+
+// The pairs of list by the general clipper.
 template <int CAP>
-__global__ void __launch_bounds__(128) k_clip(MeshView S, MeshView D, const int *__restrict__ cs,
-                                              const int *__restrict__ cd, i64 n, const int *list, double *ov,
-                                              int *over_list, int *n_over) {
+__global__ void __launch_bounds__(64) k_clip(MeshView S, MeshView D, const int *__restrict__ cs,
+                                             const int *__restrict__ cd, i64 n, const int *list, double *ov) {
     i64 t = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= n) return;
-    i64 k = list ? list[t] : t;
+    i64 k = list[t];
     DPoly<CAP> sp, dp, ba, bb;
     load_poly(S, cs[k], sp);
     load_poly(D, cd[k], dp);
     bool over = false;
-    double a = d_overlap_area(sp, dp, ba, bb, &over);
-    if (over && CAP < 32) {
-        int q = atomicAdd(n_over, 1);
-        over_list[q] = static_cast<int>(k);
-        ov[k] = 0.0;
-    } else {
-        ov[k] = a;
-    }
+    ov[k] = d_overlap_area(sp, dp, ba, bb, &over);
 }
 
 // ─── assembly ──────────────────────────────────────────────────────────────
@@ -831,11 +949,11 @@ void generate_conservative(Mesh &src, Mesh &dst, const axgb_regrid_config &cfg, 
     n_over.zero(s);
     int h_over = 0;
     if (n_cand > 0) {
-        k_clip<16><<<nblk(n_cand, 128), 128, 0, s>>>(S, D, cs.p, cd.p, n_cand, nullptr, ov.p, over_list.p, n_over.p);
+        k_clip_convex<<<nblk(n_cand, kClipT), kClipT, 0, s>>>(S, D, cs.p, cd.p, n_cand, ov.p, over_list.p, n_over.p);
         AXGB_CUDA(cudaGetLastError());
         AXGB_CUDA(cudaMemcpy(&h_over, n_over.p, sizeof(int), cudaMemcpyDeviceToHost));
         if (h_over > 0) {
-            k_clip<32><<<nblk(h_over, 64), 64, 0, s>>>(S, D, cs.p, cd.p, h_over, over_list.p, ov.p, nullptr, nullptr);
+            k_clip<32><<<nblk(h_over, 64), 64, 0, s>>>(S, D, cs.p, cd.p, h_over, over_list.p, ov.p);
             AXGB_CUDA(cudaGetLastError());
         }
     }

@@ -1,0 +1,45 @@
+"""Weight generation on cells of many shapes: vertex counts at and past what
+the convex clipper keeps, cells that are not convex, regular and
+unstructured meshes on either side. The bars are those of the parity tests:
+index set exact, values within 1e-12."""
+import numpy as np
+import pytest
+
+from axgb import grids
+
+from test_gpu_parity import _check_weights
+
+pytestmark = pytest.mark.gpu
+
+
+def _subdivided(m, k, bulge=0.0):
+    """m with k points on every edge (from its first vertex on) of each cell,
+    the inner ones moved towards the cell's mean by bulge: 4 k vertices a
+    quadrilateral, concave for bulge > 0."""
+    ll, idx = m.node_lonlat, m.conn_indices.reshape(-1, 4)
+    v = ll[idx]  # [cells, 4, 2]
+    mean = v.mean(axis=1, keepdims=True)
+    pts = []
+    for e in range(4):
+        a, b = v[:, e], v[:, (e + 1) % 4]
+        for q in range(k):
+            p = a + (b - a) * (q / k)
+            if q:
+                p = p + bulge * (mean[:, 0] - p)
+            pts.append(p)
+    node = np.stack(pts, axis=1).reshape(-1, 2)
+    n = m.n_cells
+    return grids.MeshArrays(node, np.arange(0, 4 * k * n + 1, 4 * k, dtype=np.int64), np.arange(4 * k * n), name="sub")
+
+
+@pytest.mark.parametrize("side", ["src", "dst"])
+@pytest.mark.parametrize("k,bulge", [(2, 0.0), (3, 0.0), (4, 0.0), (9, 0.0), (2, 0.15), (3, 0.3)])
+def test_many_vertices_and_concave_cells(gpu, oracle, k, bulge, side):
+    """8 to 36 vertices a cell (12 are kept by the convex clipper, 32 by any)."""
+    a = _subdivided(grids.rectilinear(np.linspace(20.0, 70.0, 21), np.linspace(-30.0, 25.0, 19)), k, bulge)
+    b = grids.cubed_sphere(12)
+    src, dst = (a, b) if side == "src" else (b, a)
+    M = gpu.generate_weights(gpu.Mesh.from_grid(src), gpu.Mesh.from_grid(dst), {"method": "conservative"})
+    _check_weights(M, oracle.conservative(src, dst))
+    if side == "src" and (bulge > 0.0 or 4 * k > 12):  # the source cell is the polygon that is cut
+        assert M.stats()["fallback_clips"] > 0

@@ -24,6 +24,8 @@ namespace {
 thread_local std::string g_last_error;
 std::atomic<int> g_autotune{0};
 
+void scratch_give_back();
+
 struct Registry {
     std::mutex mu;
     int next = 1;
@@ -51,6 +53,7 @@ struct Registry {
     template <class T>
     void drop(std::map<int, std::shared_ptr<T>> &m, int h, const char *what) {
         std::shared_ptr<T> keep;
+        bool last;
         {
             std::lock_guard<std::mutex> lk(mu);
             auto it = m.find(h);
@@ -58,7 +61,10 @@ struct Registry {
                 throw Error(AXGB_ERR_HANDLE, std::string("unknown ") + what + " handle " + std::to_string(h));
             keep = std::move(it->second);
             m.erase(it);
+            last = meshes.empty() && mats.empty() && batches.empty();
         }
+        keep.reset();
+        if (last) scratch_give_back();
     }
 };
 
@@ -194,6 +200,22 @@ void mesh_upload_impl(Mesh &m) {
         m.d_trig.upload(t.data(), t.size());
     }
     AXGB_CUDA(cudaDeviceSynchronize());
+}
+
+struct ScratchPools {
+    std::mutex mu;
+    std::map<int, cudaMemPool_t> of;  // by device
+    static ScratchPools &get() {
+        static ScratchPools p;
+        return p;
+    }
+};
+
+// What the pools keep goes back to the device (blocks in use stay).
+void scratch_give_back() {
+    auto &P = ScratchPools::get();
+    std::lock_guard<std::mutex> lk(P.mu);
+    for (auto &kv : P.of) cudaMemPoolTrimTo(kv.second, 0);
 }
 
 // Reusable device staging for the host-pointer entry points.
@@ -406,6 +428,27 @@ SplitParams default_split_params(const Matrix &m, i64 nrhs) {
 }
 
 }  // namespace
+
+cudaMemPool_t scratch_pool() {
+    int dev = 0;
+    AXGB_CUDA(cudaGetDevice(&dev));
+    auto &P = ScratchPools::get();
+    std::lock_guard<std::mutex> lk(P.mu);
+    auto it = P.of.find(dev);
+    if (it != P.of.end()) return it->second;
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool;
+    AXGB_CUDA(cudaMemPoolCreate(&pool, &props));
+    std::uint64_t keep = kScratchKept;
+    AXGB_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    P.of[dev] = pool;
+    return pool;
+}
+
 }  // namespace axgb
 
 using namespace axgb;

@@ -739,7 +739,8 @@ void build_sell(Matrix &m, int fmt, cudaStream_t s) {
     }
     scan_exclusive_i32(slen32.p, base.p, n_slices, s);
     int total = 0;
-    AXGB_CUDA(cudaMemcpy(&total, base.p + n_slices, sizeof(int), cudaMemcpyDeviceToHost));
+    AXGB_CUDA(cudaMemcpyAsync(&total, base.p + n_slices, sizeof(int), cudaMemcpyDeviceToHost, s));
+    AXGB_CUDA(cudaStreamSynchronize(s));
     S.n_slices = n_slices;
     S.n_entries = total;
     S.col.alloc(total);

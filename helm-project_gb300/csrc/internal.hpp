@@ -91,6 +91,37 @@ struct DBuf {
     }
 };
 
+// Stream-ordered scratch: taken from and returned to the library's own
+// memory pool on one stream, which must be the one its users run on. The pool
+// (one per device, api.cpp) keeps at most kScratchKept bytes between calls
+// and gives them back when the last mesh, matrix and batch is destroyed. An
+// allocation costs about a microsecond where cudaMalloc and cudaFree take tens
+// and wait for the device.
+constexpr size_t kScratchKept = size_t(512) << 20;
+cudaMemPool_t scratch_pool();
+template <class T>
+struct Scratch {
+    T *p = nullptr;
+    size_t n = 0;
+    cudaStream_t s;
+    explicit Scratch(cudaStream_t st) : s(st) {}
+    Scratch(size_t count, cudaStream_t st) : s(st) { alloc(count); }
+    Scratch(const Scratch &) = delete;
+    Scratch &operator=(const Scratch &) = delete;
+    ~Scratch() { release(); }
+    void alloc(size_t count) {
+        release();
+        n = count ? count : 1;
+        AXGB_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), n * sizeof(T), scratch_pool(), s));
+    }
+    void release() {
+        if (p) cudaFreeAsync(p, s);
+        p = nullptr;
+        n = 0;
+    }
+    void zero() { AXGB_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), s)); }
+};
+
 // Result of the regular / rectilinear grid detection
 // (detail/regular_grid_detector.hpp:64-299).
 struct GridInfo {
@@ -368,7 +399,7 @@ void slice_centroids(const MeshView &dst, Matrix &m, cudaStream_t s);
 // areas where it has them, else planar shoelace areas in degrees (nearest.cu).
 void planar_cell_areas(const MeshView &m, double *out, cudaStream_t s);
 
-// scan_sort.cu: device primitives (own implementations)
+// scan_sort.cu: device primitives (own implementations), stream-ordered
 // out[0..n] = exclusive prefix sum of in[0..n-1], out[n] = total.
 void scan_exclusive_i32_to_i64(const int *in, i64 *out, i64 n, cudaStream_t s);
 void scan_exclusive_i32(const int *in, int *out, i64 n, cudaStream_t s);

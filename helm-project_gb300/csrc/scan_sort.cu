@@ -106,12 +106,11 @@ void scan_impl(const TIn *in, TOut *out, i64 n, cudaStream_t s) {
         return;
     }
     i64 nb = (n + kScanTile - 1) / kScanTile;
-    DBuf<TOut> sums(nb);
+    Scratch<TOut> sums(nb, s);
     k_tile_sums<TIn, TOut><<<static_cast<unsigned>(nb), kScanThreads, 0, s>>>(in, n, sums.p);
     k_scan_sums<TOut><<<1, kScanThreads, 0, s>>>(sums.p, nb);
     k_tile_scan<TIn, TOut><<<static_cast<unsigned>(nb), kScanThreads, 0, s>>>(in, n, sums.p, out);
     AXGB_CUDA(cudaGetLastError());
-    AXGB_CUDA(cudaStreamSynchronize(s));
 }
 
 // ─── radix sort ────────────────────────────────────────────────────────────
@@ -189,8 +188,8 @@ void radix_impl(K *keys, int *vals, i64 n, int key_bits, cudaStream_t s) {
     if (n <= 1 || key_bits <= 0) return;
     if (n >= (i64(1) << 31)) throw Error(AXGB_ERR_UNSUPPORTED, "radix sort: more than 2^31 items");
     int nblocks = static_cast<int>((n + kRsTile - 1) / kRsTile);
-    DBuf<K> k2(n);
-    DBuf<int> v2(n), hist(static_cast<size_t>(256) * nblocks), offs(static_cast<size_t>(256) * nblocks + 1);
+    Scratch<K> k2(n, s);
+    Scratch<int> v2(n, s), hist(static_cast<size_t>(256) * nblocks, s), offs(static_cast<size_t>(256) * nblocks + 1, s);
     K *a = keys, *b = k2.p;
     int *av = vals, *bv = v2.p;
     for (int shift = 0; shift < key_bits; shift += 8) {
@@ -205,7 +204,6 @@ void radix_impl(K *keys, int *vals, i64 n, int key_bits, cudaStream_t s) {
         AXGB_CUDA(cudaMemcpyAsync(keys, a, n * sizeof(K), cudaMemcpyDeviceToDevice, s));
         AXGB_CUDA(cudaMemcpyAsync(vals, av, n * sizeof(int), cudaMemcpyDeviceToDevice, s));
     }
-    AXGB_CUDA(cudaStreamSynchronize(s));
 }
 
 }  // namespace

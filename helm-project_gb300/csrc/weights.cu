@@ -11,8 +11,8 @@
 //   3. one thread per destination cell walks the ropes; every leaf hit goes
 //      through the reference's exact gates (source mask / degenerate /
 //      area > 0, the reference's float AABB test, the FP64 cap test) and is
-//      counted (pass 1) or written (pass 2) row-grouped, so the candidate
-//      list is deterministic;
+//      kept, grouped by row in traversal order, so the candidate list is
+//      deterministic;
 //   4. one thread per candidate runs the FP64 great-circle clip and the
 //      spherical area (geom.cuh, --fmad=false); pairs whose polygons
 //      exceed 16 vertices are redone with the reference's 32-vertex cap;
@@ -70,7 +70,7 @@ __global__ void k_leaves(Bvh t, MeshView S, const int *vals) {
     t.hi[t.n - 1 + q] = hi;
 }
 
-// ─── candidate search (two passes) ─────────────────────────────────────────
+// ─── candidate search ──────────────────────────────────────────────────────
 
 __device__ __forceinline__ bool fbox_meet(const float *a, const float *b) {
 #pragma unroll
@@ -111,46 +111,62 @@ __device__ __forceinline__ bool gate(const MeshView &S, int i, const float *dbox
     return !(acos(cd) > (sc.r + dc.r));
 }
 
-template <bool FILL>
+// One thread a row walks the ropes; the first cap candidates go to slots
+// ([cap][rows]). A row that meets more, or visits more than kWalkSteps nodes,
+// gives up (slots row 0 = -1) and is listed for k_search_wide: the polar rows
+// of a lat-lon source have over a thousand candidates, and as one thread's
+// chain of dependent loads they were the length of the whole search.
+// 0.25 deg -> C384: 0.76 ms and 0.54 for the wide rows, against 2 x 2.97 ms for
+// one thread a row, counting and then writing.
+constexpr int kWalkSteps = 256;
+
+__device__ __forceinline__ bool node_meets(const float4 &lo, const float4 &hi, float qx, float qy, float qz, float rq2) {
+    const float dx = fmaxf(fmaxf(lo.x - qx, 0.f), qx - hi.x);
+    const float dy = fmaxf(fmaxf(lo.y - qy, 0.f), qy - hi.y);
+    const float dz = fmaxf(fmaxf(lo.z - qz, 0.f), qz - hi.z);
+    return dx * dx + dy * dy + dz * dz <= rq2;
+}
+
+// A destination cell's query: its gates' operands, and the ball the nodes meet.
+struct Query {
+    DCap dc;
+    float4 dcf;
+    float dbox[6];
+    float qx, qy, qz, rq2;
+    __device__ __forceinline__ Query(const MeshView &D, i64 j) : dc(D.cap[j]), dcf(D.capf[j]) {
+#pragma unroll
+        for (int d = 0; d < 6; ++d) dbox[d] = D.box[6 * j + d];
+        qx = static_cast<float>(dc.x);
+        qy = static_cast<float>(dc.y);
+        qz = static_cast<float>(dc.z);
+        const float rq = ball_radius(dc.r);
+        rq2 = __fmul_ru(rq, rq) * 1.000001f + 1e-12f;
+    }
+};
+
 __global__ void k_search(MeshView S, MeshView D, const float4 *__restrict__ nlo, const float4 *__restrict__ nhi,
-                         int root, int n_leaf_base, int *counts, const i64 *offs, int *out_src,
-                         unsigned long long *raw_hits, int *err) {
+                         int root, int n_leaf_base, int *counts, int *slots, int cap, int *wide, int *n_wide,
+                         unsigned long long *raw_hits) {
     i64 j = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     unsigned long long hits = 0;
     if (j < D.n_cells) {
         int cnt = 0;
         if (!(D.flags[j] & kExcluded) && root >= 0) {
-            DCap dc = D.cap[j];
-            const float4 dcf = D.capf[j];
-            float dbox[6];
-#pragma unroll
-            for (int d = 0; d < 6; ++d) dbox[d] = D.box[6 * j + d];
-            float qx = static_cast<float>(dc.x), qy = static_cast<float>(dc.y), qz = static_cast<float>(dc.z);
-            float rq = ball_radius(dc.r);
-            float rq2 = __fmul_ru(rq, rq) * 1.000001f + 1e-12f;
-            i64 wbase = FILL ? offs[j] : 0;
+            const Query q(D, j);
             int node = root;
-            // Ropes visit every node at most once; a longer walk means a
-            // malformed tree: flag it and stop instead of spinning.
-            const int max_steps = 2 * (2 * n_leaf_base + 1) + 8;
-            int steps = 0;
-            while (node >= 0) {
-                if (++steps > max_steps) {
-                    atomicOr(err, 1);
+            for (int steps = 0; node >= 0; ++steps) {
+                if (steps == kWalkSteps) {
+                    cnt = cap + 1;
                     break;
                 }
                 float4 lo = nlo[node], hi = nhi[node];
-                float dx = fmaxf(fmaxf(lo.x - qx, 0.f), qx - hi.x);
-                float dy = fmaxf(fmaxf(lo.y - qy, 0.f), qy - hi.y);
-                float dz = fmaxf(fmaxf(lo.z - qz, 0.f), qz - hi.z);
-                float d2 = dx * dx + dy * dy + dz * dz;
-                if (d2 <= rq2) {
+                if (node_meets(lo, hi, q.qx, q.qy, q.qz, q.rq2)) {
                     if (node >= n_leaf_base) {
                         int cell = __float_as_int(lo.w);
                         ++hits;
-                        if (gate(S, cell, dbox, dc, dcf)) {
-                            if (FILL) out_src[wbase + cnt] = cell;
-                            ++cnt;
+                        if (gate(S, cell, q.dbox, q.dc, q.dcf)) {
+                            if (cnt < cap) slots[static_cast<i64>(cnt) * D.n_cells + j] = cell;
+                            if (++cnt > cap) break;
                         }
                         node = __float_as_int(hi.w);
                     } else {
@@ -161,19 +177,102 @@ __global__ void k_search(MeshView S, MeshView D, const float4 *__restrict__ nlo,
                 }
             }
         }
-        if (!FILL) counts[j] = cnt;
+        if (cnt > cap) {
+            slots[j] = -1;
+            wide[atomicAdd(n_wide, 1)] = static_cast<int>(j);
+            cnt = 0;
+            hits = 0;  // counted by k_search_wide
+        }
+        counts[j] = cnt;
+    }
+    // warp-aggregated counter of raw leaf hits
+    for (int o = 16; o > 0; o >>= 1) hits += __shfl_down_sync(0xffffffffu, hits, o);
+    if ((threadIdx.x & 31) == 0 && hits) atomicAdd(raw_hits, hits);
+}
+
+// The listed rows, a warp each: the lanes test the 32 nodes on top of a stack
+// and push the children of those that meet the query. Popping 32 and pushing
+// up to 64 leaves at most 32 more; above kWideHigh entries one node is popped
+// at a time, which adds one a level of the tree (at most 62), so the stack
+// cannot overflow. Counts (FILL = false), then writes (the order of a row's
+// candidates does not matter: the rows are sorted by column in the end).
+constexpr int kWideStack = 1024, kWideHigh = kWideStack - 64 - 64, kWideWarps = 4;
+
+template <bool FILL>
+__global__ void __launch_bounds__(32 * kWideWarps) k_search_wide(MeshView S, MeshView D, const float4 *__restrict__ nlo,
+                                                                const float4 *__restrict__ nhi,
+                                                                const int *__restrict__ right, int root,
+                                                                int n_leaf_base, const int *wide, const int *n_wide,
+                                                                int *counts, const i64 *offs, int *out_src,
+                                                                unsigned long long *raw_hits, int *err) {
+    __shared__ int stacks[kWideWarps][kWideStack];
+    const int lane = threadIdx.x & 31;
+    int *st = stacks[threadIdx.x >> 5];
+    const int n = *n_wide;
+    unsigned long long hits = 0;
+    for (int i = blockIdx.x * kWideWarps + (threadIdx.x >> 5); i < n; i += gridDim.x * kWideWarps) {
+        const i64 j = wide[i];
+        const Query q(D, j);
+        const i64 at = FILL ? offs[j] : 0;
+        int sp = 1, cnt = 0;
+        i64 seen = 0;
+        __syncwarp();
+        if (lane == 0) st[0] = root;
+        while (sp > 0) {
+            __syncwarp();
+            const int take = sp > kWideHigh ? 1 : min(sp, 32);
+            const int node = lane < take ? st[sp - take + lane] : -1;
+            sp -= take;
+            // every node is reached once; more means a malformed tree: flag it and stop
+            if ((seen += take) > 2 * static_cast<i64>(n_leaf_base) + 1) {
+                if (lane == 0) atomicOr(err, 1);
+                break;
+            }
+            bool inner = false, keep = false;
+            int cell = -1, left = -1;
+            if (node >= 0) {
+                const float4 lo = nlo[node], hi = nhi[node];
+                if (node_meets(lo, hi, q.qx, q.qy, q.qz, q.rq2)) {
+                    if (node >= n_leaf_base) {
+                        cell = __float_as_int(lo.w);
+                        ++hits;
+                        keep = gate(S, cell, q.dbox, q.dc, q.dcf);
+                    } else {
+                        inner = true;
+                        left = __float_as_int(lo.w);
+                    }
+                }
+            }
+            const unsigned below = (1u << lane) - 1u;
+            const unsigned who = __ballot_sync(0xffffffffu, inner), got = __ballot_sync(0xffffffffu, keep);
+            if (inner) {
+                const int p = sp + 2 * __popc(who & below);
+                st[p] = left;
+                st[p + 1] = right[node];
+            }
+            sp += 2 * __popc(who);
+            if (FILL && keep) out_src[at + cnt + __popc(got & below)] = cell;
+            cnt += __popc(got);
+        }
+        if (!FILL && lane == 0) counts[j] = cnt;
     }
     if (!FILL) {
-        // warp-aggregated counter of raw leaf hits
         for (int o = 16; o > 0; o >>= 1) hits += __shfl_down_sync(0xffffffffu, hits, o);
-        if ((threadIdx.x & 31) == 0 && hits) atomicAdd(raw_hits, hits);
+        if (lane == 0 && hits) atomicAdd(raw_hits, hits);
     }
 }
 
-__global__ void k_fill_rows(const i64 *offs, i64 n_dst, int *out_dst) {
-    i64 j = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
+// Candidates kept by k_search, the row of every candidate.
+__global__ void k_take_slots(const int *counts, const i64 *offs, const int *slots, i64 n_dst, int *out_src,
+                             int *out_dst) {
+    const i64 j = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (j >= n_dst) return;
-    for (i64 k = offs[j]; k < offs[j + 1]; ++k) out_dst[k] = static_cast<int>(j);
+    const int n = counts[j];
+    if (n == 0) return;
+    const i64 b = offs[j];
+    if (slots[j] >= 0)
+        for (int q = 0; q < n; ++q) out_src[b + q] = slots[q * n_dst + j];
+    for (int q = 0; q < n; ++q) out_dst[b + q] = static_cast<int>(j);
 }
 
 // ─── clipping ──────────────────────────────────────────────────────────────
@@ -345,73 +444,131 @@ __global__ void __launch_bounds__(64) k_clip(MeshView S, MeshView D, const int *
 
 // ─── assembly ──────────────────────────────────────────────────────────────
 
+// The kept pairs (overlap > 0) of the candidate list go into CSR, columns
+// ascending. The list is grouped by row, so an entry's place is its row's
+// start plus the kept candidates of the row that come before it in column
+// order. That is counted directly, a thread an entry, where the rows are short
+// (the squares of their lengths sum to at most kRankWork per candidate: 8
+// for 0.25 deg -> C384); otherwise a stable radix sort by (row, column) gives
+// it.
+constexpr i64 kRankWork = 64;
+
+// Kept candidates per row; key = the column of a kept candidate, else -1.
+__global__ void k_row_kept(const double *ov, const int *cs, const int *cd, i64 n, int *kept, int *key) {
+    const i64 k = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const bool keep = ov[k] > 0.0;
+    key[k] = keep ? cs[k] : -1;
+    if (keep) atomicAdd(&kept[cd[k]], 1);
+}
+
+__global__ void k_row_squares(const i64 *offs, i64 n_dst, unsigned long long *squares) {
+    const i64 j = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const unsigned long long m = j < n_dst ? static_cast<unsigned long long>(offs[j + 1] - offs[j]) : 0;
+    unsigned long long sq = m * m;
+    for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, o);
+    if ((threadIdx.x & 31) == 0 && sq) atomicAdd(squares, sq);
+}
+
+__global__ void k_reciprocal(const double *a, i64 n, double *y) {
+    const i64 k = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k < n) y[k] = __drcp_rn(a[k]);
+}
+
+// What an entry carries out of the candidate list (weight_generator.cpp:
+// 3684-3716): w = overlap / destination area; fa = its contribution to
+// frac_a, overlap / source area or the one the generator gives. The
+// divisors repeat, so their reciprocals are formed once a cell (d_div_by).
+struct EntryArgs {
+    const double *ov, *fac;
+    const int *cs, *cd;
+    const double *area_src, *area_dst, *rcp_src, *rcp_dst;
+    const int *row_ptr;
+    int *col;
+    double *w, *fa;
+    unsigned *ckey;  // column and CSR index, for the column sums
+    int *cval;
+    int *gen;  // position among the kept candidates, or null
+};
+
+__device__ __forceinline__ void write_entry(const EntryArgs &a, i64 k, int at, int before) {
+    const int c = a.cs[k], j = a.cd[k];
+    const double o = a.ov[k];
+    a.col[at] = c;
+    a.w[at] = d_div_by(o, a.area_dst[j], a.rcp_dst[j]);
+    a.fa[at] = a.fac ? a.fac[k] : d_div_by(o, a.area_src[c], a.rcp_src[c]);
+    a.ckey[at] = static_cast<unsigned>(c);
+    a.cval[at] = at;
+    if (a.gen) a.gen[at] = before;
+}
+
+__global__ void k_place(EntryArgs a, const i64 *offs, const int *__restrict__ key, int n) {
+    const int k = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+    if (k >= n) return;
+    const int c = key[k];
+    if (c < 0) return;
+    const int j = a.cd[k], b = static_cast<int>(offs[j]), e = static_cast<int>(offs[j + 1]);
+    int rank = 0, before = 0;
+    for (int q = b; q < e; ++q) {
+        const int cq = key[q];
+        rank += static_cast<unsigned>(cq) < static_cast<unsigned>(c) || (cq == c && q < k) ? 1 : 0;
+        before += cq >= 0 && q < k ? 1 : 0;
+    }
+    write_entry(a, k, a.row_ptr[j] + rank, a.row_ptr[j] + before);
+}
+
+// The radix path: kept candidates compacted (pos), sorted, written.
 __global__ void k_keep_flags(const double *ov, i64 n, int *keep) {
     i64 k = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (k < n) keep[k] = ov[k] > 0.0 ? 1 : 0;
 }
 
-__global__ void k_compact(const double *ov, const double *fac, const int *cs, const int *cd, const i64 *pos, i64 n,
-                          std::uint64_t *key, int *vals, double *kov, double *kfac) {
+__global__ void k_compact(const double *ov, const int *cs, const int *cd, const i64 *pos, i64 n, std::uint64_t *key,
+                          int *vals, int *cand) {
     i64 k = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    if (ov[k] > 0.0) {
-        i64 p = pos[k];
-        key[p] = (static_cast<unsigned long long>(cd[k]) << 32) | static_cast<unsigned>(cs[k]);
-        vals[p] = static_cast<int>(p);
-        kov[p] = ov[k];
-        if (fac) kfac[p] = fac[k];
-    }
+    if (k >= n || !(ov[k] > 0.0)) return;
+    const i64 p = pos[k];
+    key[p] = (static_cast<unsigned long long>(cd[k]) << 32) | static_cast<unsigned>(cs[k]);
+    vals[p] = static_cast<int>(p);
+    cand[p] = static_cast<int>(k);
 }
 
-__global__ void k_count_keys(const std::uint64_t *key, i64 n, int *cnt) {
-    i64 k = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k < n) atomicAdd(&cnt[key[k] >> 32], 1);
+__global__ void k_write_sorted(EntryArgs a, const int *perm, const int *cand, i64 nnz) {
+    const i64 at = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (at < nnz) write_entry(a, cand[perm[at]], static_cast<int>(at), perm[at]);
 }
 
-__global__ void k_csr_cols(const std::uint64_t *key, const int *perm, const double *kov, const double *kfac, i64 n,
-                           int *col, double *ov_sorted, double *fac_sorted, std::uint64_t *key2, int *vals2) {
+__global__ void k_count_keys(const unsigned *key, i64 n, int *cnt) {
     i64 k = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    unsigned long long kk = key[k];
-    unsigned i = static_cast<unsigned>(kk & 0xffffffffu);
-    unsigned j = static_cast<unsigned>(kk >> 32);
-    col[k] = static_cast<int>(i);
-    ov_sorted[k] = kov[perm[k]];
-    if (kfac) fac_sorted[k] = kfac[perm[k]];
-    key2[k] = (static_cast<unsigned long long>(i) << 32) | j;
-    vals2[k] = static_cast<int>(k);
+    if (k < n) atomicAdd(&cnt[key[k]], 1);
 }
 
-// Weights and frac_b per row (weight_generator.cpp:3684-3716); fb_pre, when
-// given, holds the row sums already taken in the generator's own order.
-__global__ void k_rows(const int *row_ptr, const double *ov, const double *area_dst, const double *fb_pre, i64 n_dst,
-                       int fracarea, double *w, double *frac_b) {
+// Per row: frac_b, the sum of overlap / area in column order, or fb_pre, the
+// row sums already taken in the generator's own order; weights clamped at 0
+// and divided by the row's fraction under FracArea.
+__global__ void k_rows(const int *row_ptr, const double *fb_pre, i64 n_dst, int fracarea, double *w, double *frac_b) {
     i64 j = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (j >= n_dst) return;
-    double ad = area_dst[j];
+    const int b = row_ptr[j], e = row_ptr[j + 1];
     double fb = 0.0;
-    for (int k = row_ptr[j]; k < row_ptr[j + 1]; ++k) {
-        double o = ov[k];
-        double wij = o / ad;
-        w[k] = fmax(wij, 0.0);
-        fb += o / ad;
+    for (int k = b; k < e; ++k) {
+        const double q = w[k];
+        if (!(q >= 0.0)) w[k] = fmax(q, 0.0);
+        fb += q;
     }
     if (fb_pre) fb = fb_pre[j];
     if (fracarea && fb > 0.0)
-        for (int k = row_ptr[j]; k < row_ptr[j + 1]; ++k) w[k] /= fb;
+        for (int k = b; k < e; ++k) w[k] /= fb;
     frac_b[j] = fmin(fb, 1.0);
 }
 
-// frac_a per source cell, contributions in ascending row order: ov / area,
-// or the per-pair contributions fac when the generator gives them.
-__global__ void k_cols(const int *col_ptr, const int *perm2, const double *ov, const double *fac,
-                       const double *area_src, i64 n_src, double *frac_a) {
+// frac_a per source cell, contributions in ascending row order.
+__global__ void k_cols(const int *col_ptr, const int *perm, const double *fa, i64 n_src, double *frac_a) {
     i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n_src) return;
-    double as = area_src[i];
-    double fa = 0.0;
-    for (int k = col_ptr[i]; k < col_ptr[i + 1]; ++k) fa += fac ? fac[perm2[k]] : ov[perm2[k]] / as;
-    frac_a[i] = fmin(fa, 1.0);
+    double s = 0.0;
+    for (int k = col_ptr[i]; k < col_ptr[i + 1]; ++k) s += fa[perm[k]];
+    frac_a[i] = fmin(s, 1.0);
 }
 
 __global__ void k_unmapped(MeshView D, const int *row_ptr, int *bad) {
@@ -795,67 +952,94 @@ struct AssembleOpts {
 // Kept pairs (overlap > 0, weight_generator.cpp:3682) of the candidate list
 // (cs, cd, ov) into the CSR of out: weights, frac_b per row and frac_a per
 // column (the steps of :3684-3724), areas copied from area_src / area_dst.
-static void assemble(DBuf<int> &cs, DBuf<int> &cd, DBuf<double> &ov, i64 n_cand, const double *area_src,
-                     const double *area_dst, const MeshView &D, const axgb_regrid_config &cfg, Matrix &out,
-                     cudaStream_t s, const AssembleOpts &o = AssembleOpts{}) {
+static void assemble(const int *cs, const int *cd, const double *ov, const i64 *offs, i64 n_cand,
+                     const double *area_src, const double *area_dst, const MeshView &D, const axgb_regrid_config &cfg,
+                     Matrix &out, cudaStream_t s, const AssembleOpts &o = AssembleOpts{}) {
     const i64 n_src = out.n_src, n_dst = out.n_dst;
-    DBuf<int> keep(n_cand);
-    DBuf<i64> pos(n_cand + 1);
-    i64 nnz = 0;
-    if (n_cand > 0) {
-        k_keep_flags<<<nblk(n_cand, 256), 256, 0, s>>>(ov.p, n_cand, keep.p);
-        scan_exclusive_i32_to_i64(keep.p, pos.p, n_cand, s);
-        AXGB_CUDA(cudaMemcpy(&nnz, pos.p + n_cand, sizeof(i64), cudaMemcpyDeviceToHost));
-    }
-    DBuf<std::uint64_t> key(nnz), key2(nnz);
-    DBuf<int> vals(nnz), vals2(nnz);
-    DBuf<double> kov(nnz), kfac(o.fac ? nnz : 0), facs(o.fac ? nnz : 0);
+    Scratch<int> kept(n_dst, s), ccnt(n_src, s), col_ptr(n_src + 1, s);
+    Scratch<unsigned long long> squares(1, s);
+    Scratch<double> rcp_src(o.fac ? 0 : n_src, s), rcp_dst(n_dst, s);
+    Scratch<int> key(n_cand, s);
+    squares.zero();
+    ccnt.zero();
+    kept.zero();
     out.row_ptr.alloc(n_dst + 1);
+    if (n_cand > 0) {
+        k_row_kept<<<nblk(n_cand, 256), 256, 0, s>>>(ov, cs, cd, n_cand, kept.p, key.p);
+        k_row_squares<<<nblk(n_dst, 256), 256, 0, s>>>(offs, n_dst, squares.p);
+        k_reciprocal<<<nblk(n_dst, 256), 256, 0, s>>>(area_dst, n_dst, rcp_dst.p);
+        if (!o.fac) k_reciprocal<<<nblk(n_src, 256), 256, 0, s>>>(area_src, n_src, rcp_src.p);
+    }
+    AXGB_CUDA(cudaGetLastError());
+    scan_exclusive_i32(kept.p, out.row_ptr.p, n_dst, s);
+    int h_nnz = 0;
+    unsigned long long h_squares = 0;
+    AXGB_CUDA(cudaMemcpyAsync(&h_nnz, out.row_ptr.p + n_dst, sizeof(int), cudaMemcpyDeviceToHost, s));
+    AXGB_CUDA(cudaMemcpyAsync(&h_squares, squares.p, sizeof(h_squares), cudaMemcpyDeviceToHost, s));
+    AXGB_CUDA(cudaStreamSynchronize(s));
+    const i64 nnz = h_nnz;
     out.col.alloc(nnz);
     out.val.alloc(nnz);
     out.frac_a.alloc(n_src);
     out.frac_b.alloc(n_dst);
     out.area_a.alloc(n_src);
     out.area_b.alloc(n_dst);
-    DBuf<double> ovs(nnz);
-    DBuf<int> rcnt(n_dst), ccnt(n_src), col_ptr(n_src + 1);
-    rcnt.zero(s);
-    ccnt.zero(s);
+    if (o.keep_gen) out.gen_rank.alloc(nnz);
+    Scratch<double> fa(nnz, s);
+    Scratch<unsigned> ckey(nnz, s);
+    Scratch<int> cval(nnz, s);
     if (nnz > 0) {
-        k_compact<<<nblk(n_cand, 256), 256, 0, s>>>(ov.p, o.fac, cs.p, cd.p, pos.p, n_cand, key.p, vals.p, kov.p,
-                                                    kfac.p);
-        int rbits = 32;
-        while (rbits < 64 && (static_cast<unsigned long long>(n_dst) >> (rbits - 32)) > 0) ++rbits;
-        radix_sort_pairs_u64(key.p, vals.p, nnz, rbits, s);
-        k_count_keys<<<nblk(nnz, 256), 256, 0, s>>>(key.p, nnz, rcnt.p);
-        k_csr_cols<<<nblk(nnz, 256), 256, 0, s>>>(key.p, vals.p, kov.p, o.fac ? kfac.p : nullptr, nnz, out.col.p,
-                                                  ovs.p, facs.p, key2.p, vals2.p);
+        EntryArgs a{};
+        a.ov = ov;
+        a.fac = o.fac;
+        a.cs = cs;
+        a.cd = cd;
+        a.area_src = area_src;
+        a.area_dst = area_dst;
+        a.rcp_src = rcp_src.p;
+        a.rcp_dst = rcp_dst.p;
+        a.row_ptr = out.row_ptr.p;
+        a.col = out.col.p;
+        a.w = out.val.p;
+        a.fa = fa.p;
+        a.ckey = ckey.p;
+        a.cval = cval.p;
+        a.gen = o.keep_gen ? out.gen_rank.p : nullptr;
+        if (h_squares <= static_cast<unsigned long long>(kRankWork * n_cand)) {
+            k_place<<<nblk(n_cand, 256), 256, 0, s>>>(a, offs, key.p, static_cast<int>(n_cand));
+        } else {
+            Scratch<int> keep(n_cand, s), vals(nnz, s), cand(nnz, s);
+            Scratch<i64> pos(n_cand + 1, s);
+            Scratch<std::uint64_t> rc(nnz, s);
+            k_keep_flags<<<nblk(n_cand, 256), 256, 0, s>>>(ov, n_cand, keep.p);
+            scan_exclusive_i32_to_i64(keep.p, pos.p, n_cand, s);
+            k_compact<<<nblk(n_cand, 256), 256, 0, s>>>(ov, cs, cd, pos.p, n_cand, rc.p, vals.p, cand.p);
+            int rbits = 32;
+            while (rbits < 64 && (static_cast<unsigned long long>(n_dst) >> (rbits - 32)) > 0) ++rbits;
+            radix_sort_pairs_u64(rc.p, vals.p, nnz, rbits, s);
+            k_write_sorted<<<nblk(nnz, 256), 256, 0, s>>>(a, vals.p, cand.p, nnz);
+        }
         AXGB_CUDA(cudaGetLastError());
-        int cbits = 32;
-        while (cbits < 64 && (static_cast<unsigned long long>(n_src) >> (cbits - 32)) > 0) ++cbits;
-        radix_sort_pairs_u64(key2.p, vals2.p, nnz, cbits, s);
-        k_count_keys<<<nblk(nnz, 256), 256, 0, s>>>(key2.p, nnz, ccnt.p);
+        // entries by column, rows ascending: the CSR order sorted stably by column
+        k_count_keys<<<nblk(nnz, 256), 256, 0, s>>>(ckey.p, nnz, ccnt.p);
+        int cbits = 1;
+        while (cbits < 32 && (static_cast<unsigned long long>(n_src) >> cbits) > 0) ++cbits;
+        radix_sort_pairs_u32(ckey.p, cval.p, nnz, cbits, s);
         AXGB_CUDA(cudaGetLastError());
-        // vals: each CSR entry's position in the compacted candidate list,
-        // which the fast paths fill row by row in the reference's loop order
-        if (o.keep_gen) out.gen_rank = std::move(vals);
     }
-    scan_exclusive_i32(rcnt.p, out.row_ptr.p, n_dst, s);
     scan_exclusive_i32(ccnt.p, col_ptr.p, n_src, s);
     AXGB_CUDA(cudaMemcpyAsync(out.area_a.p, o.area_a_out ? o.area_a_out : area_src, sizeof(double) * n_src,
                               cudaMemcpyDeviceToDevice, s));
     AXGB_CUDA(cudaMemcpyAsync(out.area_b.p, o.area_b_out ? o.area_b_out : area_dst, sizeof(double) * n_dst,
                               cudaMemcpyDeviceToDevice, s));
     if (n_dst > 0)
-        k_rows<<<nblk(n_dst, 256), 256, 0, s>>>(out.row_ptr.p, ovs.p, area_dst, o.fb_pre, n_dst,
-                                               cfg.norm_type == AXGB_FRACAREA ? 1 : 0, out.val.p, out.frac_b.p);
-    if (n_src > 0)
-        k_cols<<<nblk(n_src, 256), 256, 0, s>>>(col_ptr.p, vals2.p, ovs.p, o.fac ? facs.p : nullptr, area_src, n_src,
-                                               out.frac_a.p);
+        k_rows<<<nblk(n_dst, 256), 256, 0, s>>>(out.row_ptr.p, o.fb_pre, n_dst, cfg.norm_type == AXGB_FRACAREA ? 1 : 0,
+                                                out.val.p, out.frac_b.p);
+    if (n_src > 0) k_cols<<<nblk(n_src, 256), 256, 0, s>>>(col_ptr.p, cval.p, fa.p, n_src, out.frac_a.p);
     AXGB_CUDA(cudaGetLastError());
     if (o.check_unmapped && cfg.unmapped == AXGB_UNMAPPED_ERROR && n_dst > 0) {
-        DBuf<int> bad(1);
-        bad.zero(s);
+        Scratch<int> bad(1, s);
+        bad.zero();
         k_unmapped<<<nblk(n_dst, 256), 256, 0, s>>>(D, out.row_ptr.p, bad.p);
         int h_bad = 0;
         AXGB_CUDA(cudaMemcpy(&h_bad, bad.p, sizeof(int), cudaMemcpyDeviceToHost));
@@ -884,19 +1068,19 @@ void generate_conservative(Mesh &src, Mesh &dst, const axgb_regrid_config &cfg, 
     // 2. LBVH
     t0 = Clock::now();
     const int n = static_cast<int>(n_src);
-    DBuf<float4> nlo(n > 0 ? 2 * n - 1 : 1), nhi(n > 0 ? 2 * n - 1 : 1);
-    DBuf<int> parent(n > 0 ? 2 * n - 1 : 1), right(n > 1 ? n - 1 : 1), flag(n > 1 ? n - 1 : 1);
+    Scratch<float4> nlo(n > 0 ? 2 * n - 1 : 1, s), nhi(n > 0 ? 2 * n - 1 : 1, s);
+    Scratch<int> right(n > 1 ? n - 1 : 1, s);
     int root = -1;
     if (n > 0) {
-        DBuf<unsigned> keys(n);
-        DBuf<int> vals(n);
+        Scratch<unsigned> keys(n, s);
+        Scratch<int> vals(n, s), parent(2 * n - 1, s), flag(n > 1 ? n - 1 : 1, s);
         k_leaf_keys<<<nblk(n, 256), 256, 0, s>>>(S, keys.p, vals.p);
         AXGB_CUDA(cudaGetLastError());
         radix_sort_pairs_u32(keys.p, vals.p, n, 30, s);
         Bvh t{n, n > 1 ? 0 : 0, nlo.p, nhi.p, parent.p, right.p, flag.p, keys.p};
         root = 0;  // internal node 0, or the single leaf (index n-1 = 0)
         AXGB_CUDA(cudaMemsetAsync(parent.p, 0xff, sizeof(int) * (2 * n - 1), s));
-        flag.zero(s);
+        flag.zero();
         k_leaves<<<nblk(n, 256), 256, 0, s>>>(t, S, vals.p);
         if (n > 1) {
             k_internal<<<nblk(n - 1, 256), 256, 0, s>>>(t);
@@ -911,42 +1095,57 @@ void generate_conservative(Mesh &src, Mesh &dst, const axgb_regrid_config &cfg, 
 
     // 3. candidates
     t0 = Clock::now();
-    DBuf<int> counts(n_dst);
-    DBuf<i64> offs(n_dst + 1);
-    DBuf<unsigned long long> raw(1);
-    raw.zero(s);
+    Scratch<int> counts(n_dst, s);
+    Scratch<i64> offs(n_dst + 1, s);
+    Scratch<unsigned long long> raw(1, s);
+    Scratch<int> wide(n_dst, s), n_wide(2, s);  // n_wide[1]: error flag
+    raw.zero();
+    n_wide.zero();
     const int n_leaf_base = n > 0 ? n - 1 : 0;
-    DBuf<int> err(1);
-    err.zero(s);
-    k_search<false><<<nblk(n_dst, 128), 128, 0, s>>>(S, D, nlo.p, nhi.p, root, n_leaf_base, counts.p, nullptr,
-                                                    nullptr, raw.p, err.p);
+    // Two tilings of ns and nd cells meet in 1 + r^2 + 2.55 r pairs a row on
+    // average (r^2 = ns / nd), and the gates admit about 1.6 times as many; a
+    // row keeps up to 2.5 times that, at most 32 (longer ones go to
+    // k_search_wide) and 1 GiB in all.
+    const double r2 = n_dst > 0 ? static_cast<double>(n_src) / static_cast<double>(n_dst) : 0.0;
+    const double room = std::min(32.0, std::max(16.0, 2.5 * 1.6 * (1.0 + r2 + 2.55 * std::sqrt(r2))));
+    const int cap = static_cast<int>(std::max<i64>(1, std::min<i64>(static_cast<i64>(room),
+                                                                   (i64(1) << 28) / std::max<i64>(1, n_dst))));
+    Scratch<int> slots(cap * n_dst, s);
+    const unsigned wide_grid = nblk(std::min<i64>(n_dst, 152 * 8 * kWideWarps), kWideWarps);
+    if (n_dst > 0) {
+        k_search<<<nblk(n_dst, 128), 128, 0, s>>>(S, D, nlo.p, nhi.p, root, n_leaf_base, counts.p, slots.p, cap, wide.p,
+                                                 n_wide.p, raw.p);
+        k_search_wide<false><<<wide_grid, 32 * kWideWarps, 0, s>>>(S, D, nlo.p, nhi.p, right.p, root, n_leaf_base, wide.p,
+                                                                  n_wide.p, counts.p, nullptr, nullptr, raw.p, n_wide.p + 1);
+    }
     AXGB_CUDA(cudaGetLastError());
     scan_exclusive_i32_to_i64(counts.p, offs.p, n_dst, s);
     i64 n_cand = 0;
     unsigned long long n_raw = 0;
-    AXGB_CUDA(cudaMemcpy(&n_cand, offs.p + n_dst, sizeof(i64), cudaMemcpyDeviceToHost));
-    AXGB_CUDA(cudaMemcpy(&n_raw, raw.p, sizeof(n_raw), cudaMemcpyDeviceToHost));
+    AXGB_CUDA(cudaMemcpyAsync(&n_cand, offs.p + n_dst, sizeof(i64), cudaMemcpyDeviceToHost, s));
+    AXGB_CUDA(cudaMemcpyAsync(&n_raw, raw.p, sizeof(n_raw), cudaMemcpyDeviceToHost, s));
+    int h_err = 0;
+    AXGB_CUDA(cudaMemcpyAsync(&h_err, n_wide.p + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+    AXGB_CUDA(cudaStreamSynchronize(s));
+    if (h_err) throw Error(AXGB_ERROR, "LBVH traversal exceeded its step bound (malformed tree)");
     AXGB_REQUIRE(n_cand < (i64(1) << 31), "more than 2^31 candidate pairs");
-    DBuf<int> cs(n_cand), cd(n_cand);
+    Scratch<int> cs(n_cand, s), cd(n_cand, s);
     if (n_cand > 0) {
-        k_search<true><<<nblk(n_dst, 128), 128, 0, s>>>(S, D, nlo.p, nhi.p, root, n_leaf_base, nullptr, offs.p, cs.p,
-                                                       nullptr, err.p);
-        k_fill_rows<<<nblk(n_dst, 256), 256, 0, s>>>(offs.p, n_dst, cd.p);
+        k_take_slots<<<nblk(n_dst, 256), 256, 0, s>>>(counts.p, offs.p, slots.p, n_dst, cs.p, cd.p);
+        k_search_wide<true><<<wide_grid, 32 * kWideWarps, 0, s>>>(S, D, nlo.p, nhi.p, right.p, root, n_leaf_base, wide.p,
+                                                                 n_wide.p, nullptr, offs.p, cs.p, nullptr, n_wide.p + 1);
         AXGB_CUDA(cudaGetLastError());
     }
-    AXGB_CUDA(cudaStreamSynchronize(s));
-    int h_err = 0;
-    AXGB_CUDA(cudaMemcpy(&h_err, err.p, sizeof(int), cudaMemcpyDeviceToHost));
-    if (h_err) throw Error(AXGB_ERROR, "LBVH traversal exceeded its step bound (malformed tree)");
+    slots.release();
     out.stats[0] = static_cast<i64>(n_raw);
     out.stats[1] = n_cand;
     out.times_ms[2] = ms_since(t0);
 
     // 4. clip
     t0 = Clock::now();
-    DBuf<double> ov(n_cand);
-    DBuf<int> over_list(n_cand), n_over(1);
-    n_over.zero(s);
+    Scratch<double> ov(n_cand, s);
+    Scratch<int> over_list(n_cand, s), n_over(1, s);
+    n_over.zero();
     int h_over = 0;
     if (n_cand > 0) {
         k_clip_convex<<<nblk(n_cand, kClipT), kClipT, 0, s>>>(S, D, cs.p, cd.p, n_cand, ov.p, over_list.p, n_over.p);
@@ -963,7 +1162,7 @@ void generate_conservative(Mesh &src, Mesh &dst, const axgb_regrid_config &cfg, 
 
     // 5. assembly
     t0 = Clock::now();
-    assemble(cs, cd, ov, n_cand, S.area, D.area, D, cfg, out, s);
+    assemble(cs.p, cd.p, ov.p, offs.p, n_cand, S.area, D.area, D, cfg, out, s);
     out.times_ms[4] = ms_since(t0);
     out.times_ms[5] = ms_since(t_all);
     slice_centroids(D, out, s);  // locality hint for the blocked apply layout (not timed)
@@ -994,13 +1193,13 @@ bool generate_conservative_regular(Mesh &src, Mesh &dst, const axgb_regrid_confi
     a.n_dst = n_dst;
     a.smask = src.has_mask ? src.d_mask.p : nullptr;
     a.dmask = dst.has_mask ? dst.d_mask.p : nullptr;
-    DBuf<double> sa(n_src), da(n_dst);
+    Scratch<double> sa(n_src, s), da(n_dst, s);
     if (n_src) k_band_area<<<nblk(n_src, 256), 256, 0, s>>>(a.sg, src.has_area ? src.d_user_area.p : nullptr, n_src, sa.p);
     if (n_dst) k_band_area<<<nblk(n_dst, 256), 256, 0, s>>>(a.dg, dst.has_area ? dst.d_user_area.p : nullptr, n_dst, da.p);
     a.sa = sa.p;
     a.da = da.p;
-    DBuf<int> counts(n_dst);
-    DBuf<i64> offs(n_dst + 1);
+    Scratch<int> counts(n_dst, s);
+    Scratch<i64> offs(n_dst + 1, s);
     if (n_dst) k_rect<false><<<nblk(n_dst, 128), 128, 0, s>>>(a, counts.p, nullptr, nullptr, nullptr, nullptr, nullptr);
     AXGB_CUDA(cudaGetLastError());
     scan_exclusive_i32_to_i64(counts.p, offs.p, n_dst, s);
@@ -1008,9 +1207,9 @@ bool generate_conservative_regular(Mesh &src, Mesh &dst, const axgb_regrid_confi
     AXGB_CUDA(cudaMemcpy(&n_cand, offs.p + n_dst, sizeof(i64), cudaMemcpyDeviceToHost));
     AXGB_REQUIRE(n_cand < (i64(1) << 31), "more than 2^31 overlapping pairs");
     if (cfg.unmapped == AXGB_UNMAPPED_ERROR && n_cand == 0) return false;  // the general path diagnoses it
-    DBuf<int> cs(n_cand), cd(n_cand);
-    DBuf<double> ov(n_cand), fb(n_dst);
-    fb.zero(s);
+    Scratch<int> cs(n_cand, s), cd(n_cand, s);
+    Scratch<double> ov(n_cand, s), fb(n_dst, s);
+    fb.zero();
     if (n_cand) k_rect<true><<<nblk(n_dst, 128), 128, 0, s>>>(a, nullptr, offs.p, cs.p, cd.p, ov.p, fb.p);
     AXGB_CUDA(cudaGetLastError());
     out.stats[0] = out.stats[1] = n_cand;
@@ -1019,7 +1218,7 @@ bool generate_conservative_regular(Mesh &src, Mesh &dst, const axgb_regrid_confi
     o.keep_gen = true;  // rows generated in the reference's (js, is) loop order
     o.fb_pre = fb.p;
     o.check_unmapped = false;  // the fast path returns its matrix as it is (:380-415)
-    assemble(cs, cd, ov, n_cand, sa.p, da.p, D, cfg, out, s, o);
+    assemble(cs.p, cd.p, ov.p, offs.p, n_cand, sa.p, da.p, D, cfg, out, s, o);
     AXGB_CUDA(cudaStreamSynchronize(s));
     out.times_ms[4] = ms_since(t0);
     out.times_ms[5] = ms_since(t_all);
@@ -1055,8 +1254,8 @@ bool generate_conservative_rectilinear(Mesh &src, Mesh &dst, const axgb_regrid_c
     a.dmask = dst.has_mask ? dst.d_mask.p : nullptr;
     a.n_src = n_src;
     a.n_dst = n_dst;
-    DBuf<int> counts(n_dst);
-    DBuf<i64> offs(n_dst + 1);
+    Scratch<int> counts(n_dst, s);
+    Scratch<i64> offs(n_dst + 1, s);
     if (n_dst)
         k_rect_nu<false><<<nblk(n_dst, 128), 128, 0, s>>>(a, counts.p, nullptr, nullptr, nullptr, nullptr, nullptr,
                                                           nullptr, nullptr);
@@ -1067,8 +1266,8 @@ bool generate_conservative_rectilinear(Mesh &src, Mesh &dst, const axgb_regrid_c
     AXGB_REQUIRE(n_cand < (i64(1) << 31), "more than 2^31 overlapping pairs");
     // under UnmappedAction::Error an empty matrix goes on to the general path (weight_generator.cpp:3286-3295)
     if (n_dst == 0 || (cfg.unmapped == AXGB_UNMAPPED_ERROR && n_cand == 0)) return false;
-    DBuf<int> cs(n_cand), cd(n_cand);
-    DBuf<double> ov(n_cand), fac(n_cand), fb(n_dst), da_w(n_dst), sa(n_src), da(n_dst);
+    Scratch<int> cs(n_cand, s), cd(n_cand, s);
+    Scratch<double> ov(n_cand, s), fac(n_cand, s), fb(n_dst, s), da_w(n_dst, s), sa(n_src, s), da(n_dst, s);
     k_rect_nu<true><<<nblk(n_dst, 128), 128, 0, s>>>(a, nullptr, offs.p, cs.p, cd.p, ov.p, fac.p, fb.p, da_w.p);
     if (n_src) k_edge_area<<<nblk(n_src, 256), 256, 0, s>>>(a.sg, a.s_user, n_src, sa.p);
     k_edge_area<<<nblk(n_dst, 256), 256, 0, s>>>(a.dg, a.d_user, n_dst, da.p);
@@ -1081,7 +1280,7 @@ bool generate_conservative_rectilinear(Mesh &src, Mesh &dst, const axgb_regrid_c
     o.fb_pre = fb.p;
     o.area_b_out = da.p;
     o.check_unmapped = false;
-    assemble(cs, cd, ov, n_cand, sa.p, da_w.p, D, cfg, out, s, o);
+    assemble(cs.p, cd.p, ov.p, offs.p, n_cand, sa.p, da_w.p, D, cfg, out, s, o);
     AXGB_CUDA(cudaStreamSynchronize(s));
     out.times_ms[4] = ms_since(t0);
     out.times_ms[5] = ms_since(t_all);
@@ -1099,9 +1298,9 @@ bool generate_bilinear_regular(Mesh &src, Mesh &dst, const axgb_regrid_config &c
     AXGB_REQUIRE(4 * n_dst < (i64(1) << 31) && n_src < (i64(1) << 31), "bilinear: meshes too large");
     BilRegArgs a{g.lon_min, g.lat_min, g.dlon, g.dlat, static_cast<int>(g.ni), static_cast<int>(g.nj),
                  std::abs((g.lon_max - g.lon_min) - 360.0) < 1.0e-10 * g.dlon};
-    DBuf<int> cnt(n_dst), col4(4 * n_dst), gen4(4 * n_dst), bad(1);
-    DBuf<double> w4(4 * n_dst);
-    bad.zero(s);
+    Scratch<int> cnt(n_dst, s), col4(4 * n_dst, s), gen4(4 * n_dst, s), bad(1, s);
+    Scratch<double> w4(4 * n_dst, s);
+    bad.zero();
     k_bilinear_reg<<<nblk(n_dst, 128), 128, 0, s>>>(dst.view(), a, cnt.p, col4.p, w4.p, gen4.p, bad.p);
     AXGB_CUDA(cudaGetLastError());
     int h_bad = 0;

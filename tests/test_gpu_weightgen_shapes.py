@@ -43,3 +43,31 @@ def test_many_vertices_and_concave_cells(gpu, oracle, k, bulge, side):
     _check_weights(M, oracle.conservative(src, dst))
     if side == "src" and (bulge > 0.0 or 4 * k > 12):  # the source cell is the polygon that is cut
         assert M.stats()["fallback_clips"] > 0
+
+
+def _band(n_lon, lat_edges):
+    return grids.rectilinear(np.linspace(0.0, 360.0, n_lon + 1), lat_edges)
+
+
+@pytest.mark.parametrize("name,src,dst", [
+    # a few destination cells over thousands of source cells: every row is walked by a warp, the CSR order
+    # comes from the radix sort
+    ("coarse", lambda: grids.cubed_sphere(48), lambda: grids.latlon_deg(60.0)),
+    # rows of 1 to 720 candidates in one matrix (polar cells of a lat-lon source), direct placement
+    ("polar", lambda: _band(720, np.linspace(-90.0, 90.0, 181)), lambda: grids.cubed_sphere(90)),
+    # rows within one candidate of what a thread keeps, few cells
+    ("tiny", lambda: grids.cubed_sphere(5), lambda: grids.cubed_sphere(3)),
+    ("one", lambda: grids.cubed_sphere(4), lambda: grids.regular_latlon(1, 1, 10.0, -20.0, 30.0, 25.0)),
+])
+@pytest.mark.parametrize("norm", [0, 1])
+def test_search_and_placement_paths(gpu, oracle, name, src, dst, norm):
+    """Candidate search by threads and by warps, CSR placement by ranks and by
+    the radix sort, both normalisations."""
+    src, dst = src(), dst()
+    M = gpu.generate_weights(gpu.Mesh.from_grid(src), gpu.Mesh.from_grid(dst),
+                             {"method": "conservative", "norm_type": norm})
+    wo = oracle.conservative(src, dst, norm_type=norm)
+    _check_weights(M, wo)
+    st = M.stats()
+    assert st["gated_pairs"] == wo.stats["cap_pass"]
+

@@ -120,15 +120,43 @@ __device__ __forceinline__ DV3 d_arc_cross_fast(const DV3 &v1, const DV3 &v2, co
     return c;
 }
 
+// Ordered as doubles for values that are not negative and not NaN, without
+// the FP64 pipe.
+__device__ __forceinline__ bool d_less_pos(double a, double b) { return __double_as_longlong(a) < __double_as_longlong(b); }
+
+// The same point where its sign is known beforehand. d = n1 x (v1 x v2) =
+// v1 (n1.v2) - v2 (n1.v1): going into the half space (n1.v1 < 0 < n1.v2) both
+// factors are positive, so d is on the side of v1 + v2; coming out both are
+// negative, and -d is. For arcs under 120 degrees with both ends clear of the
+// plane.
+__device__ __forceinline__ DV3 d_arc_cross_known(const DV3 &v1, const DV3 &v2, const DV3 &n1, bool out) {
+    const DV3 d = d_cross(n1, d_cross(v1, v2));
+    const double l2 = d_lensq(d);
+    if (d_less_pos(l2, 1.0e-30)) return d_normalize(d_add(v1, v2));
+    const double inv = 1.0 / sqrt(l2);
+    const DV3 c{d.x * inv, d.y * inv, d.z * inv};
+    return out ? DV3{-c.x, -c.y, -c.z} : c;
+}
+
 // 2 atan2(num, den) for the small triangles that cells are cut into: up to
 // num / den = 2^-7 by Gregory's series to the ninth power (the next term is
 // below 2^-73 of the first), so the error is the quotient's rounding and the
-// last addition's. Larger ones by atan2.
+// last addition's. The quotient: a float reciprocal, two Newton steps (each
+// doubles its 23 bits), one correction with the exact residual. Larger
+// angles by atan2.
 __device__ __forceinline__ double d_twice_atan(double num, double den) {
-    if (!(fabs(num) <= 0.0078125 * den)) return 2.0 * atan2(num, den);
-    const double t = num / den, q = t * t;
-    const double r = __fma_rn(q, __fma_rn(q, __fma_rn(q, 1.0 / 9.0, -1.0 / 7.0), 1.0 / 5.0), -1.0 / 3.0);
-    return 2.0 * __fma_rn(t * q, r, t);
+    if (static_cast<unsigned>(__double2hiint(den) - 0x3fe00000) < 0x00500000u) {  // 1/2 <= den < 16
+        double y = static_cast<double>(__frcp_rn(static_cast<float>(den)));
+        y = __fma_rn(__fma_rn(-den, y, 1.0), y, y);
+        y = __fma_rn(__fma_rn(-den, y, 1.0), y, y);
+        const double q0 = __dmul_rn(num, y);
+        const double t = __fma_rn(__fma_rn(-den, q0, num), y, q0), q = t * t;
+        if ((__double2hiint(t) & 0x7fffffff) < 0x3f800000) {  // |t| < 2^-7
+            const double r = __fma_rn(q, __fma_rn(q, __fma_rn(q, 1.0 / 9.0, -1.0 / 7.0), 1.0 / 5.0), -1.0 / 3.0);
+            return 2.0 * __fma_rn(t * q, r, t);
+        }
+    }
+    return 2.0 * atan2(num, den);
 }
 
 // Clip `subject` by every edge of `clip` (Sutherland-Hodgman on great

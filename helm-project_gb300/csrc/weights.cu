@@ -13,13 +13,14 @@
 //      area > 0, the reference's float AABB test, the FP64 cap test) and is
 //      kept, grouped by row in traversal order, so the candidate list is
 //      deterministic;
-//   4. one thread per candidate runs the FP64 great-circle clip and the
-//      spherical area (geom.cuh, --fmad=false); pairs whose polygons
-//      exceed 16 vertices are redone with the reference's 32-vertex cap;
-//   5. kept pairs (overlap > 0, the reference threshold at :3682) are
-//      compacted, radix-sorted by (row, col) into CSR, and the weights,
+//   4. pairs that an edge separates are settled in FP32; for the others one
+//      thread runs the FP64 great-circle clip and the spherical area
+//      (geom.cuh, --fmad=false), pairs that are not convex or exceed 12
+//      vertices with the reference's 32-vertex general clipper;
+//   5. kept pairs (overlap > 0, the reference threshold at :3682) are placed
+//      in CSR by their rank in the row (long rows: radix sort), and the weights,
 //      frac_b (row order) and frac_a (column order, rows ascending) sums are
-//      formed per row / per column by one thread each.
+//      formed.
 // Bilinear with a rectilinear source replaces
 // generate_bilinear_rect_nonuniform
 // (src/solver/weight_generator_bilinear_rect_nonuniform.cpp:22-149).
@@ -328,86 +329,218 @@ struct CellRef {
     }
 };
 
-// Overlap areas of candidate pairs, a thread each: d_overlap_area for convex
+// What decides most side tests in FP32: per connectivity entry of the
+// destination, the unit normal of the edge from that vertex to the next (w:
+// below 0, an edge that is skipped; else the margin), and per entry of the
+// source its vertex. The clipper's test is d = fl(n.p) >= -1e-14 in FP64 with
+// n = ea x eb; the float value is off from n.p / |n| by less than 6e-7, so
+// beyond kSideMargin it has the sign of d and, with |n| > 1e-7, d is clear of
+// -1e-14. Shorter edges have an infinite margin: every test in FP64.
+constexpr float kSideMargin = 2.0e-6f;
+
+__global__ void k_edge_normals(MeshView D, float4 *en) {
+    const int c = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+    if (c >= D.n_cells) return;
+    const CellRef E(D, c);
+    const int b = D.off[c];
+    if (E.n < 1) return;
+    const DV3 first = E.at(D, 0);
+    DV3 ea = first;
+    for (int k = 0; k < E.n; ++k) {
+        const DV3 eb = k + 1 == E.n ? first : E.at(D, k + 1);
+        const DV3 n = d_cross(ea, eb);
+        const double l2 = d_lensq(n), inv = rsqrt(l2);
+        const float w = l2 < 1.0e-30 ? -1.0f : l2 < 1.0e-14 ? INFINITY : kSideMargin;
+        en[b + k] = make_float4(static_cast<float>(n.x * inv), static_cast<float>(n.y * inv),
+                                static_cast<float>(n.z * inv), w);
+        ea = eb;
+    }
+}
+
+__global__ void k_vertices_f(MeshView S, float4 *vf) {
+    const int c = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+    if (c >= S.n_cells) return;
+    const CellRef C(S, c);
+    const int b = S.off[c];
+    for (int k = 0; k < C.n; ++k) {
+        const DV3 p = C.at(S, k);
+        vf[b + k] = make_float4(static_cast<float>(p.x), static_cast<float>(p.y), static_cast<float>(p.z), 0.0f);
+    }
+}
+
+__device__ __forceinline__ float side_f(const float4 &n, float x, float y, float z) {
+    return fmaf(n.x, x, fmaf(n.y, y, n.z * z));
+}
+
+// Pairs that an edge of the destination cell separates are settled here: all
+// vertices of the source cell are outside it, and so is every point the
+// clipper can put on an arc between them, so its polygon ends there with
+// overlap 0. The others are listed for the clipper, whose warps are then full
+// (two fifths of the candidates of 0.25 deg -> C384 are such pairs). The list's
+// order varies; the overlaps do not depend on it.
+__global__ void k_separate(MeshView S, MeshView D, const float4 *__restrict__ en, const float4 *__restrict__ vf,
+                           const int *__restrict__ cs, const int *__restrict__ cd, i64 n, double *ov, int *list,
+                           int *n_list) {
+    const i64 k = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
+    bool meet = false;
+    if (k < n) {
+        const int c = cs[k], d = cd[k];
+        const int sb = S.off[c], ns = min(32, S.off[c + 1] - sb), db = D.off[d], nd = min(32, D.off[d + 1] - db);
+        meet = ns >= 3 && nd >= 3;
+        for (int e = 0; e < nd && meet; ++e) {
+            const float4 nf = en[db + e];
+            if (nf.w < 0.0f) continue;
+            bool outside = true;
+            for (int i = 0; i < ns && outside; ++i) {
+                const float4 p = vf[sb + i];
+                outside = side_f(nf, p.x, p.y, p.z) < -nf.w;
+            }
+            meet = !outside;
+        }
+        if (!meet) ov[k] = 0.0;
+    }
+    const unsigned who = __ballot_sync(0xffffffffu, meet);
+    const int lane = threadIdx.x & 31;
+    int at = 0;
+    if (lane == 0 && who) at = atomicAdd(n_list, __popc(who));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (meet) list[at + __popc(who & ((1u << lane) - 1u))] = static_cast<int>(k);
+}
+
+// Overlap areas of the listed pairs, a thread each: d_overlap_area for convex
 // cells. A half space cuts a convex polygon in at most one run of vertices,
 // so an edge of the clip cell has at most one crossing into and one out of
-// it: the side tests come first, then both crossings in straight-line code,
-// once an edge for the whole warp. (In the vertex loop of d_overlap_area some
-// lane of a warp has a crossing at nearly every vertex, and all of them pay.)
-// The polygon stays in shared memory, a column a thread: a lane's vertex index
-// does not change its bank. Pairs with more crossings or more than kClipCap
-// vertices go to the general kernel through over_list.
-// Bound by the FP64 pipe. 0.25 deg -> C384, 6.9 M candidates: 10.3 ms, against
-// 24.2 ms with the loop, its polygons in local memory, normalised midpoints
-// and atan2.
-constexpr int kClipCap = 12, kClipT = 128;
-__global__ void __launch_bounds__(kClipT) k_clip_convex(MeshView S, MeshView D, const int *__restrict__ cs,
-                                                        const int *__restrict__ cd, i64 n, double *ov, int *over_list,
-                                                        int *n_over) {
+// it. Each lane goes on to its next edge that cuts (side tests, FP32), then
+// the warp forms both crossings of all its lanes together in straight-line
+// code. (In the vertex loop of d_overlap_area some lane of a warp has a
+// crossing at nearly every vertex, and all of them pay.) The polygon stays in
+// shared memory, a column a thread: a lane's vertex index does not change its
+// bank. Pairs with more crossings or more than kClipCap vertices go to the
+// general kernel through over_list.
+// Bound by the FP64 pipe, which takes a warp's instruction in 64 cycles
+// however many lanes are active; comparisons are made on the bits. 0.25 deg ->
+// C384, 6.9 M candidates: 4.3 ms with k_separate; 10.2 ms with the side
+// tests in FP64, edge by edge, on all candidates; 24.2 ms with the vertex
+// loop, polygons in local memory, normalised midpoints and atan2.
+constexpr int kClipCap = 12, kClipT = 64;
+__global__ void __launch_bounds__(kClipT) k_clip_convex(MeshView S, MeshView D, const float4 *__restrict__ en,
+                                                        const float4 *__restrict__ vf, const int *__restrict__ cs,
+                                                        const int *__restrict__ cd, const int *__restrict__ list,
+                                                        const int *n_list, double *ov, int *over_list, int *n_over) {
     __shared__ double P[3 * kClipCap][kClipT];
-    const int tid = threadIdx.x;
-    const i64 k = static_cast<i64>(blockIdx.x) * kClipT + tid;
-    if (k >= n) return;
-    const CellRef C(S, cs[k]), E(D, cd[k]);
+    __shared__ float F[3 * kClipCap][kClipT];
+    const int n = *n_list;
+    if (blockIdx.x * kClipT >= n) return;
+    const int tid = threadIdx.x, t = static_cast<int>(blockIdx.x) * kClipT + tid;
+    const int k = list[min(t, n - 1)];
     auto get = [&](int i) { return DV3{P[3 * i][tid], P[3 * i + 1][tid], P[3 * i + 2][tid]}; };
     auto put = [&](int i, const DV3 &v) {
         P[3 * i][tid] = v.x;
         P[3 * i + 1][tid] = v.y;
         P[3 * i + 2][tid] = v.z;
     };
-    bool over = C.n > kClipCap;
-    int m = over || C.n < 3 || E.n < 3 ? 0 : C.n;
-    for (int i = 0; i < m; ++i) put(i, C.at(S, i));
-    if (m > 0) {
-        constexpr double eps = -1.0e-14;
-        const DV3 first = E.at(D, 0);
-        DV3 ea = first;
-        for (int ci = 0; ci < E.n; ++ci) {
-            const DV3 eb = ci + 1 == E.n ? first : E.at(D, ci + 1);
-            const DV3 nrm = d_cross(ea, eb);
-            ea = eb;
-            if (d_lensq(nrm) < 1.0e-30) continue;
-            unsigned in = 0;
-            for (int i = 0; i < m; ++i)
-                if (d_dot(nrm, get(i)) >= eps) in |= 1u << i;
-            const unsigned all = (1u << m) - 1u;
-            if (in == all) continue;
-            if (in == 0) {
-                m = 0;
-                break;
-            }
-            const unsigned prev = ((in << 1) | (in >> (m - 1))) & all;  // bit i: vertex before i inside
-            const unsigned enter = in & ~prev, leave = ~in & prev;
-            const int kept = __popc(in);
-            if (__popc(enter) > 1 || kept + 2 > kClipCap) {
-                over = true;
-                break;
-            }
-            const int a = __ffs(enter) - 1, b = __ffs(leave) - 1;
-            const DV3 xa = d_arc_cross_fast(get(a == 0 ? m - 1 : a - 1), get(a), nrm);
-            const DV3 xb = d_arc_cross_fast(get(b == 0 ? m - 1 : b - 1), get(b), nrm);
-            // in vertex order: xa before vertex a, xb in place of vertex b
-            if (a < b) {  // xa, [a, b), xb
-                if (a == 0)
-                    for (int i = kept - 1; i >= 0; --i) put(i + 1, get(i));
-                else if (a > 1)
-                    for (int i = 0; i < kept; ++i) put(i + 1, get(a + i));
-                put(0, xa);
-                put(kept + 1, xb);
-            } else {  // the run passes the end: [0, b), xb, xa, [a, m)
-                const int tail = m - a;
-                if (a < b + 2)
-                    for (int i = tail - 1; i >= 0; --i) put(b + 2 + i, get(a + i));
-                else if (a > b + 2)
-                    for (int i = 0; i < tail; ++i) put(b + 2 + i, get(a + i));
-                put(b, xb);
-                put(b + 1, xa);
-            }
-            m = kept + 2;
+    auto putf = [&](int i, float x, float y, float z) {
+        F[3 * i][tid] = x;
+        F[3 * i + 1][tid] = y;
+        F[3 * i + 2][tid] = z;
+    };
+    auto move = [&](int to, int from) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            P[3 * to + q][tid] = P[3 * from + q][tid];
+            F[3 * to + q][tid] = F[3 * from + q][tid];
         }
+    };
+    const int c = cs[k];
+    const CellRef C(S, c), E(D, cd[k]);
+    const int sb = S.off[c], db = D.off[cd[k]];
+    const bool small = S.capf[c].w < 1.0f;  // no arc of the source cell reaches 120 degrees
+    bool over = C.n > kClipCap;
+    int m = t >= n || over ? 0 : C.n;
+    for (int i = 0; i < m; ++i) {
+        put(i, C.at(S, i));
+        const float4 p = vf[sb + i];
+        putf(i, p.x, p.y, p.z);
     }
+    int e = m > 0 ? 0 : E.n;
+    while (true) {
+        bool cut = false, unsure = false;
+        unsigned in = 0;
+        while (e < E.n) {  // the next edge that cuts
+            const float4 nf = en[db + e];
+            if (nf.w >= 0.0f) {
+                in = 0;
+                unsure = !small;
+                for (int i = 0; i < m; ++i) {
+                    const float f = side_f(nf, F[3 * i][tid], F[3 * i + 1][tid], F[3 * i + 2][tid]);
+                    bool inside = f > 0.0f;
+                    if (fabsf(f) <= nf.w) {
+                        unsure = true;
+                        inside = d_dot(d_cross(E.at(D, e), E.at(D, e + 1 == E.n ? 0 : e + 1)), get(i)) >= -1.0e-14;
+                    }
+                    in |= inside ? 1u << i : 0u;
+                }
+                if (in == 0) {
+                    m = 0;
+                    e = E.n;
+                    break;
+                }
+                if (in != (1u << m) - 1u) {
+                    cut = true;
+                    break;
+                }
+            }
+            ++e;
+        }
+        if (!__any_sync(0xffffffffu, cut)) break;
+        if (!cut) continue;
+        const unsigned all = (1u << m) - 1u;
+        const unsigned prev = ((in << 1) | (in >> (m - 1))) & all;  // bit i: vertex before i inside
+        const unsigned enter = in & ~prev, leave = ~in & prev;
+        const int kept = __popc(in);
+        if (__popc(enter) > 1 || kept + 2 > kClipCap) {
+            over = true;
+            m = 0;
+            e = E.n;
+            continue;
+        }
+        const DV3 nrm = d_cross(E.at(D, e), E.at(D, e + 1 == E.n ? 0 : e + 1));
+        const int a = __ffs(enter) - 1, b = __ffs(leave) - 1;
+        const DV3 a0 = get(a == 0 ? m - 1 : a - 1), a1 = get(a), b0 = get(b == 0 ? m - 1 : b - 1), b1 = get(b);
+        DV3 xa, xb;
+        if (unsure) {
+            xa = d_arc_cross_fast(a0, a1, nrm);
+            xb = d_arc_cross_fast(b0, b1, nrm);
+        } else {
+            xa = d_arc_cross_known(a0, a1, nrm, false);
+            xb = d_arc_cross_known(b0, b1, nrm, true);
+        }
+        // in vertex order: xa before vertex a, xb in place of vertex b
+        int ia = 0, ib = kept + 1;
+        if (a < b) {  // xa, [a, b), xb
+            if (a == 0)
+                for (int i = kept - 1; i >= 0; --i) move(i + 1, i);
+            else if (a > 1)
+                for (int i = 0; i < kept; ++i) move(i + 1, a + i);
+        } else {  // the run passes the end: [0, b), xb, xa, [a, m)
+            const int tail = m - a;
+            if (a < b + 2)
+                for (int i = tail - 1; i >= 0; --i) move(b + 2 + i, a + i);
+            else if (a > b + 2)
+                for (int i = 0; i < tail; ++i) move(b + 2 + i, a + i);
+            ib = b;
+            ia = b + 1;
+        }
+        put(ia, xa);
+        putf(ia, static_cast<float>(xa.x), static_cast<float>(xa.y), static_cast<float>(xa.z));
+        put(ib, xb);
+        putf(ib, static_cast<float>(xb.x), static_cast<float>(xb.y), static_cast<float>(xb.z));
+        m = kept + 2;
+        ++e;
+    }
+    if (t >= n) return;
     if (over) {
-        over_list[atomicAdd(n_over, 1)] = static_cast<int>(k);
+        over_list[atomicAdd(n_over, 1)] = k;
         ov[k] = 0.0;
         return;
     }
@@ -1144,11 +1277,17 @@ void generate_conservative(Mesh &src, Mesh &dst, const axgb_regrid_config &cfg, 
     // 4. clip
     t0 = Clock::now();
     Scratch<double> ov(n_cand, s);
-    Scratch<int> over_list(n_cand, s), n_over(1, s);
+    Scratch<int> over_list(n_cand, s), n_over(2, s);  // n_over[1]: pairs for the clipper
     n_over.zero();
     int h_over = 0;
     if (n_cand > 0) {
-        k_clip_convex<<<nblk(n_cand, kClipT), kClipT, 0, s>>>(S, D, cs.p, cd.p, n_cand, ov.p, over_list.p, n_over.p);
+        Scratch<float4> en(dst.n_conn, s), vf(src.n_conn, s);
+        Scratch<int> list(n_cand, s);
+        k_edge_normals<<<nblk(n_dst, 128), 128, 0, s>>>(D, en.p);
+        k_vertices_f<<<nblk(n_src, 128), 128, 0, s>>>(S, vf.p);
+        k_separate<<<nblk(n_cand, 256), 256, 0, s>>>(S, D, en.p, vf.p, cs.p, cd.p, n_cand, ov.p, list.p, n_over.p + 1);
+        k_clip_convex<<<nblk(n_cand, kClipT), kClipT, 0, s>>>(S, D, en.p, vf.p, cs.p, cd.p, list.p, n_over.p + 1, ov.p,
+                                                             over_list.p, n_over.p);
         AXGB_CUDA(cudaGetLastError());
         AXGB_CUDA(cudaMemcpy(&h_over, n_over.p, sizeof(int), cudaMemcpyDeviceToHost));
         if (h_over > 0) {

@@ -71,3 +71,20 @@ def test_search_and_placement_paths(gpu, oracle, name, src, dst, norm):
     st = M.stats()
     assert st["gated_pairs"] == wo.stats["cap_pass"]
 
+
+@pytest.mark.parametrize("name,src,dst", [
+    # edges along the same great circles: vertices on the edges they are tested against
+    ("aligned", lambda: grids.cubed_sphere(16), lambda: grids.cubed_sphere(8)),
+    # edges of 1e-8 radian, where no FP32 side test decides
+    ("tiny_cells", lambda: _subdivided(grids.rectilinear(10.0 + 6e-7 * np.arange(9), 20.0 + 6e-7 * np.arange(8)), 2),
+     lambda: _subdivided(grids.rectilinear(10.0 + 7.1e-7 * np.arange(6), 20.0 + 5.3e-7 * np.arange(7)), 2)),
+    # cells with caps of more than a radian on either side
+    ("huge_src", lambda: grids.rectilinear(np.linspace(0.0, 360.0, 4), np.array([-90.0, -10.0, 90.0])),
+     lambda: grids.cubed_sphere(6)),
+    ("huge_dst", lambda: grids.cubed_sphere(6),
+     lambda: grids.rectilinear(np.linspace(0.0, 360.0, 4), np.array([-90.0, -10.0, 90.0]))),
+])
+def test_side_tests_at_their_limits(gpu, oracle, name, src, dst):
+    src, dst = src(), dst()
+    M = gpu.generate_weights(gpu.Mesh.from_grid(src), gpu.Mesh.from_grid(dst), {"method": "conservative"})
+    _check_weights(M, oracle.conservative(src, dst))

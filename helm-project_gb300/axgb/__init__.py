@@ -301,13 +301,13 @@ class Matrix:
         self.n_src, self.n_dst, self.nnz = a.value, b.value, c.value
 
     def to_csr(self):
-        rp = np.zeros(self.n_dst + 1, np.int64)
-        col = np.zeros(self.nnz, np.int64)
-        val = np.zeros(self.nnz)
-        fa = np.zeros(self.n_src)
-        fb = np.zeros(self.n_dst)
-        aa = np.zeros(self.n_src)
-        ab = np.zeros(self.n_dst)
+        rp = np.empty(self.n_dst + 1, np.int64)
+        col = np.empty(self.nnz, np.int64)
+        val = np.empty(self.nnz)
+        fa = np.empty(self.n_src)
+        fb = np.empty(self.n_dst)
+        aa = np.empty(self.n_src)
+        ab = np.empty(self.n_dst)
         _check(lib().axgb_matrix_export_csr(self.handle, _ptr(rp), _ptr(col), _ptr(val), _ptr(fa), _ptr(fb),
                                             _ptr(aa), _ptr(ab)))
         return dict(row_ptr=rp, col=col, val=val, frac_a=fa, frac_b=fb, area_a=aa, area_b=ab)

@@ -88,3 +88,23 @@ def test_side_tests_at_their_limits(gpu, oracle, name, src, dst):
     src, dst = src(), dst()
     M = gpu.generate_weights(gpu.Mesh.from_grid(src), gpu.Mesh.from_grid(dst), {"method": "conservative"})
     _check_weights(M, oracle.conservative(src, dst))
+
+
+@pytest.mark.parametrize("nnz", [0, 10, 65536, 65537, 131072, 131073, 1048577])
+def test_export_round_trip(gpu, nnz):
+    """CSR export below and above the size from which threads move it, at the
+    ends of their pieces (131,072 indices, 65,536 values), twice into arrays
+    that hold something else."""
+    rng = np.random.default_rng(nnz)
+    n_dst, n_src = max(1, nnz // 7), 1000 + nnz // 3
+    lens = np.bincount(rng.integers(0, n_dst, nnz), minlength=n_dst)
+    rp = np.concatenate([[0], np.cumsum(lens)])
+    col = rng.integers(0, n_src, nnz)
+    row = np.repeat(np.arange(n_dst), lens)
+    col = col[np.lexsort((col, row))]
+    val, fa, fb, aa, ab = (rng.standard_normal(n) for n in (nnz, n_src, n_dst, n_src, n_dst))
+    M = gpu.Matrix.from_csr(n_src, n_dst, rp, col, val, fa, fb, aa, ab)
+    for _ in range(2):
+        c = M.to_csr()
+        for k, v in dict(row_ptr=rp, col=col, val=val, frac_a=fa, frac_b=fb, area_a=aa, area_b=ab).items():
+            assert np.array_equal(c[k], v), k

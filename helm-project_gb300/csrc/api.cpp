@@ -506,44 +506,57 @@ void host_batch(Matrix &m, const T *src, T *dst, int64_t n_vars, F apply_fn) {
     AXGB_CUDA(cudaStreamSynchronize(st.d2h));
 }
 
-SplitParams default_split_params(const Matrix &m, i64 nrhs);
-SplitParams pick_params(Matrix &m, i64 nrhs) {
-    std::lock_guard<std::mutex> lk(m.mu);
-    auto it = m.tuned.find(nrhs);
-    if (it != m.tuned.end()) return it->second;
-    return default_split_params(m, nrhs);
-}
-
-// Fields per work item of the staged kernels: 128 where that leaves about
-// two waves of work items (a block of 128 rows and the item's fields; four to
-// six CTAs fit an SM), fewer on smaller matrices, down to four tiles of four.
+// Fields per work item of the staged kernels: at most 128, and few enough
+// that there are about 3600 items (a block of 128 rows and the item's fields),
+// down to 16, in chunks of equal size. 64 fields of C192 -> 0.5 deg: 61 us with
+// 32, 71 with 64; 300 of C96 -> 1 deg: 68 us with 32, 85 with 128; 300 of C384 ->
+// 0.25 deg: 819 us with 128, 934 with 32.
 int default_item_fields(const Matrix &m, i64 nrhs) {
-    const i64 blocks = std::max<i64>(1, (m.n_dst + 127) / 128), items = 152 * 6 * 2;
-    const i64 f = (blocks * nrhs / items + 3) / 4 * 4;
-    return static_cast<int>(std::min<i64>(128, std::max<i64>(16, f)));
+    const i64 blocks = std::max<i64>(1, (m.n_dst + 127) / 128);
+    const i64 most = std::min<i64>(128, std::max<i64>(16, blocks * nrhs / 3600));
+    const i64 chunks = (nrhs + most - 1) / most;
+    return static_cast<int>(((nrhs + chunks - 1) / chunks + 3) / 4 * 4);
 }
 
+// The direct kernel, one launch that reads the sources from L1 and L2, or the
+// staged kernels, which read them once a block of rows but are a launch for
+// each row-length class, with events around them. The direct one costs about
+// 0.45 us more per million (entry, field) and 2 to 4 us less per launch of the
+// other: it is taken up to 4 million (entry, field) per staged launch, and
+// for one or two fields always. Direct against staged: 16 fields of C96 -> 1
+// deg 10.4 against 17.5 us, 4 of C384 -> 0.25 deg 38.8 against 32.2; 16 of 0.5
+// deg -> C192 (ten launches) 31.8 against 44.3, 64 of it 117.8 against 113.7.
 SplitParams default_split_params(const Matrix &m, i64 nrhs) {
     SplitParams p;
-    if (nrhs <= 2) {  // one fused launch
+    const i64 launches = m.blocked.built ? split_launches(m) : 3;
+    if (nrhs <= 2 || m.nnz * nrhs <= i64(4000000) * launches) {
         p.variant = 4;
         p.fields_per_pass = 0;
         p.unroll = 1;
         p.stages = 2;
         return p;
     }
+    p.unroll = 4;
+    p.fields_per_pass = default_item_fields(m, nrhs);
     if (nrhs >= 8) {  // producer-warp staged kernel, ring depth per row-length class
         p.variant = 3;
-        p.fields_per_pass = default_item_fields(m, nrhs);
         p.stages = 0;
-        p.unroll = 4;
         return p;
     }
     p.variant = 1;
-    p.fields_per_pass = 64;
     p.stages = 2;
-    p.unroll = 4;
     return p;
+}
+
+// The cached choice, or the default (the layout it depends on is built first).
+SplitParams pick_params(Matrix &m, i64 nrhs, cudaStream_t s) {
+    {
+        std::lock_guard<std::mutex> lk(m.mu);
+        auto it = m.tuned.find(nrhs);
+        if (it != m.tuned.end()) return it->second;
+    }
+    if (!m.blocked.built) matrix_prepare(m, 2, s);
+    return default_split_params(m, nrhs);
 }
 
 }  // namespace
@@ -1212,7 +1225,7 @@ int axgb_apply_f32split(int h, const float *x, int64_t ldx, float *y, int64_t ld
                 m->tuned[nrhs] = p;
                 have = true;
             }
-            if (!have) p = default_split_params(*m, nrhs);
+            if (!have) p = pick_params(*m, nrhs, s);
             apply_split(*m, x, ldx, y, ldy, nrhs, p, s);
         }
     });
@@ -1225,8 +1238,9 @@ int axgb_apply_f32split_hilo(int h, const float *x, int64_t ldx, float *y, int64
         check_apply(*m, x, ldx, y, ldy, nrhs);
         AXGB_REQUIRE(nrhs == 0 || m->n_dst == 0 || y_lo != nullptr, "apply_hilo: y_lo is NULL");
         AXGB_REQUIRE(nrhs == 0 || ld_lo >= m->n_dst, "apply_hilo: ld_lo < n_dst");
-        if (nrhs > 0) apply_split(*m, x, ldx, y, ldy, nrhs, pick_params(*m, nrhs), static_cast<cudaStream_t>(stream),
-                                  y_lo, ld_lo);
+        if (nrhs > 0) apply_split(*m, x, ldx, y, ldy, nrhs,
+                                  pick_params(*m, nrhs, static_cast<cudaStream_t>(stream)),
+                                  static_cast<cudaStream_t>(stream), y_lo, ld_lo);
     });
 }
 
@@ -1299,7 +1313,7 @@ int axgb_batch_apply_host_f32split(int h, const float *src, int64_t n_src, float
         if (n_vars > 0)
             host_batch<float>(*m, src, dst, n_vars,
                               [&](const float *x, int64_t lx, float *y, int64_t ly, int64_t nv, cudaStream_t s) {
-                                  apply_split(*m, x, lx, y, ly, nv, pick_params(*m, nv), s);
+                                  apply_split(*m, x, lx, y, ly, nv, pick_params(*m, nv, s), s);
                               });
     });
 }

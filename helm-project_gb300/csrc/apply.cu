@@ -47,9 +47,9 @@ struct Batch {
     // entries (lane per leaf, items = 8-field chunk x row).
     struct Desc {
         const int *base, *len, *rlen, *col;
-        const float *hi, *lo;
+        const float2 *hl;
         const int *lrow, *lptr, *lcol;  // mode 2: row-contiguous long rows
-        const float *lhi, *llo;
+        const float2 *lhl;
         const int *ids;  // slice ids (modes 0, 1)
         i64 n_ids;       // slices (modes 0, 1) or long rows (mode 2)
         int mode;
@@ -121,7 +121,7 @@ struct SellArgs {
     const int *ids;
     i64 n_ids;
     const int *base, *len, *rlen, *col;
-    const float *hi, *lo;
+    const float2 *hl;  // (hi, lo)
     const double *w64;
     i64 n_rows;
     float *ylo;  // split kernels: low parts of the outputs (hi+lo form), or null
@@ -130,159 +130,26 @@ struct SellArgs {
 
 __device__ __forceinline__ float ldg_f(const float *p) { return __ldg(p); }
 
-// ─── split-FP32 kernel ─────────────────────────────────────────────────────
-// Lane per row for slices whose rows have at most L <= 32 entries, entries
-// cached in registers (longer rows: k_split_rows).
-template <int L, int U>
-__global__ void __launch_bounds__(256) k_split(SellArgs a, const float *__restrict__ x, i64 ldx, float *__restrict__ y,
-                                               i64 ldy, i64 nrhs, i64 tile) {
-    const int lane = threadIdx.x & 31;
-    const i64 item = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const i64 n_tiles = (nrhs + tile - 1) / tile;
-    if (item >= n_tiles * a.n_ids) return;
-    const i64 t = item / a.n_ids;
-    const int sid = a.ids[item - t * a.n_ids];
-    const i64 row = static_cast<i64>(sid) * 32 + lane;
-    const int base = a.base[sid];
-    const int rl = a.rlen[static_cast<i64>(sid) * 32 + lane];
-    const i64 f0 = t * tile, f1 = min(f0 + tile, nrhs);
-    const bool store = row < a.n_rows;
-    static_assert(L > 0 && L <= 32, "lane-per-row kernels cache at most 32 entries");
-    {
-        int c[L];
-        float h[L], lw[L];
-#pragma unroll
-        for (int k = 0; k < L; ++k) {
-            if (k < rl) {
-                int e = base + k * 32 + lane;
-                c[k] = a.col[e];
-                h[k] = a.hi[e];
-                lw[k] = a.lo[e];
-            } else {
-                c[k] = 0;
-                h[k] = 0.f;
-                lw[k] = 0.f;
-            }
-        }
-        i64 f = f0;
-        if constexpr (U >= 2) {
-            F2 hp[L], lp[L];
-#pragma unroll
-            for (int k = 0; k < L; ++k) {
-                hp[k] = pk(h[k], h[k]);
-                lp[k] = pk(lw[k], lw[k]);
-            }
-            for (; f + U <= f1; f += U) {
-                F2 s[U / 2], cc[U / 2];
-#pragma unroll
-                for (int u = 0; u < U / 2; ++u) {
-                    s[u] = pk(0.f, 0.f);
-                    cc[u] = pk(0.f, 0.f);
-                }
-                const float *xf = x + f * ldx;
-#pragma unroll
-                for (int k = 0; k < L; ++k) {
-                    if (k < rl) {
-#pragma unroll
-                        for (int u = 0; u < U / 2; ++u) {
-                            float xa = ldg_f(xf + (2 * u) * ldx + c[k]);
-                            float xb = ldg_f(xf + (2 * u + 1) * ldx + c[k]);
-                            csum2(s[u], cc[u], h[k], hp[k], lp[k], xa, xb);
-                        }
-                    }
-                }
-                if (store) {
-#pragma unroll
-                    for (int u = 0; u < U / 2; ++u) {
-                        F2 r = add2(s[u], cc[u]);
-                        float ra, rb;
-                        upk(r, ra, rb);
-                        y[(f + 2 * u) * ldy + row] = ra;
-                        y[(f + 2 * u + 1) * ldy + row] = rb;
-                        if (a.ylo) {
-                            float sa, sb, ca, cb;
-                            upk(s[u], sa, sb);
-                            upk(cc[u], ca, cb);
-                            a.ylo[(f + 2 * u) * a.ldylo + row] = sum_err(sa, ca, ra);
-                            a.ylo[(f + 2 * u + 1) * a.ldylo + row] = sum_err(sb, cb, rb);
-                        }
-                    }
-                }
-            }
-        }
-        for (; f < f1; ++f) {
-            float s = 0.f, cc = 0.f;
-            const float *xf = x + f * ldx;
-#pragma unroll
-            for (int k = 0; k < L; ++k)
-                if (k < rl) csum1(s, cc, h[k], lw[k], ldg_f(xf + c[k]));
-            if (store) {
-                const float r = __fadd_rn(s, cc);
-                y[f * ldy + row] = r;
-                if (a.ylo) a.ylo[f * a.ldylo + row] = sum_err(s, cc, r);
-            }
-        }
-    }
-}
-
 // ─── long rows ─────────────────────────────────────────────────────────────
-// Slices in the long classes (some row has more than 32 entries; coarse
-// destination cells over a fine source, e.g. polar cells over a lat-lon
-// source) run in two launches:
-//   k_split_rows: rows of at most 32 entries of those slices, one warp per
-//                 (row, 32 fields), lane = field, entry order;
-//   k_split_long: rows of more than 32 entries, one warp per (row, F
-//                 fields), lane = leaf of the order in fp32x2.cuh, the F
-//                 fields carried side by side, entries read row-contiguous
-//                 (Sell::lcol/lhi/llo), shuffle tree at the end.
-// Entry k of row p of slice sid sits at base[sid] + 32k + p.
-__device__ __forceinline__ bool row_item(const SellArgs &a, i64 nrhs, i64 &row, int &sid, int &p, i64 &f) {
-    const int lane = threadIdx.x & 31;
-    const i64 w = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const i64 per = a.n_ids * 32;
-    if (w >= per * ((nrhs + 31) / 32)) return false;
-    const i64 fc = w / per;
-    const i64 q = w - fc * per;
-    sid = a.ids[q >> 5];
-    p = static_cast<int>(q & 31);
-    row = static_cast<i64>(sid) * 32 + p;
-    f = fc * 32 + lane;
-    return row < a.n_rows && f < nrhs;
-}
-
-__global__ void __launch_bounds__(256) k_split_rows(SellArgs a, const float *__restrict__ x, i64 ldx,
-                                                    float *__restrict__ y, i64 ldy, i64 nrhs) {
-    i64 row, f;
-    int sid, p;
-    if (!row_item(a, nrhs, row, sid, p, f)) return;
-    const int n = a.rlen[row];
-    if (n > 32) return;  // k_split_long
-    const int e0 = a.base[sid] + p;
-    const float *xf = x + f * ldx;
-    float s = 0.f, c = 0.f;
-    for (int k = 0; k < n; ++k) {
-        const int e = e0 + 32 * k;
-        csum1(s, c, a.hi[e], a.lo[e], ldg_f(xf + a.col[e]));
-    }
-    const float r = __fadd_rn(s, c);
-    y[f * ldy + row] = r;
-    if (a.ylo) a.ylo[f * a.ldylo + row] = sum_err(s, c, r);
-}
-
+// Rows of more than 32 entries (coarse destination cells over a fine source,
+// e.g. polar cells over a lat-lon source): one warp per (row, F fields), lane =
+// leaf of the order in fp32x2.cuh, the F fields carried side by side, entries
+// read row-contiguous (Sell::lcol/lhi/llo), shuffle tree at the end.
 constexpr int kF64F = 4;          // fields an FP64 row carries side by side
 constexpr int kFusedK = 4;        // entries a row of the fused kernels loads before gathering
 constexpr int kF64K = 2;          // the same of the FP64 kernel from three fields up
 
 struct LongRows {
     const int *row, *ptr, *col;
-    const float *hi, *lo;
+    const float2 *hl;
     const double *w64;
     i64 n;
     float *ylo;  // split: low parts of the outputs (hi+lo form), or null
     i64 ldylo;
 };
 constexpr int kLongF = 8;  // fields per warp in the long-row kernels
-constexpr int kLongQ1 = 8;  // entries a lane loads ahead in a single-field long row
+constexpr int kLongQ1 = 12;  // entries a lane loads ahead in a single-field long row
+constexpr int kLongQ1D = 8;  // the same in FP64
 constexpr int kLongQ = 4;   // the same with several fields
 constexpr int kBatchLongF = 4;  // fields per long-row item of the persistent batch kernel (k_batch<true>)
 
@@ -347,23 +214,26 @@ __device__ __forceinline__ void split_long_row(const LongRows &L, i64 i, i64 fc,
     if constexpr (F == 1) {
         // kLongQ1 of the leaf's entries per step: their loads are issued
         // together (memory-level parallelism for rows of hundreds of
-        // entries), then summed in order, as one entry per step would
+        // entries), then summed in order, as one entry per step would. The
+        // last step is partial.
         v[0] = {0.f, 0.f};
-        for (; k + 32 * (kLongQ1 - 1) < n; k += 32 * kLongQ1) {
+        for (; k - lane < n; k += 32 * kLongQ1) {
             int cq[kLongQ1];
-            float hq[kLongQ1], lq[kLongQ1], xq[kLongQ1];
+            float2 wq[kLongQ1];
+            float xq[kLongQ1];
 #pragma unroll
-            for (int q = 0; q < kLongQ1; ++q) {
-                cq[q] = L.col[b + k + 32 * q];
-                hq[q] = L.hi[b + k + 32 * q];
-                lq[q] = L.lo[b + k + 32 * q];
-            }
+            for (int q = 0; q < kLongQ1; ++q)
+                if (k + 32 * q < n) {
+                    cq[q] = L.col[b + k + 32 * q];
+                    wq[q] = L.hl[b + k + 32 * q];
+                }
 #pragma unroll
-            for (int q = 0; q < kLongQ1; ++q) xq[q] = ldg_f(x + cq[q]);
+            for (int q = 0; q < kLongQ1; ++q)
+                if (k + 32 * q < n) xq[q] = ldg_f(x + cq[q]);
 #pragma unroll
-            for (int q = 0; q < kLongQ1; ++q) csum1(v[0].s, v[0].c, hq[q], lq[q], xq[q]);
+            for (int q = 0; q < kLongQ1; ++q)
+                if (k + 32 * q < n) csum1(v[0].s, v[0].c, wq[q].x, wq[q].y, xq[q]);
         }
-        for (; k < n; k += 32) csum1(v[0].s, v[0].c, L.hi[b + k], L.lo[b + k], ldg_f(x + L.col[b + k]));
     } else {
         F2 s[F / 2], c[F / 2];
 #pragma unroll
@@ -374,13 +244,13 @@ __device__ __forceinline__ void split_long_row(const LongRows &L, i64 i, i64 fc,
         auto rounds = [&](auto q_tag, bool partial) {
             constexpr int Q = decltype(q_tag)::value;
             int cq[Q];
-            float hq[Q], lq[Q], xq[Q][F];
+            float2 wq[Q];
+            float xq[Q][F];
 #pragma unroll
             for (int q = 0; q < Q; ++q) {
                 const bool on = q < Q - 1 || !partial || k + 32 * q < n;
                 cq[q] = on ? L.col[b + k + 32 * q] : -1;
-                hq[q] = on ? L.hi[b + k + 32 * q] : 0.f;
-                lq[q] = on ? L.lo[b + k + 32 * q] : 0.f;
+                wq[q] = on ? L.hl[b + k + 32 * q] : make_float2(0.f, 0.f);
             }
 #pragma unroll
             for (int q = 0; q < Q; ++q)
@@ -388,9 +258,9 @@ __device__ __forceinline__ void split_long_row(const LongRows &L, i64 i, i64 fc,
                 for (int f = 0; f < F; ++f) xq[q][f] = f < nf && cq[q] >= 0 ? ldg_f(x + f * ldx + cq[q]) : 0.f;
 #pragma unroll
             for (int q = 0; q < Q; ++q) {
-                const F2 hp = pk(hq[q], hq[q]), lp = pk(lq[q], lq[q]);
+                const F2 hp = pk(wq[q].x, wq[q].x), lp = pk(wq[q].y, wq[q].y);
 #pragma unroll
-                for (int f = 0; f < F / 2; ++f) csum2(s[f], c[f], hq[q], hp, lp, xq[q][2 * f], xq[q][2 * f + 1]);
+                for (int f = 0; f < F / 2; ++f) csum2(s[f], c[f], wq[q].x, hp, lp, xq[q][2 * f], xq[q][2 * f + 1]);
             }
             k += 32 * Q;
         };
@@ -476,7 +346,7 @@ __device__ __forceinline__ void f64_long_row(const LongRows &L, i64 i, i64 fc, c
                 if (f < nf) s[f] = fma(wq[q], xq[q][f], s[f]);
         k += 32 * Q;
     };
-    constexpr int kQ = F == 1 ? kLongQ1 : kLongQ;
+    constexpr int kQ = F == 1 ? kLongQ1D : kLongQ;
     int left = n;  // warp-uniform
     for (; left >= 32 * kQ; left -= 32 * kQ) rounds(std::integral_constant<int, kQ>{}, false);
     if (kQ > 4 && left >= 128) {
@@ -499,64 +369,187 @@ __device__ __forceinline__ void f64_long_row(const LongRows &L, i64 i, i64 fc, c
     if (lane < F && f < nf) y[(f0 + f) * ldy + row] = s[0];
 }
 
-// ─── few fields: one launch over the whole matrix ────────────────────────
-// Warps [0, n_slices): lane per row of one slice, rows of at most 32 entries,
-// each entry read from the sliced layout per field (nothing cached: with
-// one or two fields there is nothing to reuse); warps [n_slices, n_slices +
-// n_lrows): one row of more than 32 entries each, for all fields, 8 at a time
-// (split_long_row / f64_long_row). Same summation order as the class
-// kernels, so the same bits, in one launch instead of one per class.
-// F: fields a long-row warp carries (the call's field count, at most
-// kLongF); few fields need few registers, so more warps fit.
-template <int F>
-__global__ void __launch_bounds__(256, F <= 2 ? 4 : 2) k_split_fused(SellArgs a, LongRows L, i64 n_slices,
-                                                                   const float *__restrict__ x, i64 ldx,
-                                                                   float *__restrict__ y, i64 ldy, i64 nrhs) {
+// ─── direct split kernel: one launch over the whole matrix ───────────────
+// blockIdx.y: a tile of fields. Warps [0, n_long): a row of more than 32
+// entries (split_long_row; the chunks of F fields shared out over blockIdx.y);
+// the others: lane per row of one slice (of ids, or all), rows of at most 32
+// entries, F fields side by side: K entries' loads, then their gathers, then the compensated steps in
+// entry order (two memory round trips a chunk instead of two an entry). The
+// entries are read again for the tile's next F fields, from L1. Nothing is
+// asked of the fields' alignment. Bound by the latency of its dependent round
+// trips and by instruction issue: it is the kernel for few fields, small
+// matrices (the rule is default_split_params in api.cpp) and unaligned
+// fields. 45 unaligned fields of a 361 x 271 ocean grid -> 1 deg: 30 us, against
+// 184 us for a launch per length class whose warps walked all fields; 7 fields
+// of C192 -> 0.5 deg with hi+lo outputs 16.4 us, against 20 staged.
+// The same for one field. There is too little work in a row to hide its chain
+// of dependent loads (length, entries, source values) behind other warps: the
+// short rows' warps stay and take slice after slice, with the lengths read
+// two slices ahead and the first kOneK entries one slice ahead, so that only
+// the gathers are waited for. The first blocks take the long rows, a warp
+// each. 0.25 deg -> C384: 16.7 us, against 23 us with a warp a slice.
+constexpr int kOneK = 5;
+constexpr int kOneBlocks = 3;  // an SM
+__global__ void __launch_bounds__(256, kOneBlocks) k_split_one(SellArgs a, LongRows L, int n_long, int long_blocks,
+                                                               int n_slices, const float *__restrict__ x,
+                                                               float *__restrict__ y) {
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    if (static_cast<int>(blockIdx.x) < long_blocks) {
+        const int i = static_cast<int>(blockIdx.x) * 8 + wp;
+        if (i < n_long) split_long_row<1>(L, i, 0, x, 0, y, 0, 1);
+        return;
+    }
+    const int step = static_cast<int>(gridDim.x - long_blocks) * 8;
+    int sid = static_cast<int>(blockIdx.x - long_blocks) * 8 + wp;
+    // entries (-1: a long row or none to store) and first entry of the lane's row
+    auto meta = [&](int s, int &n, int &e) {
+        n = -1;
+        e = 0;
+        const i64 row = static_cast<i64>(s) * 32 + lane;
+        if (s < n_slices && row < a.n_rows) {
+            n = a.rlen[row];
+            e = a.base[s] + lane;
+        }
+        if (n > 32) n = -1;
+    };
+    int n0, e0, n1, e1;
+    int c0[kOneK];
+    float2 w0[kOneK];
+    meta(sid, n0, e0);
+    meta(sid + step, n1, e1);
+#pragma unroll
+    for (int j = 0; j < kOneK; ++j)
+        if (j < n0) {
+            c0[j] = a.col[e0 + 32 * j];
+            w0[j] = a.hl[e0 + 32 * j];
+        }
+    for (; sid < n_slices; sid += step) {
+        int n2, e2, c1[kOneK];
+        float2 w1[kOneK];
+        float xv[kOneK];
+        meta(sid + 2 * step, n2, e2);
+#pragma unroll
+        for (int j = 0; j < kOneK; ++j)
+            if (j < n0) xv[j] = ldg_f(x + c0[j]);
+#pragma unroll
+        for (int j = 0; j < kOneK; ++j)
+            if (j < n1) {
+                c1[j] = a.col[e1 + 32 * j];
+                w1[j] = a.hl[e1 + 32 * j];
+            }
+        float s = 0.f, c = 0.f;
+#pragma unroll
+        for (int j = 0; j < kOneK; ++j)
+            if (j < n0) csum1(s, c, w0[j].x, w0[j].y, xv[j]);
+        for (int k0 = kOneK; k0 < n0; k0 += kFusedK) {
+            int cl[kFusedK];
+            float2 w[kFusedK];
+            float xr[kFusedK];
+#pragma unroll
+            for (int j = 0; j < kFusedK; ++j)
+                if (k0 + j < n0) {
+                    cl[j] = a.col[e0 + 32 * (k0 + j)];
+                    w[j] = a.hl[e0 + 32 * (k0 + j)];
+                }
+#pragma unroll
+            for (int j = 0; j < kFusedK; ++j)
+                if (k0 + j < n0) xr[j] = ldg_f(x + cl[j]);
+#pragma unroll
+            for (int j = 0; j < kFusedK; ++j)
+                if (k0 + j < n0) csum1(s, c, w[j].x, w[j].y, xr[j]);
+        }
+        if (n0 >= 0) {
+            const i64 row = static_cast<i64>(sid) * 32 + lane;
+            const float r = __fadd_rn(s, c);
+            y[row] = r;
+            if (a.ylo) a.ylo[row] = sum_err(s, c, r);
+        }
+        n0 = n1;
+        e0 = e1;
+        n1 = n2;
+        e1 = e2;
+#pragma unroll
+        for (int j = 0; j < kOneK; ++j) {
+            c0[j] = c1[j];
+            w0[j] = w1[j];
+        }
+    }
+}
+
+template <int F, int K, bool ALL>
+__device__ __forceinline__ void short_rows(const SellArgs &a, int n, int e0, i64 row, const float *__restrict__ x,
+                                           i64 ldx, float *__restrict__ y, i64 ldy, i64 f, int nf) {
+    const float *xf = x + f * ldx;
+    F2 s[F / 2], c[F / 2];
+#pragma unroll
+    for (int u = 0; u < F / 2; ++u) s[u] = c[u] = pk(0.f, 0.f);
+    for (int k0 = 0; k0 < n; k0 += K) {
+        int cl[K];
+        float2 w[K];
+        float xv[K][F];
+#pragma unroll
+        for (int j = 0; j < K; ++j)
+            if (k0 + j < n) {
+                cl[j] = a.col[e0 + 32 * (k0 + j)];
+                w[j] = a.hl[e0 + 32 * (k0 + j)];
+            }
+#pragma unroll
+        for (int j = 0; j < K; ++j)
+            if (k0 + j < n) {
+#pragma unroll
+                for (int u = 0; u < F; ++u) xv[j][u] = ALL || u < nf ? ldg_f(xf + u * ldx + cl[j]) : 0.f;
+            }
+#pragma unroll
+        for (int j = 0; j < K; ++j)
+            if (k0 + j < n) {
+                const F2 hp = pk(w[j].x, w[j].x), lp = pk(w[j].y, w[j].y);
+#pragma unroll
+                for (int u = 0; u < F / 2; ++u) csum2(s[u], c[u], w[j].x, hp, lp, xv[j][2 * u], xv[j][2 * u + 1]);
+            }
+    }
+    float *yf = y + f * ldy + row;
+#pragma unroll
+    for (int u = 0; u < F; ++u) {
+        if (!ALL && u >= nf) break;
+        float sv, cv, o;
+        if (u & 1) {
+            upk(s[u / 2], o, sv);
+            upk(c[u / 2], o, cv);
+        } else {
+            upk(s[u / 2], sv, o);
+            upk(c[u / 2], cv, o);
+        }
+        const float r = __fadd_rn(sv, cv);
+        yf[u * ldy] = r;
+        if (a.ylo) a.ylo[(f + u) * a.ldylo + row] = sum_err(sv, cv, r);
+    }
+}
+
+template <int F, int K>
+__global__ void __launch_bounds__(256, F <= 4 ? 4 : 3) k_split_fused(SellArgs a, LongRows L, int n_long, int n_slices,
+                                                                    const float *__restrict__ x, i64 ldx,
+                                                                    float *__restrict__ y, i64 ldy, i64 nrhs, int tile) {
     const int lane = threadIdx.x & 31;
-    const i64 wg = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    int w = static_cast<int>(blockIdx.x * 8 + (threadIdx.x >> 5));
     // the long rows' warps come first in the grid: each is a long chain of
     // dependent loads, and starting them with the first wave overlaps them
     // with the short rows instead of leaving them as the tail
-    if (wg < L.n) {
-        for (i64 fc = 0; fc * F < nrhs; ++fc) split_long_row<F>(L, wg, fc, x, ldx, y, ldy, nrhs);
+    if (w < n_long) {
+        for (i64 fc = blockIdx.y; fc * F < nrhs; fc += gridDim.y) split_long_row<F>(L, w, fc, x, ldx, y, ldy, nrhs);
         return;
     }
-    const i64 w = wg - L.n;
-    if (w < n_slices) {
-        const i64 row = w * 32 + lane;
-        if (row >= a.n_rows) return;
-        const int n = a.rlen[row];
-        if (n > 32) return;  // a long row: its own warp above
-        const int e0 = a.base[w] + lane;
-        for (i64 f = 0; f < nrhs; ++f) {
-            const float *xf = x + f * ldx;
-            float s = 0.f, c = 0.f;
-            // kFusedK entries at a time: their loads, then their gathers, then
-            // the compensated steps in entry order (two memory round trips a
-            // chunk instead of two an entry)
-            for (int k0 = 0; k0 < n; k0 += kFusedK) {
-                int cl[kFusedK];
-                float hv[kFusedK], lv[kFusedK], xv[kFusedK];
-#pragma unroll
-                for (int j = 0; j < kFusedK; ++j)
-                    if (k0 + j < n) {
-                        const int e = e0 + 32 * (k0 + j);
-                        cl[j] = a.col[e];
-                        hv[j] = a.hi[e];
-                        lv[j] = a.lo[e];
-                    }
-#pragma unroll
-                for (int j = 0; j < kFusedK; ++j)
-                    if (k0 + j < n) xv[j] = ldg_f(xf + cl[j]);
-#pragma unroll
-                for (int j = 0; j < kFusedK; ++j)
-                    if (k0 + j < n) csum1(s, c, hv[j], lv[j], xv[j]);
-            }
-            const float r = __fadd_rn(s, c);
-            y[f * ldy + row] = r;
-            if (a.ylo) a.ylo[f * a.ldylo + row] = sum_err(s, c, r);
-        }
-    }
+    w -= n_long;
+    if (w >= n_slices) return;
+    const int sid = a.ids ? a.ids[w] : w;
+    const i64 row = static_cast<i64>(sid) * 32 + lane;
+    if (row >= a.n_rows) return;
+    const int n = a.rlen[row];
+    if (n > 32) return;  // a long row: its own warp above
+    const int e0 = a.base[sid] + lane;
+    const i64 fa = static_cast<i64>(blockIdx.y) * tile, fb = min(fa + tile, nrhs);
+    i64 f = fa;
+    for (; f + F <= fb; f += F) short_rows<F, K, true>(a, n, e0, row, x, ldx, y, ldy, f, F);
+    if (f < fb) short_rows<F, K, false>(a, n, e0, row, x, ldx, y, ldy, f, static_cast<int>(fb - f));
 }
 
 // FP64 apply in one launch. Warps [0, L.n * ceil(nrhs / F)): a long row and F
@@ -579,11 +572,12 @@ __global__ void __launch_bounds__(256, 4) k_f64_fused(SellArgs a, LongRows L, co
     // the long rows' warps come first in the grid, as in k_split_fused
     const i64 n_long = L.n * ((nrhs + F - 1) / F);
     if (w < n_long) {
-        f64_long_row<F>(L, w % L.n, w / L.n, x, ldx, y, ldy, nrhs);
+        const i64 fc = nrhs <= F ? 0 : w / L.n;
+        f64_long_row<F>(L, w - fc * L.n, fc, x, ldx, y, ldy, nrhs);
         return;
     }
     w -= n_long;
-    const i64 t = w / n_slices, pos = (w - t * n_slices) * 32 + lane;
+    const i64 t = nrhs <= tile ? 0 : w / n_slices, pos = (w - t * n_slices) * 32 + lane;
     const i64 fa = t * tile, fb = min(fa + tile, nrhs);
     if (fa >= nrhs) return;
     const i64 row = F > 2 ? ord[pos] : pos;
@@ -629,7 +623,7 @@ __global__ void __launch_bounds__(256, 4) k_f64_fused(SellArgs a, LongRows L, co
 
 // Row-contiguous copy of the long rows' entries (in the layout's order).
 __global__ void k_long_fill(const int *rp, const int *ccol, const double *val, const int *perm, const int *lrow,
-                            const int *lptr, i64 n_lrows, int *lcol, float *lhi, float *llo, double *lw64) {
+                            const int *lptr, i64 n_lrows, int *lcol, float2 *lhl, double *lw64) {
     const i64 i = blockIdx.x;
     if (i >= n_lrows) return;
     const int r = lrow[i], r0 = rp[r], b = lptr[i], n = lptr[i + 1] - b;
@@ -637,10 +631,9 @@ __global__ void k_long_fill(const int *rp, const int *ccol, const double *val, c
         const int src = perm ? perm[r0 + k] : r0 + k;
         const double w = val[src];
         lcol[b + k] = ccol[src];
-        if (lhi) {
+        if (lhl) {
             const float h = __double2float_rn(w);
-            lhi[b + k] = h;
-            llo[b + k] = __double2float_rn(w - static_cast<double>(h));
+            lhl[b + k] = make_float2(h, __double2float_rn(w - static_cast<double>(h)));
         }
         if (lw64) lw64[b + k] = w;
     }
@@ -661,8 +654,8 @@ __global__ void k_slice_len(const int *rp, i64 n_rows, i64 n_slices, int *len) {
 
 // perm (optional): CSR index of the k-th entry of each row (split layouts).
 __global__ void k_sell_fill(const int *rp, const int *ccol, const double *val, const int *perm, i64 n_rows,
-                            i64 n_slices, const int *base, const int *slen32, int *rlen, int *col, float *hi,
-                            float *lo, double *w64, double *total) {
+                            i64 n_slices, const int *base, const int *slen32, int *rlen, int *col, float2 *hl,
+                            double *w64, double *total) {
     i64 r = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (r >= n_slices * 32) return;
     i64 s = r >> 5;
@@ -684,18 +677,14 @@ __global__ void k_sell_fill(const int *rp, const int *ccol, const double *val, c
             double w = val[src];
             tot = __dadd_rn(tot, w);
             col[e] = ccol[src];
-            if (hi) {
+            if (hl) {
                 float h = __double2float_rn(w);
-                hi[e] = h;
-                lo[e] = __double2float_rn(w - static_cast<double>(h));
+                hl[e] = make_float2(h, __double2float_rn(w - static_cast<double>(h)));
             }
             if (w64) w64[e] = w;
         } else {
             col[e] = last;
-            if (hi) {
-                hi[e] = 0.f;
-                lo[e] = 0.f;
-            }
+            if (hl) hl[e] = make_float2(0.f, 0.f);
             if (w64) w64[e] = 0.0;
         }
     }
@@ -748,8 +737,7 @@ void build_sell(Matrix &m, int fmt, cudaStream_t s) {
     S.base = std::move(base);
     DBuf<int> rlen(n_slices * 32);
     if (fmt == 1) {
-        S.hi.alloc(total);
-        S.lo.alloc(total);
+        S.hl.alloc(total);
     } else {
         S.w64.alloc(total);
         S.total.alloc(n_rows);
@@ -759,7 +747,7 @@ void build_sell(Matrix &m, int fmt, cudaStream_t s) {
         const int *ccol = (fmt == 1 && m.src_renum) ? m.split_col.p : m.col.p;
         k_sell_fill<<<nblk(n_slices * 32, 256), 256, 0, s>>>(m.row_ptr.p, ccol, m.val.p, perm, n_rows, n_slices,
                                                             S.base.p, slen32.p, rlen.p, S.col.p,
-                                                            fmt == 1 ? S.hi.p : nullptr, fmt == 1 ? S.lo.p : nullptr,
+                                                            fmt == 1 ? S.hl.p : nullptr,
                                                             fmt == 0 ? S.w64.p : nullptr, fmt == 0 ? S.total.p : nullptr);
         AXGB_CUDA(cudaGetLastError());
     }
@@ -800,8 +788,7 @@ void build_sell(Matrix &m, int fmt, cudaStream_t s) {
         const size_t ne = std::max<size_t>(1, lptr.back());
         S.lcol.alloc(ne);
         if (fmt == 1) {
-            S.lhi.alloc(ne);
-            S.llo.alloc(ne);
+            S.lhl.alloc(ne);
         } else {
             S.lw64.alloc(ne);
         }
@@ -810,7 +797,7 @@ void build_sell(Matrix &m, int fmt, cudaStream_t s) {
             const int *ccol = (fmt == 1 && m.src_renum) ? m.split_col.p : m.col.p;
             k_long_fill<<<static_cast<unsigned>(S.n_lrows), 128, 0, s>>>(
                 m.row_ptr.p, ccol, m.val.p, perm, S.lrow.p, S.lptr.p, S.n_lrows, S.lcol.p,
-                fmt == 1 ? S.lhi.p : nullptr, fmt == 1 ? S.llo.p : nullptr, fmt == 0 ? S.lw64.p : nullptr);
+                fmt == 1 ? S.lhl.p : nullptr, fmt == 0 ? S.lw64.p : nullptr);
             AXGB_CUDA(cudaGetLastError());
         }
     }
@@ -833,25 +820,10 @@ SellArgs sell_args(const Matrix &m, const Sell &S, int cls, float *ylo = nullptr
     a.len = nullptr;
     a.rlen = S.len.p;
     a.col = S.col.p;
-    a.hi = S.hi.p;
-    a.lo = S.lo.p;
+    a.hl = S.hl.p;
     a.w64 = S.w64.p;
     a.n_rows = m.n_dst;
     return a;
-}
-
-template <int L>
-void launch_split(const SellArgs &a, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, i64 tile, int U,
-                  cudaStream_t s) {
-    i64 items = ((nrhs + tile - 1) / tile) * a.n_ids;
-    if (items == 0) return;
-    unsigned blocks = nblk(items * 32, 256);
-    if (U >= 4)
-        k_split<L, 4><<<blocks, 256, 0, s>>>(a, x, ldx, y, ldy, nrhs, tile);
-    else if (U >= 2)
-        k_split<L, 2><<<blocks, 256, 0, s>>>(a, x, ldx, y, ldy, nrhs, tile);
-    else
-        k_split<L, 1><<<blocks, 256, 0, s>>>(a, x, ldx, y, ldy, nrhs, tile);
 }
 
 LongRows long_rows(const Sell &S) {
@@ -859,8 +831,7 @@ LongRows long_rows(const Sell &S) {
     L.row = S.lrow.p;
     L.ptr = S.lptr.p;
     L.col = S.lcol.p;
-    L.hi = S.lhi.p;
-    L.lo = S.llo.p;
+    L.hl = S.lhl.p;
     L.w64 = S.lw64.p;
     L.n = S.n_lrows;
     return L;
@@ -875,11 +846,6 @@ dim3 long_grid(i64 rows, i64 nrhs) {
 
 // Slices of the long classes: their short rows (k_*_rows), then every row
 // of more than 32 entries (k_*_long).
-void launch_split_rows(const SellArgs &a, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, cudaStream_t s) {
-    if (a.n_ids == 0 || nrhs == 0) return;
-    const i64 warps = a.n_ids * 32 * ((nrhs + 31) / 32);
-    k_split_rows<<<nblk(warps * 32, 256), 256, 0, s>>>(a, x, ldx, y, ldy, nrhs);
-}
 void launch_split_long(const Sell &S, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, cudaStream_t s,
                        float *ylo = nullptr, i64 ldylo = 0) {
     if (S.n_lrows == 0 || nrhs == 0) return;
@@ -892,15 +858,13 @@ void launch_split_long(const Sell &S, const float *x, i64 ldx, float *y, i64 ldy
 
 // Rows of more than 32 entries given row-contiguous (the segmented layout's
 // own copy, original source numbering): k_split_long, same summation order.
-void launch_long_rows(const int *row, const int *ptr, const int *col, const float *hi, const float *lo, i64 n,
-                      const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, cudaStream_t s, float *ylo, i64 ldylo) {
+void launch_long_rows(const int *row, const int *ptr, const int *col, const float2 *hl, i64 n, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, cudaStream_t s, float *ylo, i64 ldylo) {
     if (n == 0 || nrhs == 0) return;
     LongRows L{};
     L.row = row;
     L.ptr = ptr;
     L.col = col;
-    L.hi = hi;
-    L.lo = lo;
+    L.hl = hl;
     L.n = n;
     L.ylo = ylo;
     L.ldylo = ldylo;
@@ -909,24 +873,42 @@ void launch_long_rows(const int *row, const int *ptr, const int *col, const floa
 
 namespace {
 
-// One launch for the whole matrix (few fields): warp per slice, then warp per long row.
+// F fields side by side (0: by the count), tile fields a warp (0: by the
+// size, as launch_f64_fused); ids / n_ids: these slices only, without the
+// long rows.
 void launch_split_fused(const Matrix &m, const Sell &S, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs,
-                        cudaStream_t s, float *ylo, i64 ldylo) {
-    const i64 warps = S.n_slices + S.n_lrows;
-    if (warps == 0 || nrhs == 0) return;
+                        cudaStream_t s, float *ylo, i64 ldylo, int F = 0, i64 tile = 0, const int *ids = nullptr,
+                        i64 n_ids = 0) {
     LongRows L = long_rows(S);
     L.ylo = ylo;
     L.ldylo = ldylo;
-    const SellArgs a = sell_args(m, S, 0, ylo, ldylo);
-    const unsigned g = nblk(warps * 32, 256);
-    if (nrhs == 1)
-        k_split_fused<1><<<g, 256, 0, s>>>(a, L, S.n_slices, x, ldx, y, ldy, nrhs);
-    else if (nrhs == 2)
-        k_split_fused<2><<<g, 256, 0, s>>>(a, L, S.n_slices, x, ldx, y, ldy, nrhs);
-    else if (nrhs <= 4)
-        k_split_fused<4><<<g, 256, 0, s>>>(a, L, S.n_slices, x, ldx, y, ldy, nrhs);
+    SellArgs a = sell_args(m, S, 0, ylo, ldylo);
+    a.ids = ids;
+    const i64 n_slices = ids ? n_ids : S.n_slices;
+    const int n_long = ids ? 0 : static_cast<int>(L.n);
+    if (n_slices + n_long == 0 || nrhs == 0) return;
+    if (nrhs == 1 && !ids) {
+        const int long_blocks = static_cast<int>(nblk(n_long, 8));
+        const int room = std::max(152 * 2, 152 * kOneBlocks - long_blocks);
+        const int blocks = std::min<int>(static_cast<int>(nblk(n_slices, 8)), room);
+        k_split_one<<<long_blocks + blocks, 256, 0, s>>>(a, L, n_long, long_blocks, static_cast<int>(n_slices), x, y);
+        return;
+    }
+    if (F == 0) F = nrhs == 2 ? 2 : nrhs <= 4 ? 4 : 8;
+    if (tile <= 0) tile = std::min<i64>(64, n_slices * nrhs / (152 * 24 * 4));
+    tile = std::max<i64>(tile, (nrhs + 65534) / 65535);
+    F = std::max(F, 2);
+    tile = (tile + F - 1) / F * F;
+    const dim3 g(nblk(n_long + n_slices, 8), static_cast<unsigned>((nrhs + tile - 1) / tile));
+    auto launch = [&](auto kernel) {
+        kernel<<<g, 256, 0, s>>>(a, L, n_long, static_cast<int>(n_slices), x, ldx, y, ldy, nrhs, static_cast<int>(tile));
+    };
+    if (F <= 2)
+        launch(k_split_fused<2, 4>);
+    else if (F <= 4)
+        launch(k_split_fused<4, 4>);
     else
-        k_split_fused<kLongF><<<g, 256, 0, s>>>(a, L, S.n_slices, x, ldx, y, ldy, nrhs);
+        launch(k_split_fused<8, 2>);
 }
 void launch_f64_fused(const Matrix &m, const Sell &S, const double *x, i64 ldx, double *y, i64 ldy, i64 nrhs,
                       cudaStream_t s) {
@@ -1384,8 +1366,7 @@ __global__ void __launch_bounds__(256, ROWS ? 4 : 2) k_batch(const Batch::Desc *
             L.row = d.lrow;
             L.ptr = d.lptr;
             L.col = d.lcol;
-            L.hi = d.lhi;
-            L.lo = d.llo;
+            L.hl = d.lhl;
             L.w64 = nullptr;
             L.n = d.n_ids;
             split_long_row<kBatchLongF>(L, local % L.n, local / L.n, d.x, d.ldx, d.y, d.ldy, d.nrhs);
@@ -1407,7 +1388,7 @@ __global__ void __launch_bounds__(256, ROWS ? 4 : 2) k_batch(const Batch::Desc *
                     float s = 0.f, c = 0.f;
                     for (int k = 0; k < n; ++k) {
                         const int e = e0 + 32 * k;
-                        csum1(s, c, d.hi[e], d.lo[e], __ldg(xf + d.col[e]));
+                        csum1(s, c, d.hl[e].x, d.hl[e].y, __ldg(xf + d.col[e]));
                     }
                     d.y[f * d.ldy + row] = __fadd_rn(s, c);
                 }
@@ -1430,8 +1411,8 @@ __global__ void __launch_bounds__(256, ROWS ? 4 : 2) k_batch(const Batch::Desc *
             if (k < rl) {
                 int e = base + k * 32 + lane;
                 c[k] = d.col[e];
-                h[k] = d.hi[e];
-                lw[k] = d.lo[e];
+                h[k] = d.hl[e].x;
+                lw[k] = d.hl[e].y;
             } else {
                 c[k] = 0;
                 h[k] = 0.f;
@@ -1446,7 +1427,7 @@ __global__ void __launch_bounds__(256, ROWS ? 4 : 2) k_batch(const Batch::Desc *
                 if (k < rl) csum1(s, cc, h[k], lw[k], __ldg(xf + c[k]));
             for (int k = L; k < rl; ++k) {  // rows of 17..32 entries: the tail from global memory
                 int e = base + k * 32 + lane;
-                csum1(s, cc, d.hi[e], d.lo[e], __ldg(xf + d.col[e]));
+                csum1(s, cc, d.hl[e].x, d.hl[e].y, __ldg(xf + d.col[e]));
             }
             if (store) d.y[f * d.ldy + row] = __fadd_rn(s, cc);
         }
@@ -1510,6 +1491,8 @@ void gather_source(const Matrix &m, const float *x, i64 ldx, i64 nrhs, float *xr
     AXGB_CUDA(cudaGetLastError());
 }
 
+int split_launches(const Matrix &m) { return blocked_launches(m) + (m.sell32.n_lrows > 0 ? 1 : 0); }
+
 void apply_split_layouts(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, const SplitParams &p,
                          cudaStream_t s, float *ylo, i64 ldylo);
 
@@ -1544,10 +1527,8 @@ void apply_split_layouts(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, 
         apply_blocked(m, x, ldx, y, ldy, nrhs, p.variant, p.unroll, p.stages, p.fields_per_pass, s, ylo, ldylo);
         const Blocked &B = m.blocked;
         if (B.n_fallback > 0) {
-            SellArgs a = sell_args(m, m.sell32, 4, ylo, ldylo);
-            a.ids = B.fallback_slices.p;
-            a.n_ids = B.n_fallback;
-            launch_split_rows(a, x, ldx, y, ldy, nrhs, s);
+            launch_split_fused(m, m.sell32, x, ldx, y, ldy, nrhs, s, ylo, ldylo, 0, 0, B.fallback_slices.p,
+                               B.n_fallback);
         }
         launch_split_long(m.sell32, x, ldx, y, ldy, nrhs, s, ylo, ldylo);
         AXGB_CUDA(cudaGetLastError());
@@ -1555,19 +1536,12 @@ void apply_split_layouts(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, 
     }
     if (!m.sell32.built) matrix_prepare(m, 1, s);
     const Sell &S = m.sell32;
-    if (p.variant == 4) {  // one launch for the whole matrix (few fields)
+    // direct kernel: with the caller's knobs (variant 0), else its own choice
+    if (p.variant == 0)
+        launch_split_fused(m, S, x, ldx, y, ldy, nrhs, s, ylo, ldylo, p.unroll,
+                           p.fields_per_pass <= 0 || p.fields_per_pass > nrhs ? nrhs : p.fields_per_pass);
+    else
         launch_split_fused(m, S, x, ldx, y, ldy, nrhs, s, ylo, ldylo);
-        AXGB_CUDA(cudaGetLastError());
-        return;
-    }
-    i64 tile = (p.fields_per_pass <= 0 || p.fields_per_pass > nrhs) ? nrhs : p.fields_per_pass;
-    const int unroll = p.variant == 0 ? p.unroll : 4;
-    launch_split<8>(sell_args(m, S, 0, ylo, ldylo), x, ldx, y, ldy, nrhs, tile, unroll, s);
-    launch_split<16>(sell_args(m, S, 1, ylo, ldylo), x, ldx, y, ldy, nrhs, tile, unroll, s);
-    launch_split<32>(sell_args(m, S, 2, ylo, ldylo), x, ldx, y, ldy, nrhs, tile, unroll, s);
-    launch_split_rows(sell_args(m, S, 3, ylo, ldylo), x, ldx, y, ldy, nrhs, s);
-    launch_split_rows(sell_args(m, S, 4, ylo, ldylo), x, ldx, y, ldy, nrhs, s);
-    launch_split_long(S, x, ldx, y, ldy, nrhs, s, ylo, ldylo);
     AXGB_CUDA(cudaGetLastError());
 }
 
@@ -1684,13 +1658,11 @@ void plan_direct(Batch &b) {
             d.len = nullptr;
             d.rlen = S.len.p;
             d.col = S.col.p;
-            d.hi = S.hi.p;
-            d.lo = S.lo.p;
+            d.hl = S.hl.p;
             d.lrow = S.lrow.p;
             d.lptr = S.lptr.p;
             d.lcol = S.lcol.p;
-            d.lhi = S.lhi.p;
-            d.llo = S.llo.p;
+            d.lhl = S.lhl.p;
             d.mode = mode;
             d.mat = static_cast<int>(q);
             d.n_rows = m.n_dst;

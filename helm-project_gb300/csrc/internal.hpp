@@ -180,7 +180,7 @@ struct Sell {
     bool built = false;
     i64 n_slices = 0, n_entries = 0;
     DBuf<int> base, len, col;
-    DBuf<float> hi, lo;     // split weights (format 1)
+    DBuf<float2> hl;        // split weights (hi, lo) (format 1)
     DBuf<double> w64;       // FP64 weights (format 0)
     DBuf<double> total;     // sum of each row's weights in CSR order (format 0; NaN-aware apply)
     DBuf<int> ord;          // rows of every 128 by length, longest first (format 0)
@@ -193,7 +193,7 @@ struct Sell {
     // order (for the warp-per-row kernels): row ids, offsets, entries.
     i64 n_lrows = 0;
     DBuf<int> lrow, lptr, lcol;
-    DBuf<float> lhi, llo;   // format 1
+    DBuf<float2> lhl;       // format 1
     DBuf<double> lw64;      // format 0
 };
 
@@ -266,7 +266,7 @@ struct Segmented {
     // rows of more than 32 entries, row-contiguous (original numbering)
     i64 n_long = 0;
     DBuf<int> l_row, l_ptr, l_col;
-    DBuf<float> l_hi, l_lo;
+    DBuf<float2> l_hl;
     DBuf<int> status;  // 1 = a bounded wait timed out
     std::mutex pool_mu;
     std::vector<cudaStream_t> pool;
@@ -378,14 +378,14 @@ void batch_apply(Batch &b, const float *const *x, const i64 *ldx, float *const *
 // staged.cu
 void build_blocked(Matrix &m, cudaStream_t s);
 bool blocked_eligible(const Matrix &m, const void *x, i64 ldx, bool bulk);
-void launch_long_rows(const int *row, const int *ptr, const int *col, const float *hi, const float *lo, i64 n,
-                      const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, cudaStream_t s, float *ylo, i64 ldylo);
+void launch_long_rows(const int *row, const int *ptr, const int *col, const float2 *hl, i64 n, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, cudaStream_t s, float *ylo, i64 ldylo);
 void build_segmented(Matrix &m, cudaStream_t s);
 void apply_segmented(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, cudaStream_t s, float *ylo,
                      i64 ldylo, int ns);
 void apply_blocked(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, int kind, int T, int ns,
                    i64 fchunk, cudaStream_t s, float *ylo = nullptr, i64 ldylo = 0);
 int blocked_launches(const Matrix &m);
+int split_launches(const Matrix &m);  // launches of a staged apply, long rows included
 // persistent staged kernels over the blocked layouts of several matrices
 // (batches); use[q] selects the matrices whose fields allow the staged kernels
 struct BlkBatch;

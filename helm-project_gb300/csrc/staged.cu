@@ -1728,7 +1728,24 @@ void build_segmented(Matrix &m, cudaStream_t s) {
     for (i64 r = 0; r < n; ++r)
         if (rp[r + 1] - rp[r] > 32) long_rows.push_back(static_cast<int>(r));
     rowlist(fb_rows, G.fb_row, G.fb_ptr, G.fb_col, G.fb_hi, G.fb_lo);
-    rowlist(long_rows, G.l_row, G.l_ptr, G.l_col, G.l_hi, G.l_lo);
+    {
+        std::vector<int> ptr(1, 0), c;
+        std::vector<float2> hl;
+        for (int r : long_rows) {
+            for (int k = rp[r]; k < rp[r + 1]; ++k) {
+                float h, l;
+                split(perm[k], h, l);
+                c.push_back(col[perm[k]]);
+                hl.push_back(make_float2(h, l));
+            }
+            ptr.push_back(static_cast<int>(c.size()));
+        }
+        G.l_row.upload_vec(long_rows, s);
+        G.l_ptr.upload_vec(ptr, s);
+        G.l_col.upload_vec(c, s);
+        G.l_hl.upload_vec(hl, s);
+        AXGB_CUDA(cudaStreamSynchronize(s));  // the vectors above are gone after this block
+    }
     G.n_fb = static_cast<i64>(fb_rows.size());
     G.n_long = static_cast<i64>(long_rows.size());
     G.grp.upload_vec(grp, s);
@@ -1792,7 +1809,7 @@ void apply_segmented(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, i64 
                                                                       ldylo);
     }
     if (G.n_long > 0)
-        launch_long_rows(G.l_row.p, G.l_ptr.p, G.l_col.p, G.l_hi.p, G.l_lo.p, G.n_long, x, ldx, y, ldy, nrhs,
+        launch_long_rows(G.l_row.p, G.l_ptr.p, G.l_col.p, G.l_hl.p, G.n_long, x, ldx, y, ldy, nrhs,
                          G.pool[q++ % 3], ylo, ldylo);
     AXGB_CUDA(cudaGetLastError());
     for (int k = 0; k < used; ++k) {

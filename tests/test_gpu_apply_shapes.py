@@ -145,3 +145,46 @@ def test_nan_apply_row_shapes(gpu, oracle, nf, weights, na_thres):
     y = gpu.nan_apply_f64(M, torch.tensor(X, device="cuda"), na_thres).cpu().numpy()
     assert np.array_equal(np.isnan(y), np.isnan(ref))
     assert np.array_equal(y[~np.isnan(y)], ref[~np.isnan(ref)])
+
+
+@pytest.mark.parametrize("nf", [1, 2, 3, 4, 5, 8, 9, 45])
+def test_unaligned_fields(gpu, oracle, nf):
+    """Fields whose rows do not start on 16 bytes (an odd number of cells, and
+    a view one element into a buffer): the same bits as from aligned rows,
+    the hi+lo form included."""
+    import torch
+    M = _rows_matrix(gpu, _mixed_lens(31), 4001, 32)
+    X = np.random.default_rng(33).standard_normal((nf, M.n_src)).astype(np.float32)
+    xs = torch.tensor(X, device="cuda")
+    pad = torch.zeros((nf, 4004), dtype=torch.float32, device="cuda")
+    pad[:, :4001] = xs
+    off = torch.zeros(nf * 4004 + 1, dtype=torch.float32, device="cuda")[1:].view(nf, 4004)
+    off[:, :4001] = xs
+    y, lo = gpu.apply_f32split_hilo(M, pad[:, :4001])
+    _check_split(y.cpu().numpy(), *_reference(M, oracle, X))
+    for x in (xs, off[:, :4001]):
+        y2, lo2 = gpu.apply_f32split_hilo(M, x)
+        assert torch.equal(y2, y) and torch.equal(lo2, lo)
+        assert torch.equal(gpu.apply_f32split(M, x), y)
+    for v, u in ((0, 1), (0, 2), (0, 4), (1, 4), (3, 4)):
+        assert torch.equal(gpu.apply_f32split(M, xs, fields_per_pass=3, unroll=u, variant=v), y)
+
+
+@pytest.mark.parametrize("nf", [1, 2, 3, 8, 40])
+def test_rows_too_scattered_to_stage(gpu, oracle, nf):
+    """Blocks of 128 rows that touch more source chunks than a staging slot
+    holds go to the direct kernel, slice by slice."""
+    import torch
+    rng = np.random.default_rng(41)
+    lens = rng.integers(20, 33, 400)
+    lens[128:256] = rng.integers(0, 4, 128)  # one block that is staged
+    rp = np.concatenate([[0], np.cumsum(lens)])
+    col = np.concatenate([np.sort(rng.choice(60000, n, replace=False)) for n in lens])
+    M = gpu.Matrix.from_csr(60000, 400, rp, col, rng.uniform(0.0, 1.0, rp[-1]))
+    X = rng.standard_normal((nf, M.n_src)).astype(np.float32)
+    xs = torch.tensor(X, device="cuda")
+    y = gpu.apply_f32split(M, xs, fields_per_pass=0, unroll=4, variant=3)
+    _check_split(y.cpu().numpy(), *_reference(M, oracle, X))
+    for v, fpp, u in ((0, 0, 1), (0, 4, 4), (1, 0, 4), (2, 0, 4), (4, 0, 1)):
+        assert torch.equal(gpu.apply_f32split(M, xs, fields_per_pass=fpp, unroll=u, variant=v), y)
+    assert torch.equal(gpu.apply_f32split(M, xs), y)

@@ -310,6 +310,7 @@ struct Matrix {
     // apply first gathers the fields into the new order.
     bool src_renum = false;
     DBuf<int> split_col, src_inv;
+    DBuf<int2> src_span;  // per kGatherTile new cells: least and greatest original cell
     // Per CSR entry, a key of its place in its row's generation order, for
     // the paths whose rows are not generated in column order (regular and
     // rectilinear conservative fast paths: candidate position; bilinear:
@@ -322,6 +323,8 @@ struct Matrix {
     std::map<i64, SplitParams> tuned;  // nrhs -> best kernel choice
     std::mutex mu;
 };
+
+constexpr int kGatherTile = 4096;  // new cells a block of the source gather takes
 
 struct Batch;
 

@@ -796,8 +796,15 @@ void plan_source_order(Matrix &m, const std::vector<int> &rp, std::vector<int> &
     std::vector<int> inv(ns);
     for (i64 c = 0; c < ns; ++c) inv[rank[c]] = static_cast<int>(c);
     for (i64 e = 0; e < nnz; ++e) col[e] = rank[col[e]];
+    std::vector<int2> span;
+    for (i64 t = 0; t < ns; t += kGatherTile) {
+        const auto mm = std::minmax_element(inv.begin() + t, inv.begin() + std::min<i64>(ns, t + kGatherTile));
+        span.push_back(make_int2(*mm.first, *mm.second));
+    }
     m.src_inv.upload_vec(inv, s);
+    m.src_span.upload_vec(span, s);
     m.split_col.upload_vec(col, s);
+    AXGB_CUDA(cudaStreamSynchronize(s));  // inv and span are gone after this call
     m.src_renum = true;
 }
 

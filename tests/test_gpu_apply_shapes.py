@@ -188,3 +188,31 @@ def test_rows_too_scattered_to_stage(gpu, oracle, nf):
     for v, fpp, u in ((0, 0, 1), (0, 4, 4), (1, 0, 4), (2, 0, 4), (4, 0, 1)):
         assert torch.equal(gpu.apply_f32split(M, xs, fields_per_pass=fpp, unroll=u, variant=v), y)
     assert torch.equal(gpu.apply_f32split(M, xs), y)
+
+
+@pytest.mark.parametrize("nf", [1, 3, 70])
+@pytest.mark.parametrize("window", [3000, 9000, 20003])
+def test_renumbered_sources(gpu, oracle, window, nf):
+    """Source cells numbered without locality inside windows of a latitude
+    band's size (gathered through shared memory) or of the whole mesh (gathered
+    from memory); an odd number of cells, the last tile and window in part."""
+    import torch
+    n_src, n_dst = 20003, 9000
+    rng = np.random.default_rng(51)
+    perm = np.concatenate([w + rng.permutation(min(window, n_src - w)) for w in range(0, n_src, window)])
+    lens = rng.integers(1, 8, n_dst)
+    rp = np.concatenate([[0], np.cumsum(lens)])
+    start = np.minimum(np.arange(n_dst) * n_src // n_dst, n_src - 8)
+    col = np.concatenate([np.sort(perm[s:s + n]) for s, n in zip(start, lens)])
+    M = gpu.Matrix.from_csr(n_src, n_dst, rp, col, rng.uniform(0.1, 1.0, rp[-1]))
+    X = rng.standard_normal((nf, n_src)).astype(np.float32)
+    xs = torch.tensor(X, device="cuda")
+    y = gpu.apply_f32split(M, xs)
+    assert M.stats()["source_renumbered"]
+    _check_split(y.cpu().numpy(), *_reference(M, oracle, X))
+    for v, fpp, u in ((0, 0, 2), (3, 8, 4), (4, 0, 1), (5, 0, 32)):
+        assert torch.equal(gpu.apply_f32split(M, xs, fields_per_pass=fpp, unroll=u, variant=v), y)
+    B = gpu.Batch([M], [nf])
+    yb = torch.empty_like(y)
+    B.apply([xs], [yb])
+    assert torch.equal(yb, y)

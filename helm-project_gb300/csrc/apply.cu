@@ -152,7 +152,7 @@ constexpr int kLongF = 8;  // fields per warp in the long-row kernels
 constexpr int kLongQ1 = 12;  // entries a lane loads ahead in a single-field long row
 constexpr int kLongQ1D = 8;  // the same in FP64
 constexpr int kLongQ = 4;   // the same with several fields
-constexpr int kBatchLongF = 4;  // fields per long-row item of the persistent batch kernel (k_batch<true>)
+constexpr int kBatchLongF = 8;  // fields per long-row item of the persistent batch kernel (k_batch<true>)
 
 // In-order pairwise tree over the 32 leaves (lane = leaf) for F values a
 // lane, F a power of two up to 32. While a lane holds more than one value,
@@ -1343,13 +1343,11 @@ double *noalloc_scratch() {
 // registers; longer rows are read from global memory.
 // ROWS: the row items (modes 1, 2), else the slice items (mode 0). The two
 // run as separate kernels: the slice items cache 16 entries a lane and need
-// about 128 registers (two blocks an SM); the row items are chains of
-// dependent gathers that want warps, so their kernel carries four fields a
-// long-row item and is held to 64 registers, four blocks an SM (measured on
-// the 17-pair batch: 1.14 ms, against 1.18 ms at three blocks, 1.23 ms with
-// two fields an item at five, 1.45 ms with eight fields at two).
+// about 128 registers (two blocks an SM); the long-row items carry eight
+// fields a warp in 80 registers, three blocks an SM, as k_split_long (17-pair
+// batch 1043 us, against 1096 us with four fields in 64 registers).
 template <bool ROWS>
-__global__ void __launch_bounds__(256, ROWS ? 4 : 2) k_batch(const Batch::Desc *__restrict__ desc, int n_desc, i64 total,
+__global__ void __launch_bounds__(256, ROWS ? 3 : 2) k_batch(const Batch::Desc *__restrict__ desc, int n_desc, i64 total,
                                                unsigned long long *counter) {
     const int lane = threadIdx.x & 31;
     while (true) {

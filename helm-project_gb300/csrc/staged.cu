@@ -59,6 +59,14 @@ constexpr int kPool = 4;         // streams the class launches are spread over
 // leave the sums unchanged.
 constexpr int kGroup = 4;
 const int kUsBuckets[] = {kUsSmall, kUsLarge};
+// Blocks of short rows (at most kShortL entries) that stage little, as under a
+// destination much finer than the source, are launched with a smaller stride
+// and more fields a stage (16, reduced four at a time; 8 in batches): what a
+// tile costs whatever its rows, the waits and copies, is then shared by more
+// fields. 100 fields of C48 -> 0.25 deg: 168 -> 146 us. (A stride of 512 with 8
+// fields for C192 -> 0.5 deg: 380 us against 371 for 500 fields.)
+constexpr int kUsTiny = 256, kTinyT = 16, kTinyBatchT = 8;
+constexpr int kShortL = 8;
 // Zero floats staged after a block's chunks, one in every shared-memory bank:
 // a padding read can then take a bank no entry of its gather step uses. A
 // block whose chunks nearly fill its staging stride gets what is left (at
@@ -423,15 +431,12 @@ __global__ void __launch_bounds__(kRows) k_blk_chunk(BlkArgs a, const float *__r
 // registers, so their classes are held to the counts that two staging slots
 // of 1024 floats a field also allow; the long-row classes take what they
 // need.
-template <int L, int NS>
+template <int L>
 constexpr int ws_min_blocks() {
-#ifdef WS_MINB16
-    if (L == 16 && NS == 2) return WS_MINB16;
-#endif
     return L <= 8 ? 6 : L <= 12 ? 5 : L <= 20 ? 4 : 1;
 }
 template <int L, int T, int NS, int US>
-__global__ void __launch_bounds__(kRows + 32, ws_min_blocks<L, NS>()) k_blk_ws(BlkArgs a, const float *__restrict__ x, i64 ldx,
+__global__ void __launch_bounds__(kRows + 32, ws_min_blocks<L>()) k_blk_ws(BlkArgs a, const float *__restrict__ x, i64 ldx,
                                                       float *__restrict__ y, i64 ldy, i64 nrhs) {
     static_assert(T % 2 == 0, "fields per stage must be even");
     static_assert(NS >= 2 && NS <= 3, "two or three ring slots");
@@ -500,7 +505,12 @@ __global__ void __launch_bounds__(kRows + 32, ws_min_blocks<L, NS>()) k_blk_ws(B
             atomicExch(a.status, 1);
             break;
         }
-        reduce_tile_c<L, T, US>(xs + s * T * US, li, h, lw, wl, t * T, nrhs, row, y, ldy, ylo, a.ldylo);
+        if constexpr (T <= 4) {
+            reduce_tile_c<L, T, US>(xs + s * T * US, li, h, lw, wl, t * T, nrhs, row, y, ldy, ylo, a.ldylo);
+        } else {
+            for (int g = 0; g < T && t * T + g < nrhs; g += 4)
+                reduce_tile_c<L, 4, US>(xs + (s * T + g) * US, li, h, lw, wl, t * T + g, nrhs, row, y, ldy, ylo, a.ldylo);
+        }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
     }
@@ -904,6 +914,18 @@ void build_blocked(Matrix &m, cudaStream_t s) {
     std::vector<float> hi, lo;
     std::map<std::pair<int, int>, std::vector<int>> cls;
     std::vector<int> fb;
+    // the stride of each short class: the small one where half of its blocks
+    // fit it (the others are then a launch of their own)
+    int short_us[2] = {kUsSmall, kUsSmall};
+    for (int c = 0; c < 2; ++c) {
+        i64 all = 0, tiny = 0;
+        for (const HostBlock &H : hb)
+            if (H.staged && H.rows[0] >= 0 && H.L == 4 * (c + 1)) {
+                ++all;
+                tiny += H.us <= kUsTiny;
+            }
+        if (2 * tiny >= all) short_us[c] = kUsTiny;
+    }
     for (i64 b = 0; b < nb; ++b) {
         HostBlock &H = hb[b];
         const int ebase = static_cast<int>(lidx.size());
@@ -923,7 +945,9 @@ void build_blocked(Matrix &m, cudaStream_t s) {
         if (H.staged) {
             int ub = 0;
             while (kUsBuckets[ub] < H.us) ++ub;
-            cls[{H.L, kUsBuckets[ub]}].push_back(static_cast<int>(b));
+            int us = kUsBuckets[ub];
+            if (H.L <= kShortL && H.us <= short_us[H.L <= 4 ? 0 : 1]) us = short_us[H.L <= 4 ? 0 : 1];
+            cls[{H.L, us}].push_back(static_cast<int>(b));
         } else {
             for (int g : groups[b])
                 if (g >= 0) fb.push_back(g);
@@ -953,9 +977,6 @@ void build_blocked(Matrix &m, cudaStream_t s) {
                      [&](int p1, int p2) { return B.launches[p1].n > B.launches[p2].n; });
     B.n_blocks = nb;
     B.n_src = m.n_src;
-    B.h_us.resize(nb);
-    for (i64 b = 0; b < nb; ++b) B.h_us[b] = hb[b].us;
-    B.h_block_ids = ids;
     B.brow.upload_vec(brow, s);
     B.wbase.upload_vec(wbase, s);
     B.wlen.upload_vec(wlen, s);
@@ -1042,6 +1063,15 @@ int ws_auto_stages() {
 template <int L, int T>
 void launch_ws(const BlkArgs &a, int us, int ns, i64 grid, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs,
                cudaStream_t s) {
+    if constexpr (L <= kShortL) {
+        if (us <= kUsTiny) {
+            BlkArgs b = a;
+            b.fchunk = (a.fchunk + kTinyT - 1) / kTinyT * kTinyT;
+            const i64 g = b.nbl * ((nrhs + b.fchunk - 1) / b.fchunk);
+            launch_ws_us<L, kTinyT, 2, kUsTiny>(b, g, x, ldx, y, ldy, nrhs, s);
+            return;
+        }
+    }
     if (us <= kUsSmall) {
         if (ns == 0) ns = ws_auto_stages<L, T>();
         if (ns >= 3)
@@ -1129,12 +1159,7 @@ namespace {
 
 constexpr int kBatchT = 4, kBatchNS = 2;
 constexpr i64 kBatchFChunk = 32;  // fields per work item
-// Short-row blocks (at most 8 entries a row) whose staging needs at most
-// kUsTiny floats a field (a coarse source under a fine destination) run in a
-// batch with that stride and 8 fields per stage: 16 KB of staging instead of
-// 32 KB, so more CTAs fit, and twice the work per tile.
-constexpr int kUsTiny = 256, kTinyT = 8, kTinyMaxL = 8;
-constexpr i64 kTinyFChunk = 64;  // fields per work item there (32 measured 6% slower on the 17-pair batch)
+constexpr i64 kTinyFChunk = 64;  // the same where little is staged (32 measured 6% slower on the 17-pair batch)
 
 BlkArgs blk_args(const Blocked &B, const Blocked::Launch &l, i64 n_src) {
     BlkArgs a{};
@@ -1169,17 +1194,20 @@ void persist_launch(const BlkDesc *d, int nd, i64 total, unsigned long long *cou
     k<<<static_cast<unsigned>(grid), kRows, bytes, s>>>(d, nd, total, counter);
 }
 
-template <int US>
+// Two fields a stage with the largest stride: 49 KB of staging, four CTAs an
+// SM, where four fields (two CTAs) leave it at eight row warps (17-pair batch
+// 1096 -> 1010 us; the producer-warp kernel is better off with four).
+template <int US, int T = US == kUsLarge ? 2 : kBatchT>
 void persist_dispatch(int L, const BlkDesc *d, int nd, i64 total, unsigned long long *counter, cudaStream_t s) {
     switch (L) {
-        case 4: persist_launch<4, US>(d, nd, total, counter, s); break;
-        case 8: persist_launch<8, US>(d, nd, total, counter, s); break;
-        case 12: persist_launch<12, US>(d, nd, total, counter, s); break;
-        case 16: persist_launch<16, US>(d, nd, total, counter, s); break;
-        case 20: persist_launch<20, US>(d, nd, total, counter, s); break;
-        case 24: persist_launch<24, US>(d, nd, total, counter, s); break;
-        case 28: persist_launch<28, US>(d, nd, total, counter, s); break;
-        default: persist_launch<32, US>(d, nd, total, counter, s); break;
+        case 4: persist_launch<4, US, T>(d, nd, total, counter, s); break;
+        case 8: persist_launch<8, US, T>(d, nd, total, counter, s); break;
+        case 12: persist_launch<12, US, T>(d, nd, total, counter, s); break;
+        case 16: persist_launch<16, US, T>(d, nd, total, counter, s); break;
+        case 20: persist_launch<20, US, T>(d, nd, total, counter, s); break;
+        case 24: persist_launch<24, US, T>(d, nd, total, counter, s); break;
+        case 28: persist_launch<28, US, T>(d, nd, total, counter, s); break;
+        default: persist_launch<32, US, T>(d, nd, total, counter, s); break;
     }
 }
 
@@ -1188,14 +1216,12 @@ void persist_dispatch(int L, const BlkDesc *d, int nd, i64 total, unsigned long 
 struct BlkBatch {
     struct Part {
         int mat, launch;
-        std::vector<int> ids;  // the launch's blocks in this group (empty: all of them)
     };
     struct Group {
         int L = 0, us = 0;
         std::vector<Part> parts;
         std::vector<BlkDesc> desc;
         DBuf<BlkDesc> d_desc;
-        DBuf<int> d_ids;  // concatenated block subsets of the parts that have one
         DBuf<unsigned long long> counter;
         i64 total = 0;
     };
@@ -1227,47 +1253,19 @@ std::shared_ptr<BlkBatch> blk_batch_create(const std::vector<Matrix *> &mats, co
         for (size_t li = 0; li < B.launches.size(); ++li) {
             const Blocked::Launch &l = B.launches[li];
             if (l.n == 0) continue;
-            if (l.L <= kTinyMaxL && l.us == kUsSmall && !B.h_block_ids.empty()) {
-                std::vector<int> tiny, rest;
-                for (i64 k = l.begin; k < l.begin + l.n; ++k) {
-                    const int b = B.h_block_ids[k];
-                    (B.h_us[b] <= kUsTiny ? tiny : rest).push_back(b);
-                }
-                if (!tiny.empty() && !rest.empty()) {
-                    add(l.L, kUsTiny, {static_cast<int>(q), static_cast<int>(li), std::move(tiny)});
-                    add(l.L, l.us, {static_cast<int>(q), static_cast<int>(li), std::move(rest)});
-                    continue;
-                }
-                if (!tiny.empty()) {
-                    add(l.L, kUsTiny, {static_cast<int>(q), static_cast<int>(li), {}});
-                    continue;
-                }
-            }
-            add(l.L, l.us, {static_cast<int>(q), static_cast<int>(li), {}});
+            add(l.L, l.us, {static_cast<int>(q), static_cast<int>(li)});
         }
     }
     for (auto &g : bb->groups) {
         g.d_desc.alloc(g.parts.size());
         g.counter.alloc(1);
         g.desc.resize(g.parts.size());
-        std::vector<int> ids;
-        std::vector<i64> off(g.parts.size(), -1);
-        for (size_t i = 0; i < g.parts.size(); ++i)
-            if (!g.parts[i].ids.empty()) {
-                off[i] = static_cast<i64>(ids.size());
-                ids.insert(ids.end(), g.parts[i].ids.begin(), g.parts[i].ids.end());
-            }
-        g.d_ids.upload_vec(ids);
         i64 items = 0;
         for (size_t i = 0; i < g.parts.size(); ++i) {
             const int q = g.parts[i].mat;
             const Blocked &B = mats[q]->blocked;
             BlkDesc &D = g.desc[i];
             D.a = blk_args(B, B.launches[g.parts[i].launch], mats[q]->n_src);
-            if (off[i] >= 0) {  // a subset of the launch's blocks
-                D.a.blocks = g.d_ids.p + off[i];
-                D.a.nbl = static_cast<i64>(g.parts[i].ids.size());
-            }
             D.a.us = g.us;
             D.a.fchunk = std::min<i64>(g.us <= kUsTiny ? kTinyFChunk : kBatchFChunk, nrhs[q]);
             D.nrhs = nrhs[q];
@@ -1276,7 +1274,6 @@ std::shared_ptr<BlkBatch> blk_batch_create(const std::vector<Matrix *> &mats, co
         }
         g.total = items;
     }
-    AXGB_CUDA(cudaDeviceSynchronize());  // the block subsets are uploaded before any launch reads them
     return bb;
 }
 
@@ -1308,11 +1305,12 @@ void blk_batch_launch(BlkBatch &bb, const cudaStream_t *streams, int n_streams) 
         auto &g = bb.groups[order[i]];
         cudaStream_t s = streams[i % n_streams];
         AXGB_CUDA(cudaMemsetAsync(g.counter.p, 0, sizeof(unsigned long long), s));
+        const int nd = static_cast<int>(g.desc.size());
         if (g.us <= kUsTiny) {
             if (g.L <= 4)
-                persist_launch<4, kUsTiny, kTinyT>(g.d_desc.p, static_cast<int>(g.desc.size()), g.total, g.counter.p, s);
+                persist_launch<4, kUsTiny, kTinyBatchT>(g.d_desc.p, nd, g.total, g.counter.p, s);
             else
-                persist_launch<8, kUsTiny, kTinyT>(g.d_desc.p, static_cast<int>(g.desc.size()), g.total, g.counter.p, s);
+                persist_launch<8, kUsTiny, kTinyBatchT>(g.d_desc.p, nd, g.total, g.counter.p, s);
         } else if (g.us <= kUsSmall)
             persist_dispatch<kUsSmall>(g.L, g.d_desc.p, static_cast<int>(g.desc.size()), g.total, g.counter.p, s);
         else

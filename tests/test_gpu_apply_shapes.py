@@ -216,3 +216,29 @@ def test_renumbered_sources(gpu, oracle, window, nf):
     yb = torch.empty_like(y)
     B.apply([xs], [yb])
     assert torch.equal(yb, y)
+
+
+@pytest.mark.parametrize("most", [4, 8])
+@pytest.mark.parametrize("nf", [8, 15, 16, 17, 31, 33, 100])
+def test_short_rows_little_staging(gpu, oracle, nf, most):
+    """A destination much finer than the source: short rows, few source chunks a
+    block, 16 fields a stage (8 in a batch), the last stage in part."""
+    import torch
+    rng = np.random.default_rng(61)
+    n_src, n_dst = 500, 3001
+    lens = rng.integers(0, most + 1, n_dst)
+    rp = np.concatenate([[0], np.cumsum(lens)])
+    start = np.minimum(np.arange(n_dst) * n_src // n_dst, n_src - 9)
+    col = np.concatenate([s + np.sort(rng.choice(9, n, replace=False)) for s, n in zip(start, lens)])
+    M = gpu.Matrix.from_csr(n_src, n_dst, rp, col, rng.uniform(0.1, 1.0, rp[-1]))
+    X = rng.standard_normal((nf, n_src)).astype(np.float32)
+    xs = torch.tensor(X, device="cuda")
+    y = gpu.apply_f32split(M, xs, fields_per_pass=0, unroll=4, variant=3)
+    _check_split(y.cpu().numpy(), *_reference(M, oracle, X))
+    for v, fpp, u in ((0, 0, 4), (1, 0, 8), (2, 0, 4), (3, 20, 4), (4, 0, 1)):
+        assert torch.equal(gpu.apply_f32split(M, xs, fields_per_pass=fpp, unroll=u, variant=v), y)
+    B = gpu.Batch([M, M], [nf, 5])
+    yb = [torch.empty((n, n_dst), dtype=torch.float32, device="cuda") for n in (nf, 5)]
+    B.apply([xs, xs[:5]], yb)
+    assert torch.equal(yb[0], y) and torch.equal(yb[1], y[:5])
+    assert M.device_status() == 0

@@ -41,38 +41,32 @@ struct GatherDesc {
 };
 
 struct Batch {
-    // One descriptor per (matrix, kind): mode 0 covers the slices whose rows
-    // have at most 32 entries (lane per row, items = field tile x slice);
-    // mode 1 the rows of at most 32 entries of the other slices (lane per
-    // field, items = 32-field chunk x row); mode 2 the rows of more than 32
-    // entries (lane per leaf, items = 8-field chunk x row).
+    // One descriptor per (matrix, kind): slice items (lane per row of at most 32
+    // entries, items = tile of kBatchTile fields x slice), or long-row items
+    // (rows of more than 32 entries, lane = leaf, items = kBatchLongF fields x row).
     struct Desc {
-        const int *base, *len, *rlen, *col;
+        const int *base, *rlen, *col;
         const float2 *hl;
-        const int *lrow, *lptr, *lcol;  // mode 2: row-contiguous long rows
+        const int *lrow, *lptr, *lcol;  // long rows, row-contiguous
         const float2 *lhl;
-        const int *ids;  // slice ids (modes 0, 1)
-        i64 n_ids;       // slices (modes 0, 1) or long rows (mode 2)
-        int mode;
+        const int *ids;  // slice ids (null: all slices)
+        i64 n_ids;       // slices or long rows
         int mat;  // index of the matrix in the batch
-        i64 n_rows, n_slices;
+        i64 n_rows;
         const float *x;
         i64 ldx;
         float *y;
         i64 ldy;
         i64 nrhs;
-        i64 tile;
-        i64 n_tiles;
         i64 item_begin;  // first global item of this matrix
     };
     std::vector<std::shared_ptr<Matrix>> mats;
     std::vector<i64> nrhs;
-    // descriptors: the slice items (mode 0) first, then the row items
-    // (modes 1, 2); each group has its own persistent kernel and counter
+    // descriptors: the slice items first, then the long-row items; each group
+    // has its own persistent kernel and counter
     std::vector<Desc> desc;
     DBuf<Desc> d_desc;
     DBuf<unsigned long long> counter;  // [0]: slice items, [1]: row items
-    i64 total_items = 0;               // both groups
     i64 total_slice_items = 0, total_row_items = 0;
     int n_slice_desc = 0;
     int blocks_slices = 0, blocks_rows = 0;
@@ -120,8 +114,7 @@ inline unsigned nblk(i64 n, int t) { return static_cast<unsigned>((n + t - 1) / 
 
 struct SellArgs {
     const int *ids;
-    i64 n_ids;
-    const int *base, *len, *rlen, *col;
+    const int *base, *rlen, *col;
     const float2 *hl;  // (hi, lo)
     const double *w64;
     i64 n_rows;
@@ -752,26 +745,6 @@ void build_sell(Matrix &m, int fmt, cudaStream_t s) {
                                                             fmt == 0 ? S.w64.p : nullptr, fmt == 0 ? S.total.p : nullptr);
         AXGB_CUDA(cudaGetLastError());
     }
-    // length classes on the host
-    std::vector<int> h_len(n_slices);
-    if (n_slices) AXGB_CUDA(cudaMemcpy(h_len.data(), slen32.p, sizeof(int) * n_slices, cudaMemcpyDeviceToHost));
-    const int bounds[5] = {8, 16, 32, 64, 1 << 30};
-    std::vector<std::vector<int>> cls(5);
-    for (i64 q = 0; q < n_slices; ++q) {
-        int L = h_len[q] / 32;
-        int c = 0;
-        while (L > bounds[c]) ++c;
-        cls[c].push_back(static_cast<int>(q));
-    }
-    std::vector<int> ids;
-    S.class_begin.assign(6, 0);
-    S.class_maxlen.assign(5, 0);
-    for (int c = 0; c < 5; ++c) {
-        S.class_begin[c] = static_cast<i64>(ids.size());
-        for (int q : cls[c]) S.class_maxlen[c] = std::max(S.class_maxlen[c], h_len[q] / 32);
-        ids.insert(ids.end(), cls[c].begin(), cls[c].end());
-    }
-    S.class_begin[5] = static_cast<i64>(ids.size());
     // rows of more than 32 entries, row-contiguous
     {
         std::vector<int> rp(n_rows + 1);
@@ -802,23 +775,17 @@ void build_sell(Matrix &m, int fmt, cudaStream_t s) {
             AXGB_CUDA(cudaGetLastError());
         }
     }
-    S.class_ids.upload(ids.data(), ids.size(), s);
-    S.h_slice_len.resize(n_slices);
-    for (i64 q = 0; q < n_slices; ++q) S.h_slice_len[q] = h_len[q] / 32;
     // keep row lengths in the len buffer's companion: store rlen in 'len' slot
     S.len = std::move(rlen);
     AXGB_CUDA(cudaStreamSynchronize(s));
     S.built = true;
 }
 
-SellArgs sell_args(const Matrix &m, const Sell &S, int cls, float *ylo = nullptr, i64 ldylo = 0) {
+SellArgs sell_args(const Matrix &m, const Sell &S, float *ylo = nullptr, i64 ldylo = 0) {
     SellArgs a{};
     a.ylo = ylo;
     a.ldylo = ldylo;
-    a.ids = S.class_ids.p + S.class_begin[cls];
-    a.n_ids = S.class_begin[cls + 1] - S.class_begin[cls];
     a.base = S.base.p;
-    a.len = nullptr;
     a.rlen = S.len.p;
     a.col = S.col.p;
     a.hl = S.hl.p;
@@ -883,7 +850,7 @@ void launch_split_fused(const Matrix &m, const Sell &S, const float *x, i64 ldx,
     LongRows L = long_rows(S);
     L.ylo = ylo;
     L.ldylo = ldylo;
-    SellArgs a = sell_args(m, S, 0, ylo, ldylo);
+    SellArgs a = sell_args(m, S, ylo, ldylo);
     a.ids = ids;
     const i64 n_slices = ids ? n_ids : S.n_slices;
     const int n_long = ids ? 0 : static_cast<int>(L.n);
@@ -915,7 +882,7 @@ void launch_f64_fused(const Matrix &m, const Sell &S, const double *x, i64 ldx, 
                       cudaStream_t s) {
     const i64 warps = S.n_slices + S.n_lrows;
     if (warps == 0 || nrhs == 0) return;
-    const SellArgs a = sell_args(m, S, 0);
+    const SellArgs a = sell_args(m, S);
     const LongRows L = long_rows(S);
     // Fields of a short row's warp: up to 64, so that its entries are read once
     // from L2 and the tile's other passes find them in L1; fewer, down to 8,
@@ -1337,18 +1304,16 @@ double *noalloc_scratch() {
     return ptr[dev];
 }
 
-// ─── persistent batch kernel ───────────────────────────────────────────────
-// Items of all matrices are handed out by one atomic counter (no waiting):
-// item -> (matrix, tile, slice). Entries of up to 32 per row are cached in
-// registers; longer rows are read from global memory.
-// ROWS: the row items (modes 1, 2), else the slice items (mode 0). The two
-// run as separate kernels: the slice items cache 16 entries a lane and need
-// about 128 registers (two blocks an SM); the long-row items carry eight
-// fields a warp in 80 registers, three blocks an SM, as k_split_long (17-pair
-// batch 1043 us, against 1096 us with four fields in 64 registers).
+// ─── persistent batch kernels ──────────────────────────────────────────────
+// Items of all matrices are handed out by one atomic counter (no waiting).
+// ROWS: the long-row items, else the slice items, with the row functions of
+// the direct kernel: eight fields side by side in 80 registers, three blocks
+// an SM (17-pair batch 1043 us, against 1096 us with four fields a long row in
+// 64 registers).
+constexpr int kBatchTile = 8;  // fields of a slice item
 template <bool ROWS>
 __global__ void __launch_bounds__(256, ROWS ? 3 : 2) k_batch(const Batch::Desc *__restrict__ desc, int n_desc, i64 total,
-                                               unsigned long long *counter) {
+                                                  unsigned long long *counter) {
     const int lane = threadIdx.x & 31;
     while (true) {
         unsigned long long it = 0;
@@ -1359,77 +1324,33 @@ __global__ void __launch_bounds__(256, ROWS ? 3 : 2) k_batch(const Batch::Desc *
         while (m + 1 < n_desc && desc[m + 1].item_begin <= static_cast<i64>(it)) ++m;
         const Batch::Desc &d = desc[m];
         const i64 local = static_cast<i64>(it) - d.item_begin;
+        const i64 t = local / d.n_ids, i = local - t * d.n_ids;
         if constexpr (ROWS) {
-        if (d.mode == 2) {  // rows of more than 32 entries
             LongRows L{};
             L.row = d.lrow;
             L.ptr = d.lptr;
             L.col = d.lcol;
             L.hl = d.lhl;
-            L.w64 = nullptr;
             L.n = d.n_ids;
-            split_long_row<kBatchLongF>(L, local % L.n, local / L.n, d.x, d.ldx, d.y, d.ldy, d.nrhs);
-            continue;
-        }
-        if (d.mode == 1) {  // short rows of long-class slices: lane = field
-            const i64 per = d.n_ids * 32;
-            const i64 fc = local / per;
-            const i64 q = local - fc * per;
-            const int sid = d.ids[q >> 5];
-            const int p = static_cast<int>(q & 31);
-            const i64 row = static_cast<i64>(sid) * 32 + p;
-            const i64 f = fc * 32 + lane;
-            if (row < d.n_rows && f < d.nrhs) {
+            split_long_row<kBatchLongF>(L, i, t, d.x, d.ldx, d.y, d.ldy, d.nrhs);
+        } else {
+            const i64 sid = d.ids ? d.ids[i] : i;
+            const i64 row = sid * 32 + lane;
+            if (row < d.n_rows) {
                 const int n = d.rlen[row];
+                SellArgs a{};
+                a.col = d.col;
+                a.hl = d.hl;
+                const i64 f = t * kBatchTile;
+                const int nf = static_cast<int>(d.nrhs - f < kBatchTile ? d.nrhs - f : kBatchTile);
                 if (n <= 32) {
-                    const int e0 = d.base[sid] + p;
-                    const float *xf = d.x + f * d.ldx;
-                    float s = 0.f, c = 0.f;
-                    for (int k = 0; k < n; ++k) {
-                        const int e = e0 + 32 * k;
-                        csum1(s, c, d.hl[e].x, d.hl[e].y, __ldg(xf + d.col[e]));
-                    }
-                    d.y[f * d.ldy + row] = __fadd_rn(s, c);
+                    if (nf == kBatchTile)
+                        short_rows<kBatchTile, 2, true>(a, n, d.base[sid] + lane, row, d.x, d.ldx, d.y, d.ldy, f, nf);
+                    else
+                        short_rows<kBatchTile, 2, false>(a, n, d.base[sid] + lane, row, d.x, d.ldx, d.y, d.ldy, f, nf);
                 }
             }
-            continue;
-        }
-        } else {
-        const i64 t = local / d.n_ids;
-        const i64 sid = d.ids[local - t * d.n_ids];
-        const i64 row = sid * 32 + lane;
-        const int base = d.base[sid];
-        const int rl = d.rlen[sid * 32 + lane];
-        const i64 f0 = t * d.tile, f1 = min(f0 + d.tile, d.nrhs);
-        const bool store = row < d.n_rows;
-        constexpr int L = 16;
-        int c[L];
-        float h[L], lw[L];
-#pragma unroll
-        for (int k = 0; k < L; ++k) {
-            if (k < rl) {
-                int e = base + k * 32 + lane;
-                c[k] = d.col[e];
-                h[k] = d.hl[e].x;
-                lw[k] = d.hl[e].y;
-            } else {
-                c[k] = 0;
-                h[k] = 0.f;
-                lw[k] = 0.f;
-            }
-        }
-        for (i64 f = f0; f < f1; ++f) {
-            float s = 0.f, cc = 0.f;
-            const float *xf = d.x + f * d.ldx;
-#pragma unroll
-            for (int k = 0; k < L; ++k)
-                if (k < rl) csum1(s, cc, h[k], lw[k], __ldg(xf + c[k]));
-            for (int k = L; k < rl; ++k) {  // rows of 17..32 entries: the tail from global memory
-                int e = base + k * 32 + lane;
-                csum1(s, cc, d.hl[e].x, d.hl[e].y, __ldg(xf + d.col[e]));
-            }
-            if (store) d.y[f * d.ldy + row] = __fadd_rn(s, cc);
-        }
+            __syncwarp();
         }
     }
 }
@@ -1449,13 +1370,7 @@ void matrix_prepare(Matrix &m, int format, cudaStream_t s) {
         return;
     }
     build_sell(m, format == 0 ? 0 : 1, s);
-    if (format == 1) {
-        const Sell &S = m.sell32;
-        int launches = 0;
-        for (int c = 0; c < 5; ++c)
-            if (S.class_begin[c + 1] > S.class_begin[c]) ++launches;
-        m.stats[5] = launches;
-    }
+    if (format == 1) m.stats[5] = 1;  // the direct kernel is one launch
 }
 
 namespace {
@@ -1653,7 +1568,7 @@ void nan_batch_apply_f64(Matrix &m, const double *x, i64 ldx, double *y, i64 ldy
     for (i64 f = 0; f < nrhs; f += 65535 * kNanG) {
         const i64 nf = std::min<i64>(nrhs - f, 65535 * kNanG);
         const dim3 grid(nblk(warps, 8), nblk(nf, kNanG));
-        k_nan<<<grid, 256, 0, s>>>(sell_args(m, S, 0), long_rows(S), S.total.p, S.ord.p, S.n_slices, x + f * ldx, ldx,
+        k_nan<<<grid, 256, 0, s>>>(sell_args(m, S), long_rows(S), S.total.p, S.ord.p, S.n_slices, x + f * ldx, ldx,
                                    y + f * ldy, ldy, nf, na_thres);
     }
     AXGB_CUDA(cudaGetLastError());
@@ -1684,25 +1599,19 @@ std::shared_ptr<Batch> batch_create(const std::vector<std::shared_ptr<Matrix>> &
 
 namespace {
 
-// Work of the direct persistent kernel: for a matrix on the staged kernels,
-// the slices the blocked layout leaves out (their rows of at most 32
-// entries) and the rows of more than 32 entries; for the others, all of it.
+// Work of the direct persistent kernels: for a matrix on the staged kernels,
+// the slices the blocked layout leaves out, for the others all slices; and
+// the rows of more than 32 entries.
 void plan_direct(Batch &b) {
     b.desc.clear();
-    i64 items = 0;
-    b.n_slice_desc = 0;
-    b.total_slice_items = 0;
-    for (int group = 0; group < 2; ++group) {  // slice items (mode 0), then row items (modes 1, 2)
-    items = 0;
-    for (size_t q = 0; q < b.mats.size(); ++q) {
-        Matrix &m = *b.mats[q];
-        const Sell &S = m.sell32;
-        const i64 k = b.nrhs[q];
-        for (int mode = 0; mode < 3; ++mode) {
-            if ((mode == 0) != (group == 0)) continue;
+    for (int group = 0; group < 2; ++group) {  // slice items, then long-row items
+        i64 items = 0;
+        for (size_t q = 0; q < b.mats.size(); ++q) {
+            Matrix &m = *b.mats[q];
+            const Sell &S = m.sell32;
+            const i64 k = b.nrhs[q];
             Batch::Desc d{};
             d.base = S.base.p;
-            d.len = nullptr;
             d.rlen = S.len.p;
             d.col = S.col.p;
             d.hl = S.hl.p;
@@ -1710,42 +1619,31 @@ void plan_direct(Batch &b) {
             d.lptr = S.lptr.p;
             d.lcol = S.lcol.p;
             d.lhl = S.lhl.p;
-            d.mode = mode;
             d.mat = static_cast<int>(q);
             d.n_rows = m.n_dst;
-            d.n_slices = S.n_slices;
             d.nrhs = k;
-            d.tile = std::max<i64>(1, std::min<i64>(k, 8));
-            d.n_tiles = (k + d.tile - 1) / d.tile;
-            if (mode == 2) {
+            if (group == 1) {
                 d.n_ids = S.n_lrows;
             } else if (b.use[q]) {
-                if (mode == 0) continue;
-                d.ids = m.blocked.fallback_slices.p;  // classes of the blocked layout's left-out slices
+                d.ids = m.blocked.fallback_slices.p;
                 d.n_ids = m.blocked.n_fallback;
             } else {
-                // classes 0..2: slices of rows of at most 32 entries; 3..4: the others
-                const i64 c0 = S.class_begin[mode == 0 ? 0 : 3], c1 = S.class_begin[mode == 0 ? 3 : 5];
-                d.ids = S.class_ids.p + c0;
-                d.n_ids = c1 - c0;
+                d.n_ids = S.n_slices;
             }
-            const i64 n_items = mode == 0   ? d.n_tiles * d.n_ids
-                                : mode == 1 ? d.n_ids * 32 * ((k + 31) / 32)
-                                            : d.n_ids * ((k + kBatchLongF - 1) / kBatchLongF);
+            const i64 per = group == 0 ? kBatchTile : kBatchLongF;
+            const i64 n_items = d.n_ids * ((k + per - 1) / per);
             if (n_items == 0) continue;
             d.item_begin = items;
             items += n_items;
             b.desc.push_back(d);
         }
+        if (group == 0) {
+            b.n_slice_desc = static_cast<int>(b.desc.size());
+            b.total_slice_items = items;
+        } else {
+            b.total_row_items = items;
+        }
     }
-    if (group == 0) {
-        b.n_slice_desc = static_cast<int>(b.desc.size());
-        b.total_slice_items = items;
-    } else {
-        b.total_row_items = items;
-    }
-    }
-    b.total_items = b.total_slice_items + b.total_row_items;
     b.d_desc.alloc(std::max<size_t>(1, b.desc.size()));
 }
 

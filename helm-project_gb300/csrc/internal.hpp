@@ -184,11 +184,6 @@ struct Sell {
     DBuf<double> w64;       // FP64 weights (format 0)
     DBuf<double> total;     // sum of each row's weights in CSR order (format 0; NaN-aware apply)
     DBuf<int> ord;          // rows of every 128 by length, longest first (format 0)
-    // slice ids grouped by length class: <=8, <=16, <=32, <=64, >64
-    std::vector<i64> class_begin;  // 6 entries into class_ids
-    DBuf<int> class_ids;
-    std::vector<int> class_maxlen;
-    std::vector<int> h_slice_len;  // entries per row slot of each slice
     // Rows of more than 32 entries, row-contiguous in the layout's entry
     // order (for the warp-per-row kernels): row ids, offsets, entries.
     i64 n_lrows = 0;

@@ -150,7 +150,7 @@ int axgb_generate_weights_c(int src_mesh, int dst_mesh, int method, int *matrix_
  * axgb_matrix_prepare of its format), and 1 when the split layouts renumber
  * the source cells (known after axgb_matrix_prepare of format 1 or 2; a
  * split apply then first gathers the fields into that order, in scratch of
- * the fields' size taken with cudaMallocAsync on the apply's stream).
+ * the fields' size taken from the library's memory pool on the apply's stream).
  * times_ms (double[8]): cell prep,
  * LBVH build, candidate search, clip, CSR assembly, total, 0, 0. */
 int axgb_matrix_stats(int matrix_handle, int64_t *stats, double *times_ms);

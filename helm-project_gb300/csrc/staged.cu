@@ -30,6 +30,7 @@
 // with packed f32x2 compensated arithmetic (fp32x2.cuh).
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <cstdint>
 #include <map>
 #include <memory>
@@ -51,7 +52,7 @@ constexpr int kUsSmall = 256 * kWarps;
 constexpr int kUsLarge = 768 * kWarps;
 constexpr int kMaxUS = kUsLarge;  // staging floats per field a block may use
 constexpr int kMaxL = 32;        // longest row handled by the blocked kernels
-constexpr int kPool = 4;         // streams the class launches are spread over
+constexpr int kPool = 3;         // streams the class launches are spread over, besides the caller's
 // A warp steps through its entries in whole groups of kGroup (straight-line
 // code, so the scheduler overlaps the compensated steps of neighbouring
 // entries) and then through the 1 .. kGroup-1 entries left up to its longest
@@ -1010,11 +1011,23 @@ int blocked_launches(const Matrix &m) {
 
 namespace {
 
+// Allows `kernel` its dynamic shared memory, once a device (the call costs
+// about as much as a launch).
+template <auto kernel>
+void allow_smem(size_t bytes) {
+    static std::atomic<unsigned long long> done{0};  // bit per device
+    int dev = 0;
+    AXGB_CUDA(cudaGetDevice(&dev));
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+    if (done.load(std::memory_order_acquire) & bit) return;
+    AXGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+    done.fetch_or(bit, std::memory_order_release);
+}
+
 template <int L, int T, int NS, int US>
 void launch_chunk_us(const BlkArgs &a, i64 grid, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, cudaStream_t s) {
     size_t bytes = sizeof(float) * static_cast<size_t>(US) * NS * T + sizeof(int) * static_cast<size_t>(US / 4);
-    AXGB_CUDA(cudaFuncSetAttribute(k_blk_chunk<L, T, NS, US>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(bytes)));
+    allow_smem<k_blk_chunk<L, T, NS, US>>(bytes);
     k_blk_chunk<L, T, NS, US><<<static_cast<unsigned>(grid), kRows, bytes, s>>>(a, x, ldx, y, ldy, nrhs);
 }
 
@@ -1035,8 +1048,7 @@ void launch_chunk(const BlkArgs &a, int us, int ns, i64 grid, const float *x, i6
 template <int L, int T, int NS, int US>
 void launch_ws_us(const BlkArgs &a, i64 grid, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, cudaStream_t s) {
     size_t bytes = sizeof(float) * static_cast<size_t>(US) * NS * T + sizeof(int) * static_cast<size_t>(US / 4);
-    AXGB_CUDA(cudaFuncSetAttribute(k_blk_ws<L, T, NS, US>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(bytes)));
+    allow_smem<k_blk_ws<L, T, NS, US>>(bytes);
     k_blk_ws<L, T, NS, US><<<static_cast<unsigned>(grid), kRows + 32, bytes, s>>>(a, x, ldx, y, ldy, nrhs);
 }
 
@@ -1335,12 +1347,14 @@ void apply_blocked(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, i64 nr
         }
         AXGB_CUDA(cudaEventCreateWithFlags(&B.fork, cudaEventDisableTiming));
     }
-    AXGB_CUDA(cudaEventRecord(B.fork, s));
-    const int used = static_cast<int>(std::min<size_t>(kPool, B.order.size()));
+    // the largest class stays on the caller's stream, the others go round the pool
+    const int used = static_cast<int>(std::min<size_t>(kPool, B.order.empty() ? 0 : B.order.size() - 1));
+    if (used > 0) AXGB_CUDA(cudaEventRecord(B.fork, s));
     for (int q = 0; q < used; ++q) AXGB_CUDA(cudaStreamWaitEvent(B.pool[q], B.fork, 0));
     for (size_t i = 0; i < B.order.size(); ++i) {
         const Blocked::Launch &l = B.launches[B.order[i]];
-        cudaStream_t st = B.pool[i % kPool];
+        const size_t slot = i % (kPool + 1);
+        cudaStream_t st = slot == 0 ? s : B.pool[slot - 1];
         if (T >= 8)
             launch_class<8>(B, l, kind, ns, x, ldx, y, ldy, nrhs, fchunk, st, ylo, ldylo);
         else if (T >= 4)

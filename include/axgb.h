@@ -255,8 +255,8 @@ int axgb_apply_f32split_hilo(int matrix_handle, const float *x, int64_t ld_x, fl
                              int64_t ld_lo, int64_t nrhs, axgb_stream_t stream);
 
 /* Same, kernel choice explicit. variant 0: direct gathers from global
- * memory, fields_per_pass = RHS tile width (0 = all), unroll = fields per
- * thread iteration (1, 2 or 4). variants 1 to 3: rows in blocks of 4
+ * memory in one launch, fields_per_pass = fields a thread walks (0 = all),
+ * unroll = fields side by side in a thread (1, 2 or 4). variants 1 to 3: rows in blocks of 4
  * slices grouped by source locality; per block the source values are staged
  * in shared memory as 16-byte chunks, variant 1 with cp.async by all
  * threads (two staging buffers), variant 2 with bulk (TMA) copies completing
@@ -265,12 +265,13 @@ int axgb_apply_f32split_hilo(int matrix_handle, const float *x, int64_t ld_x, fl
  * fields per stage (2, 4 or 8),
  * fields_per_pass = fields per work item of a block (0 = all). Variants 1
  * to 3 need x 16-byte aligned and ld_x a multiple of 4 (variant 2 also n_src
- * a multiple of 4); otherwise the direct kernel runs. variant 4: the whole
- * matrix in one launch (for one or a few fields); the other knobs are
- * unused. variant 5: segmented, one lane per field: groups of 32 nearby
- * rows stage their distinct source cells (original numbering, any x
- * alignment) for 32 fields at a time; stages = staging slots (2 or 3).
- * Every variant gives the same bits. */
+ * a multiple of 4); otherwise the direct kernel runs. variant 4: the direct
+ * kernel with its own tile and unroll (the default for one or two fields,
+ * and while weights * fields is at most 4 million for each launch that the
+ * staged form would take); the other knobs are unused. variant 5: segmented,
+ * one lane per field: groups of 32 nearby rows stage their distinct source
+ * cells (original numbering, any x alignment) for 32 fields at a time;
+ * stages = staging slots (2 or 3). Every variant gives the same bits. */
 int axgb_apply_f32split_tuned(int matrix_handle, const float *x, int64_t ld_x, float *y, int64_t ld_y, int64_t nrhs,
                               int variant, int fields_per_pass, int unroll, axgb_stream_t stream);
 

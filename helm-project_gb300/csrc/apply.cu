@@ -130,6 +130,8 @@ __device__ __forceinline__ float ldg_f(const float *p) { return __ldg(p); }
 // leaf of the order in fp32x2.cuh, the F fields carried side by side, entries
 // read row-contiguous (Sell::lcol/lhi/llo), shuffle tree at the end.
 constexpr int kF64F = 4;          // fields an FP64 row carries side by side
+constexpr int kOrdGain = 16;       // twentieths, see rows_by_length
+constexpr int kOrdPlain = static_cast<int>(0x80000000u);  // in Sell::ord: the group gains little
 constexpr int kFusedK = 4;        // entries a row of the fused kernels loads before gathering
 constexpr int kF64K = 2;          // the same of the FP64 kernel from three fields up
 
@@ -574,7 +576,8 @@ __global__ void __launch_bounds__(256, 4) k_f64_fused(SellArgs a, LongRows L, co
     const i64 t = nrhs <= tile ? 0 : w / n_slices, pos = (w - t * n_slices) * 32 + lane;
     const i64 fa = t * tile, fb = min(fa + tile, nrhs);
     if (fa >= nrhs) return;
-    const i64 row = F > 2 ? ord[pos] : pos;
+    const int o = F > 2 ? ord[pos] : kOrdPlain;
+    const i64 row = o & kOrdPlain ? pos : o;
     if (row >= a.n_rows) return;
     const int n = a.rlen[row];
     if (n > 32) return;
@@ -694,6 +697,14 @@ __global__ void k_sell_fill(const int *rp, const int *ccol, const double *val, c
 // 1% of 256 (16 NaN fields of 0.25 deg -> C384 651 / 646 us, 20 FP64 fields of
 // C384 -> 1 deg 121 / 125, 300 of C384 -> 0.25 deg 2836 / 2867); 64 is slower
 // on the first (665).
+//
+// Out of row order a warp's entries, gathers and stores touch more sectors, which
+// the plain FP64 kernel (one operation an entry) notices: where the order
+// leaves more than 0.8 of a group's steps, the group is flagged kOrdPlain and
+// that kernel keeps its row order. 64 fields of a 2.6 M-cell Voronoi mesh (in a
+// numbering that is not local) -> 0.1 deg, most groups near 0.8: 3.24 ms, 3.81
+// with every group in order of length, 3.09 with the line at 0.75; there 64
+// fields of C192 -> 0.5 deg, by length 171 us, take 183 (174 at 0.8).
 std::vector<int> rows_by_length(const std::vector<int> &rp, i64 n_rows, i64 n_pos) {
     std::vector<int> ord(n_pos);
     for (i64 g = 0; g < n_pos; g += 128) {
@@ -706,6 +717,18 @@ std::vector<int> rows_by_length(const std::vector<int> &rp, i64 n_rows, i64 n_po
         for (i64 r = g; r < e; ++r) ++at[33 - len(r)];
         for (int k = 1; k < 34; ++k) at[k] += at[k - 1];
         for (i64 r = g; r < e; ++r) ord[g + at[32 - len(r)]++] = static_cast<int>(r);
+        int plain = 0, sorted = 0;  // steps of the four warps in either order
+        for (i64 q = g; q < e; q += 32) {
+            int lp = 0, ls = 0;
+            for (i64 r = q; r < q + 32; ++r) {
+                lp = std::max(lp, len(r));
+                ls = std::max(ls, len(ord[r]));
+            }
+            plain += lp;
+            sorted += ls;
+        }
+        if (sorted * 20 > plain * kOrdGain)
+            for (i64 r = g; r < e; ++r) ord[r] |= kOrdPlain;
     }
     return ord;
 }
@@ -1032,7 +1055,7 @@ __global__ void __launch_bounds__(256) k_nan(SellArgs a, LongRows L, const doubl
     }
     const i64 sid = wg - L.n;
     if (sid >= n_slices) return;
-    const i64 row = ord[sid * 32 + lane];
+    const i64 row = ord[sid * 32 + lane] & ~kOrdPlain;
     const bool live = row < a.n_rows && a.rlen[row] <= 32;
     const int n = live ? a.rlen[row] : 0;
     const int base = a.base[row >> 5] + static_cast<int>(row & 31);

@@ -183,7 +183,7 @@ struct Sell {
     DBuf<float2> hl;        // split weights (hi, lo) (format 1)
     DBuf<double> w64;       // FP64 weights (format 0)
     DBuf<double> total;     // sum of each row's weights in CSR order (format 0; NaN-aware apply)
-    DBuf<int> ord;          // rows of every 128 by length, longest first (format 0)
+    DBuf<int> ord;          // rows of every 128 by length, longest first, with kOrdPlain (format 0)
     // Rows of more than 32 entries, row-contiguous in the layout's entry
     // order (for the warp-per-row kernels): row ids, offsets, entries.
     i64 n_lrows = 0;

@@ -112,6 +112,22 @@ def test_f64_field_tiles(gpu, oracle, nf, rows):
         assert np.array_equal(gpu.apply_f64(M, xs[f:f + 1]).cpu().numpy()[0], d[f])
 
 
+@pytest.mark.parametrize("lens", [[3], [1, 8], [4] * 31 + [5], list(range(33)), [2] * 128 + [1, 30], [40] + [0] * 40 + [2]],
+                         ids=["equal", "alternating", "one longer", "ascending", "by group", "empty"])
+@pytest.mark.parametrize("nf,rows", [(3, 127), (4, 129), (9, 1001)])
+def test_f64_row_orders(gpu, oracle, nf, rows, lens):
+    """FP64 applies whose groups of rows run in their own order and by length,
+    the last group in part: from three fields up, against one field."""
+    import torch
+    M = _rows_matrix(gpu, np.resize(lens, rows).astype(np.int64), 900, 41)
+    X = np.random.default_rng(42).standard_normal((nf, M.n_src))
+    xs = torch.tensor(X, device="cuda")
+    d = gpu.apply_f64(M, xs).cpu().numpy()
+    _check_f64(d, *_reference(M, oracle, X))
+    for f in range(nf):
+        assert np.array_equal(gpu.apply_f64(M, xs[f:f + 1]).cpu().numpy()[0], d[f])
+
+
 @pytest.mark.parametrize("nf", [1, 3, 16, 17, 37])
 @pytest.mark.parametrize("weights,na_thres", [("positive", 0.5), ("positive", 0.0), ("positive", 1.0), ("signed", 0.5),
                                               ("positive", -1.0), ("tiny", 0.3)])

@@ -702,9 +702,10 @@ __global__ void k_sell_fill(const int *rp, const int *ccol, const double *val, c
 // the plain FP64 kernel (one operation an entry) notices: where the order
 // leaves more than 0.8 of a group's steps, the group is flagged kOrdPlain and
 // that kernel keeps its row order. 64 fields of a 2.6 M-cell Voronoi mesh (in a
-// numbering that is not local) -> 0.1 deg, most groups near 0.8: 3.24 ms, 3.81
-// with every group in order of length, 3.09 with the line at 0.75; there 64
-// fields of C192 -> 0.5 deg, by length 171 us, take 183 (174 at 0.8).
+// numbering that is not local) -> 0.1 deg: 3.13 ms, 3.78 with every group in
+// order of length; 1016 of C768 -> 0.25 deg 21.1 against 24.2. With the line at
+// 0.75 the first is another 5% faster, but 64 fields of C192 -> 0.5 deg take
+// 183 us instead of 171.
 std::vector<int> rows_by_length(const std::vector<int> &rp, i64 n_rows, i64 n_pos) {
     std::vector<int> ord(n_pos);
     for (i64 g = 0; g < n_pos; g += 128) {
@@ -909,9 +910,10 @@ void launch_f64_fused(const Matrix &m, const Sell &S, const double *x, i64 ldx, 
     const LongRows L = long_rows(S);
     // Fields of a short row's warp: up to 64, so that its entries are read once
     // from L2 and the tile's other passes find them in L1; fewer, down to 8,
-    // where that would leave less than about four waves of warps. 300 fields of
-    // C384 -> 0.25 deg: 3.58 ms with 64, 3.91 with 16, 4.70 with all; 20 fields
-    // of C384 -> 1 deg: 148 us with 8, 191 with 16.
+    // where that would leave less than about four waves of warps. With all rows
+    // in row order, 300 fields of C384 -> 0.25 deg: 3.58 ms with 64, 3.91 with 16,
+    // 4.70 with all; 20 fields of C384 -> 1 deg: 148 us with 8, 191 with 16 (2.80
+    // ms and 114 us with rows by length).
     const i64 fit = S.n_slices * nrhs / (152 * 24 * 4) / kF64F * kF64F;
     const i64 tile = std::min<i64>(64, std::max<i64>(8, fit));
     auto grid = [&](int F) {

@@ -551,40 +551,42 @@ __global__ void __launch_bounds__(256, F <= 4 ? 4 : 3) k_split_fused(SellArgs a,
 // FP64 apply in one launch. Warps [0, L.n * ceil(nrhs / F)): a long row and F
 // fields; the others: lane per row (rows of at most 32 entries, in the order
 // of Sell::ord from three fields up) and a tile of fields, F side by side,
-// kFusedK entries at a time (their loads, then their gathers, then the FMAs
-// in entry order). The entries are read again for the next F fields (from
-// L1), so rows of every length run in one launch without a register array
-// for the longest. The bound is the FP64 pipe (half a lane an SM
+// K entries at a time (their loads, then their gathers, then the FMAs in
+// entry order; entries past the row's end and fields past the last load the
+// last one again, since a load under a condition of its own waits: 10 fields
+// of 0.25 deg -> C384 159 -> 143 us). The entries are read again for the next
+// F fields (from L1), so rows of every length run in one launch without a
+// register array for the longest. The bound is the FP64 pipe (half a lane an SM
 // sub-partition and cycle). 64 fields of C192 -> 0.5 deg: 169 us, against
 // 297 us for one launch per length class with the entries in registers, the
 // last launches on a few blocks (three blocks an SM and four entries ahead:
 // 210 us; eight fields side by side: 223).
-template <int F>
-__global__ void __launch_bounds__(256, 4) k_f64_fused(SellArgs a, LongRows L, const int *__restrict__ ord,
-                                                                 i64 n_slices, const double *__restrict__ x, i64 ldx,
-                                                                 double *__restrict__ y, i64 ldy, i64 nrhs, i64 tile) {
+template <int F, int K, bool BY_LENGTH>
+__global__ void __launch_bounds__(256, 4)
+    k_f64_fused(SellArgs a, LongRows L, const int *__restrict__ ord, i64 n_slices, const double *__restrict__ x, i64 ldx,
+                double *__restrict__ y, i64 ldy, i64 nrhs, i64 tile) {
+    constexpr bool kAll = F <= 2;  // nrhs == F
     const int lane = threadIdx.x & 31;
     i64 w = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     // the long rows' warps come first in the grid, as in k_split_fused
-    const i64 n_long = L.n * ((nrhs + F - 1) / F);
+    const i64 n_long = kAll ? L.n : L.n * ((nrhs + F - 1) / F);
     if (w < n_long) {
         const i64 fc = nrhs <= F ? 0 : w / L.n;
         f64_long_row<F>(L, w - fc * L.n, fc, x, ldx, y, ldy, nrhs);
         return;
     }
     w -= n_long;
-    const i64 t = nrhs <= tile ? 0 : w / n_slices, pos = (w - t * n_slices) * 32 + lane;
-    const i64 fa = t * tile, fb = min(fa + tile, nrhs);
-    if (fa >= nrhs) return;
-    const int o = F > 2 ? ord[pos] : kOrdPlain;
+    const i64 t = kAll || nrhs <= tile ? 0 : w / n_slices, pos = (w - t * n_slices) * 32 + lane;
+    const i64 fa = t * tile, fb = kAll ? F : min(fa + tile, nrhs);
+    if (kAll ? w >= n_slices : fa >= nrhs) return;
+    const int o = BY_LENGTH ? ord[pos] : kOrdPlain;
     const i64 row = o & kOrdPlain ? pos : o;
     if (row >= a.n_rows) return;
     const int n = a.rlen[row];
     if (n > 32) return;
-    constexpr int K = F <= 2 ? kFusedK : kF64K;
     const int e0 = a.base[row >> 5] + static_cast<int>(row & 31);
-    for (i64 f = fa; f < fb; f += F) {
-        const int nf = static_cast<int>(min(static_cast<i64>(F), fb - f));
+    for (i64 f = kAll ? 0 : fa; f < fb; f += F) {
+        const int nf = kAll ? F : static_cast<int>(min(static_cast<i64>(F), fb - f));
         const double *xf = x + f * ldx;
         double s[F];
 #pragma unroll
@@ -593,23 +595,20 @@ __global__ void __launch_bounds__(256, 4) k_f64_fused(SellArgs a, LongRows L, co
             int cl[K];
             double wv[K], xv[K][F];
 #pragma unroll
+            for (int j = 0; j < K; ++j) {
+                const int e = e0 + 32 * min(k0 + j, n - 1);
+                cl[j] = a.col[e];
+                wv[j] = a.w64[e];
+            }
+#pragma unroll
+            for (int j = 0; j < K; ++j)
+#pragma unroll
+                for (int u = 0; u < F; ++u) xv[j][u] = __ldg(xf + min(u, nf - 1) * ldx + cl[j]);
+#pragma unroll
             for (int j = 0; j < K; ++j)
                 if (k0 + j < n) {
-                    const int e = e0 + 32 * (k0 + j);
-                    cl[j] = a.col[e];
-                    wv[j] = a.w64[e];
-                }
 #pragma unroll
-            for (int j = 0; j < K; ++j)
-#pragma unroll
-                for (int u = 0; u < F; ++u)
-                    if (k0 + j < n && u < nf) xv[j][u] = __ldg(xf + u * ldx + cl[j]);
-#pragma unroll
-            for (int j = 0; j < K; ++j)
-                if (k0 + j < n) {
-#pragma unroll
-                    for (int u = 0; u < F; ++u)
-                        if (u < nf) s[u] = fma(wv[j], xv[j][u], s[u]);
+                    for (int u = 0; u < F; ++u) s[u] = fma(wv[j], xv[j][u], s[u]);
                 }
         }
 #pragma unroll
@@ -914,17 +913,21 @@ void launch_f64_fused(const Matrix &m, const Sell &S, const double *x, i64 ldx, 
     // in row order, 300 fields of C384 -> 0.25 deg: 3.58 ms with 64, 3.91 with 16,
     // 4.70 with all; 20 fields of C384 -> 1 deg: 148 us with 8, 191 with 16 (2.80
     // ms and 114 us with rows by length).
+    // Four where eight would not fill the chip once: 10 fields of C384 -> 41 k
+    // Voronoi cells 122 -> 103 us, 20 of C48 -> 2 deg 13.5 -> 11.1.
     const i64 fit = S.n_slices * nrhs / (152 * 24 * 4) / kF64F * kF64F;
-    const i64 tile = std::min<i64>(64, std::max<i64>(8, fit));
-    auto grid = [&](int F) {
-        return nblk((L.n * ((nrhs + F - 1) / F) + S.n_slices * ((nrhs + tile - 1) / tile)) * 32, 256);
+    const i64 least = S.n_slices * nrhs < 152 * 32 * 8 ? kF64F : 2 * kF64F;
+    const i64 tile = std::min<i64>(64, std::max<i64>(least, fit));
+    auto launch = [&](auto kernel, int F) {
+        const i64 warps = L.n * ((nrhs + F - 1) / F) + S.n_slices * ((nrhs + tile - 1) / tile);
+        kernel<<<nblk(warps * 32, 256), 256, 0, s>>>(a, L, S.ord.p, S.n_slices, x, ldx, y, ldy, nrhs, tile);
     };
     if (nrhs == 1)
-        k_f64_fused<1><<<grid(1), 256, 0, s>>>(a, L, S.ord.p, S.n_slices, x, ldx, y, ldy, nrhs, tile);
+        launch(k_f64_fused<1, kFusedK, false>, 1);
     else if (nrhs == 2)
-        k_f64_fused<2><<<grid(2), 256, 0, s>>>(a, L, S.ord.p, S.n_slices, x, ldx, y, ldy, nrhs, tile);
+        launch(k_f64_fused<2, kFusedK, false>, 2);
     else
-        k_f64_fused<kF64F><<<grid(kF64F), 256, 0, s>>>(a, L, S.ord.p, S.n_slices, x, ldx, y, ldy, nrhs, tile);
+        launch(k_f64_fused<kF64F, kF64K, true>, kF64F);
 }
 
 // ─── NaN-aware and masked FP64 applies ────────────────────────────────────

@@ -996,10 +996,16 @@ struct NanRow {
     }
 };
 
-// Warps [0, L.n): one row of more than 32 entries each. The lanes multiply 32
-// entries of each field side by side; then lane f < 16 adds the products of
-// field f in entry order and lane 16 + f the valid weights. Warps from L.n
-// on: lane per row (Sell::ord). blockIdx.y: 16 fields. The long rows come
+// The first warps: rows_w rows of more than 32 entries each. The lanes multiply 32
+// entries of each (row, field) side by side; then lane q < 16 adds the products
+// of the q-th (row, field) in entry order and lane 16 + q the valid weights.
+// rows_w is one from nine fields up and more with fewer, so that the additions,
+// which cost the same with any number of lanes, have lanes to serve (one
+// field of C384 -> 41 k Voronoi cells, most rows long: 249 -> 42 us; 5
+// fields: 324 -> 187).
+// The warps after them: lane per row (Sell::ord), U fields side by side and K
+// entries ahead, loads past a row's end or the last field repeated, not left
+// out (k_f64_fused). blockIdx.y: 16 fields. The long rows come
 // first in the grid: their additions are chains of up to some thousand. The
 // outputs of short rows with some sources NaN need a second sum and a
 // division of their own; a warp with a coast has a few such lanes for every
@@ -1010,19 +1016,92 @@ struct NanItem {
     unsigned short lane, field;
 };
 constexpr int kNanPs = 33;  // products a field (32, and one against bank conflicts)
+constexpr int kNanRows = kNanG + 4;  // rows of products and of weights a warp holds
+// Long rows a warp takes side by side.
+__host__ __device__ inline int nan_rows_w(i64 nrhs) {
+    const int g = static_cast<int>(nrhs < kNanG ? nrhs : kNanG);
+    return kNanG / g < kNanRows / (g + 1) ? kNanG / g : kNanRows / (g + 1);
+}
 static_assert(sizeof(NanItem) * (31 + 32 * kNanU) <= sizeof(double) * kNanG * kNanPs, "items put aside fit a warp's ps");
-__global__ void __launch_bounds__(256) k_nan(SellArgs a, LongRows L, const double *__restrict__ totals,
-                                             const int *__restrict__ ord, i64 n_slices, const double *__restrict__ x,
-                                             i64 ldx, double *__restrict__ y, i64 ldy, i64 nrhs, double na_thres) {
-    __shared__ double ps[8][kNanG][kNanPs];
-    __shared__ double wsh[8][32];
+template <int U, int K>
+__global__ void __launch_bounds__(256, U == 1 ? 4 : 2)
+    k_nan(SellArgs a, LongRows L, const double *__restrict__ totals, const int *__restrict__ ord, i64 n_slices,
+          const double *__restrict__ x, i64 ldx, double *__restrict__ y, i64 ldy, i64 nrhs, int rows_w,
+          double na_thres) {
+    __shared__ double ps[8][kNanRows][kNanPs];
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     const i64 wg = static_cast<i64>(blockIdx.x) * 8 + wp;
     const double thres = __dsub_rn(__dsub_rn(1.0, na_thres), 1e-6);
-    if (wg < L.n) {
+    const i64 n_long = (L.n + rows_w - 1) / rows_w;
+    if (wg < n_long && (U == 1 || rows_w > 1)) {  // one chunk of fewer than kNanG fields
+        const int G = static_cast<int>(nrhs), R = static_cast<int>(min(static_cast<i64>(rows_w), L.n - wg * rows_w));
+        const int q = lane & 15, qr = q / G, qf = q - qr * G;
+        const bool has = qr < R;  // the lane serves a (row, field)
+        const i64 at = wg * rows_w + min(lane, R - 1);
+        const int b = L.ptr[at], n = lane < R ? L.ptr[at + 1] - b : 0;
+        const int from = has ? qr : 0;
+        const int qn = __shfl_sync(0xffffffffu, n, from);
+        const double *const src = ps[wp][has ? (lane < 16 ? q : R * G + qr) : 0];
+        int most = n;
+        for (int d = 16; d > 0; d >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, d));
+        double acc = 0.0;
+        for (int k0 = 0; k0 < most; k0 += 32) {
+            double xv[kNanG];
+            int r = 0, f = 0, e = 0, c = 0;
+            bool on = false;
+#pragma unroll
+            for (int j = 0; j < kNanG; ++j) {
+                xv[j] = 0.0;
+                if (r < R) {  // warp-uniform, as r and f are
+                    if (f == 0) {
+                        const int nr = __shfl_sync(0xffffffffu, n, r);
+                        e = __shfl_sync(0xffffffffu, b, r) + k0 + lane;
+                        on = k0 + lane < nr;
+                        c = on ? L.col[e] : 0;
+                        ps[wp][R * G + r][lane] = on ? L.w64[e] : 0.0;
+                    }
+                    if (on) xv[j] = __ldg(x + f * ldx + c);
+                    if (++f == G) {
+                        f = 0;
+                        ++r;
+                    }
+                }
+            }
+            const int left = max(0, qn - k0);
+            unsigned skip = left >= 32 ? 0u : ~0u << left;  // the entries the lane leaves out
+            r = f = 0;
+#pragma unroll
+            for (int j = 0; j < kNanG; ++j)
+                if (r < R) {
+                    const unsigned nan_mask = __ballot_sync(0xffffffffu, nan_bits(xv[j]));
+                    if (q == j) skip |= nan_mask;
+                    ps[wp][j][lane] = __dmul_rn(ps[wp][R * G + r][lane], xv[j]);
+                    if (++f == G) {
+                        f = 0;
+                        ++r;
+                    }
+                }
+            __syncwarp();
+            const int m = min(32, most - k0);
+#pragma unroll 8
+            for (int k = 0; k < m; ++k) {
+                const double t = __dadd_rn(acc, src[k]);
+                if (!((skip >> k) & 1u)) acc = t;
+            }
+            __syncwarp();
+        }
+        const double valid = __shfl_down_sync(0xffffffffu, acc, 16);
+        if (has && lane < 16) {
+            const i64 row = L.row[wg * rows_w + qr];
+            y[qf * ldy + row] = nan_result(totals[row], acc, valid, thres);
+        }
+        return;
+    }
+    if (U > 1 && wg < n_long) {  // rows_w 1
         const i64 row = L.row[wg];
         const int b = L.ptr[wg], n = L.ptr[wg + 1] - b;
         const double total = totals[row];
+        double *const wsh = ps[wp][kNanG];
         {
             const i64 f0 = static_cast<i64>(blockIdx.y) * kNanG;
             const int nf = static_cast<int>(min(static_cast<i64>(kNanG), nrhs - f0));
@@ -1036,7 +1115,7 @@ __global__ void __launch_bounds__(256) k_nan(SellArgs a, LongRows L, const doubl
 #pragma unroll
                 for (int f = 0; f < kNanG; ++f) xv[f] = on && f < nf ? __ldg(xf + f * ldx + c) : 0.0;
                 unsigned skip = 0;
-                wsh[wp][lane] = w;
+                wsh[lane] = w;
 #pragma unroll
                 for (int f = 0; f < kNanG; ++f) {
                     const unsigned nan_mask = __ballot_sync(0xffffffffu, nan_bits(xv[f]));
@@ -1045,7 +1124,7 @@ __global__ void __launch_bounds__(256) k_nan(SellArgs a, LongRows L, const doubl
                 }
                 __syncwarp();
                 const int m = min(32, n - k0);
-                const double *src = lane < kNanG ? ps[wp][lane] : wsh[wp];
+                const double *src = lane < kNanG ? ps[wp][lane] : wsh;
 #pragma unroll 8
                 for (int k = 0; k < m; ++k) {
                     const double t = __dadd_rn(acc, src[k]);
@@ -1058,7 +1137,7 @@ __global__ void __launch_bounds__(256) k_nan(SellArgs a, LongRows L, const doubl
         }
         return;
     }
-    const i64 sid = wg - L.n;
+    const i64 sid = wg - n_long;
     if (sid >= n_slices) return;
     const i64 row = ord[sid * 32 + lane] & ~kOrdPlain;
     const bool live = row < a.n_rows && a.rlen[row] <= 32;
@@ -1096,34 +1175,33 @@ __global__ void __launch_bounds__(256) k_nan(SellArgs a, LongRows L, const doubl
     {
         const i64 f0 = static_cast<i64>(blockIdx.y) * kNanG;
         const int nf = static_cast<int>(min(static_cast<i64>(kNanG), nrhs - f0));
-        for (int g = 0; g < nf; g += kNanU) {
+        for (int g = 0; g < nf; g += U) {
             const double *xf = x + (f0 + g) * ldx;
-            double ws[kNanU];
-            unsigned nm[kNanU];  // the row's entries whose source is NaN
+            double ws[U];
+            unsigned nm[U];  // the row's entries whose source is NaN
 #pragma unroll
-            for (int u = 0; u < kNanU; ++u) {
+            for (int u = 0; u < U; ++u) {
                 ws[u] = 0.0;
                 nm[u] = 0;
             }
-            for (int k0 = 0; k0 < n; k0 += kNanK) {
-                int c[kNanK];
-                double w[kNanK], xv[kNanK][kNanU];
+            for (int k0 = 0; k0 < n; k0 += K) {
+                int c[K];
+                double w[K], xv[K][U];
 #pragma unroll
-                for (int j = 0; j < kNanK; ++j)
+                for (int j = 0; j < K; ++j) {
+                    const int e = base + 32 * min(k0 + j, n - 1);
+                    c[j] = a.col[e];
+                    w[j] = a.w64[e];
+                }
+#pragma unroll
+                for (int j = 0; j < K; ++j)
+#pragma unroll
+                    for (int u = 0; u < U; ++u) xv[j][u] = __ldg(xf + min(u, nf - g - 1) * ldx + c[j]);
+#pragma unroll
+                for (int j = 0; j < K; ++j)
                     if (k0 + j < n) {
-                        c[j] = a.col[base + 32 * (k0 + j)];
-                        w[j] = a.w64[base + 32 * (k0 + j)];
-                    }
 #pragma unroll
-                for (int j = 0; j < kNanK; ++j)
-#pragma unroll
-                    for (int u = 0; u < kNanU; ++u)
-                        if (k0 + j < n && g + u < nf) xv[j][u] = __ldg(xf + u * ldx + c[j]);
-#pragma unroll
-                for (int j = 0; j < kNanK; ++j)
-                    if (k0 + j < n) {
-#pragma unroll
-                        for (int u = 0; u < kNanU; ++u)
+                        for (int u = 0; u < U; ++u)
                             if (g + u < nf) {
                                 const bool bad = nan_bits(xv[j][u]);
                                 const double t = __dadd_rn(ws[u], __dmul_rn(w[j], xv[j][u]));
@@ -1134,7 +1212,7 @@ __global__ void __launch_bounds__(256) k_nan(SellArgs a, LongRows L, const doubl
             }
             __syncwarp();
 #pragma unroll
-            for (int u = 0; u < kNanU; ++u) {
+            for (int u = 0; u < U; ++u) {
                 if (g + u >= nf) break;
                 const bool aside = live && nm[u] != 0 && nm[u] != full;
                 const unsigned who = __ballot_sync(0xffffffffu, aside);
@@ -1592,12 +1670,16 @@ void nan_batch_apply_f64(Matrix &m, const double *x, i64 ldx, double *y, i64 ldy
     if (nrhs <= 0 || m.n_dst == 0) return;
     if (!m.sell64.built) matrix_prepare(m, 0, s);
     const Sell &S = m.sell64;
-    const i64 warps = S.n_lrows + S.n_slices;
+    // One field alone: without others side by side, twice the blocks an SM (0.25
+    // -> 0.5 deg: 35 -> 26 us; eight entries ahead instead of four 28).
+    const auto kernel = nrhs == 1 ? k_nan<1, kNanK> : k_nan<kNanU, kNanK>;
+    const int rows_w = nan_rows_w(nrhs);
+    const i64 warps = (S.n_lrows + rows_w - 1) / rows_w + S.n_slices;
     for (i64 f = 0; f < nrhs; f += 65535 * kNanG) {
         const i64 nf = std::min<i64>(nrhs - f, 65535 * kNanG);
         const dim3 grid(nblk(warps, 8), nblk(nf, kNanG));
-        k_nan<<<grid, 256, 0, s>>>(sell_args(m, S), long_rows(S), S.total.p, S.ord.p, S.n_slices, x + f * ldx, ldx,
-                                   y + f * ldy, ldy, nf, na_thres);
+        kernel<<<grid, 256, 0, s>>>(sell_args(m, S), long_rows(S), S.total.p, S.ord.p, S.n_slices, x + f * ldx, ldx,
+                                    y + f * ldy, ldy, nf, rows_w, na_thres);
     }
     AXGB_CUDA(cudaGetLastError());
 }

@@ -163,6 +163,27 @@ def test_nan_apply_row_shapes(gpu, oracle, nf, weights, na_thres):
     assert np.array_equal(y[~np.isnan(y)], ref[~np.isnan(ref)])
 
 
+@pytest.mark.parametrize("nf", [1, 2, 3, 4, 5, 6, 7, 8, 9, 15])
+@pytest.mark.parametrize("lens", [LONG, [40, 33] * 33, [33, 1000, 5, 64, 0, 128, 32] * 3], ids=["long", "even", "mixed"])
+def test_nan_long_rows_side_by_side(gpu, oracle, nf, lens):
+    """Few fields: a warp takes several long rows, of different lengths, the
+    last warp fewer; bit for bit."""
+    import torch
+    from oracle import Weights
+    M = _rows_matrix(gpu, np.array(lens, np.int64), 4000, 51)
+    X = np.random.default_rng(52).standard_normal((nf, M.n_src))
+    X[:, ::5] = np.nan
+    X[nf - 1, 1000:3000] = np.nan
+    c = M.to_csr()
+    row = np.repeat(np.arange(M.n_dst), np.diff(c["row_ptr"])).astype(np.int64)
+    w = Weights(M.n_src, M.n_dst, row, c["col"].astype(np.int64), c["val"], c["frac_a"], c["frac_b"], c["area_a"],
+                c["area_b"])
+    ref = oracle.nan_batch_apply(w, X, 0.5)
+    y = gpu.nan_apply_f64(M, torch.tensor(X, device="cuda"), 0.5).cpu().numpy()
+    assert np.array_equal(np.isnan(y), np.isnan(ref))
+    assert np.array_equal(y[~np.isnan(y)], ref[~np.isnan(ref)])
+
+
 @pytest.mark.parametrize("nf", [1, 2, 3, 4, 5, 8, 9, 45])
 def test_unaligned_fields(gpu, oracle, nf):
     """Fields whose rows do not start on 16 bytes (an odd number of cells, and

@@ -941,7 +941,7 @@ void launch_f64_fused(const Matrix &m, const Sell &S, const double *x, i64 ldx, 
 // FP64 work is what is left out: NaN is tested on the bits, the valid weight
 // is summed only in rows that have a NaN (else it is the total, the same
 // additions), and the divisions are shortened (NanRow). 16 fields of 0.25 deg -> C384 with a third of the cells missing:
-// 651 us, against 2485 us with three FP64 operations an entry, two
+// 617 us, against 2485 us with three FP64 operations an entry, two
 // divisions an output, and a lane walking each long row.
 constexpr int kNanG = 16;  // fields a warp
 constexpr int kNanU = 4;   // fields of a short row carried side by side

@@ -26,6 +26,7 @@
 
 #include "fp32x2.cuh"
 #include "internal.hpp"
+#include "row_items.hpp"
 
 namespace axgb {
 
@@ -567,7 +568,7 @@ __global__ void __launch_bounds__(256, 4)
                 double *__restrict__ y, i64 ldy, i64 nrhs, i64 tile) {
     constexpr bool kAll = F <= 2;  // nrhs == F
     const int lane = threadIdx.x & 31;
-    i64 w = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const i64 w = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     // the long rows' warps come first in the grid, as in k_split_fused
     const i64 n_long = kAll ? L.n : L.n * ((nrhs + F - 1) / F);
     if (w < n_long) {
@@ -575,17 +576,18 @@ __global__ void __launch_bounds__(256, 4)
         f64_long_row<F>(L, w - fc * L.n, fc, x, ldx, y, ldy, nrhs);
         return;
     }
-    w -= n_long;
-    const i64 t = kAll || nrhs <= tile ? 0 : w / n_slices, pos = (w - t * n_slices) * 32 + lane;
-    const i64 fa = t * tile, fb = kAll ? F : min(fa + tile, nrhs);
-    if (kAll ? w >= n_slices : fa >= nrhs) return;
+    // the grid's surplus warps leave before ord is read
+    const RowItem it = row_item(w - n_long, n_slices, kAll ? F : nrhs, kAll ? F : tile);
+    if (!it.on) return;
+    const i64 pos = it.slice * 32 + lane;
+    const i64 fa = kAll ? 0 : it.tile * tile, fb = kAll ? F : min(fa + tile, nrhs);
     const int o = BY_LENGTH ? ord[pos] : kOrdPlain;
     const i64 row = o & kOrdPlain ? pos : o;
     if (row >= a.n_rows) return;
     const int n = a.rlen[row];
     if (n > 32) return;
     const int e0 = a.base[row >> 5] + static_cast<int>(row & 31);
-    for (i64 f = kAll ? 0 : fa; f < fb; f += F) {
+    for (i64 f = fa; f < fb; f += F) {
         const int nf = kAll ? F : static_cast<int>(min(static_cast<i64>(F), fb - f));
         const double *xf = x + f * ldx;
         double s[F];
@@ -919,7 +921,7 @@ void launch_f64_fused(const Matrix &m, const Sell &S, const double *x, i64 ldx, 
     const i64 least = S.n_slices * nrhs < 152 * 32 * 8 ? kF64F : 2 * kF64F;
     const i64 tile = std::min<i64>(64, std::max<i64>(least, fit));
     auto launch = [&](auto kernel, int F) {
-        const i64 warps = L.n * ((nrhs + F - 1) / F) + S.n_slices * ((nrhs + tile - 1) / tile);
+        const i64 warps = row_item_warps(L.n, F, S.n_slices, nrhs, tile);
         kernel<<<nblk(warps * 32, 256), 256, 0, s>>>(a, L, S.ord.p, S.n_slices, x, ldx, y, ldy, nrhs, tile);
     };
     if (nrhs == 1)

@@ -197,7 +197,7 @@ void mesh_upload_impl(Mesh &m) {
             t[2 * (g.ni + 1) + j] = std::sin(r);
             t[2 * (g.ni + 1) + (g.nj + 1) + j] = std::cos(r);
         }
-        m.d_trig.upload(t.data(), t.size());
+        m.d_trig.upload_vec(t);
     }
     AXGB_CUDA(cudaDeviceSynchronize());
 }
@@ -658,7 +658,7 @@ int axgb_mesh_create(const double *node_coords, int64_t n_nodes, const int64_t *
         if (mask) {
             m->has_mask = true;
             std::vector<int> mk(mask, mask + n_cells);
-            m->d_mask.upload(mk.data(), mk.size());
+            m->d_mask.upload_vec(mk);
         }
         mesh_upload_impl(*m);
         *mesh_handle = Registry::get().add(Registry::get().meshes, m);

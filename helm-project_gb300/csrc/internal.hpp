@@ -73,15 +73,20 @@ struct DBuf {
         p = nullptr;
         n = 0;
     }
+    // h must stay as it is until the stream has been waited for: a copy from
+    // pageable memory may still read it after the call.
     void upload(const T *h, size_t count, cudaStream_t s = 0) {
         if (count > n) alloc(count);
         if (count) AXGB_CUDA(cudaMemcpyAsync(p, h, count * sizeof(T), cudaMemcpyHostToDevice, s));
     }
-    // Allocates at least one element and copies the vector's elements (none for an empty vector).
+    // Allocates at least one element and copies the vector's elements (none for
+    // an empty vector). Waits for the copy, so v may be a temporary.
     template <class V>
     void upload_vec(const V &v, cudaStream_t s = 0) {
         if (v.size() + 1 > n || !p) alloc(v.size() > 0 ? v.size() : 1);
-        if (!v.empty()) AXGB_CUDA(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s));
+        if (v.empty()) return;
+        AXGB_CUDA(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s));
+        AXGB_CUDA(cudaStreamSynchronize(s));
     }
     void download(T *h, size_t count, cudaStream_t s = 0) const {
         if (count) AXGB_CUDA(cudaMemcpyAsync(h, p, count * sizeof(T), cudaMemcpyDeviceToHost, s));

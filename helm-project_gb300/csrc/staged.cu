@@ -815,7 +815,6 @@ void plan_source_order(Matrix &m, const std::vector<int> &rp, std::vector<int> &
     m.src_inv.upload_vec(inv, s);
     m.src_span.upload_vec(span, s);
     m.split_col.upload_vec(col, s);
-    AXGB_CUDA(cudaStreamSynchronize(s));  // inv and span are gone after this call
     m.src_renum = true;
 }
 
@@ -1763,7 +1762,6 @@ void build_segmented(Matrix &m, cudaStream_t s) {
         G.l_ptr.upload_vec(ptr, s);
         G.l_col.upload_vec(c, s);
         G.l_hl.upload_vec(hl, s);
-        AXGB_CUDA(cudaStreamSynchronize(s));  // the vectors above are gone after this block
     }
     G.n_fb = static_cast<i64>(fb_rows.size());
     G.n_long = static_cast<i64>(long_rows.size());

@@ -528,7 +528,7 @@ int default_item_fields(const Matrix &m, i64 nrhs) {
 // deg -> C192 (ten launches) 31.8 against 44.3, 64 of it 117.8 against 113.7.
 SplitParams default_split_params(const Matrix &m, i64 nrhs) {
     SplitParams p;
-    const i64 launches = m.blocked.built ? split_launches(m) : 3;
+    const i64 launches = m.split_ready() ? split_launches(m) : 3;
     if (nrhs <= 2 || m.nnz * nrhs <= i64(4000000) * launches) {
         p.variant = 4;
         p.fields_per_pass = 0;
@@ -555,7 +555,7 @@ SplitParams pick_params(Matrix &m, i64 nrhs, cudaStream_t s) {
         auto it = m.tuned.find(nrhs);
         if (it != m.tuned.end()) return it->second;
     }
-    if (!m.blocked.built) matrix_prepare(m, 2, s);
+    if (!m.split_ready()) matrix_prepare(m, 2, s);
     return default_split_params(m, nrhs);
 }
 

@@ -1467,18 +1467,15 @@ __global__ void __launch_bounds__(256, ROWS ? 3 : 2) k_batch(const Batch::Desc *
 
 void matrix_prepare(Matrix &m, int format, cudaStream_t s) {
     std::lock_guard<std::mutex> lk(m.mu);
-    if (format == 3) {  // segmented layout (it fixes the split order through the blocked build first)
-        build_segmented(m, s);
+    if (format == 0) {
+        build_sell(m, 0, s);
         return;
     }
-    if (format >= 1) build_blocked(m, s);  // fixes the split entry order (split_perm) first
-    if (format == 2) {
-        build_sell(m, 1, s);  // slices of blocks that do not fit the blocked kernels use the direct kernel
-        m.stats[6] = blocked_launches(m);
-        return;
-    }
-    build_sell(m, format == 0 ? 0 : 1, s);
+    build_blocked(m, s);  // fixes the split entry order (split_perm) first
+    if (format == 3) build_segmented(m, s);
+    build_sell(m, 1, s);  // the direct kernels' and, for long rows and blocks that do not fit, the staged ones'
     if (format == 1) m.stats[5] = 1;  // the direct kernel is one launch
+    if (format >= 2) m.stats[6] = blocked_launches(m);
 }
 
 namespace {
@@ -1578,7 +1575,7 @@ void apply_split(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs
         apply_segmented(m, x, ldx, y, ldy, nrhs, s, ylo, ldylo, p.stages);
         return;
     }
-    if (!m.blocked.built) matrix_prepare(m, 2, s);
+    if (!m.split_ready()) matrix_prepare(m, 2, s);
     if (!m.src_renum) {
         apply_split_layouts(m, x, ldx, y, ldy, nrhs, p, s, ylo, ldylo);
         return;
@@ -1589,11 +1586,10 @@ void apply_split(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs
     apply_split_layouts(m, xr.p, ldr, y, ldy, nrhs, p, s, ylo, ldylo);
 }
 
+// The layouts are there (apply_split).
 void apply_split_layouts(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, const SplitParams &p,
                          cudaStream_t s, float *ylo, i64 ldylo) {
-    if (nrhs <= 0) return;
     if (p.variant >= 1 && p.variant <= 3 && blocked_eligible(m, x, ldx, p.variant == 2)) {
-        if (!m.blocked.built) matrix_prepare(m, 2, s);
         apply_blocked(m, x, ldx, y, ldy, nrhs, p.variant, p.unroll, p.stages, p.fields_per_pass, s, ylo, ldylo);
         const Blocked &B = m.blocked;
         if (B.n_fallback > 0) {
@@ -1604,7 +1600,6 @@ void apply_split_layouts(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, 
         AXGB_CUDA(cudaGetLastError());
         return;
     }
-    if (!m.sell32.built) matrix_prepare(m, 1, s);
     const Sell &S = m.sell32;
     // direct kernel: with the caller's knobs (variant 0), else its own choice
     if (p.variant == 0)

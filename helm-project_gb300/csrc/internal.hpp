@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <map>
 #include <memory>
@@ -182,7 +183,7 @@ struct Mesh {
 // Sliced-ELL (32-row slices) apply layout. Entry k of row r of slice s is at
 // base[s] + k*32 + (r % 32); padding entries have column 0 and weight 0.
 struct Sell {
-    bool built = false;
+    std::atomic<bool> built{false};  // set last, by matrix_prepare under Matrix::mu; read without it
     i64 n_slices = 0, n_entries = 0;
     DBuf<int> base, len, col;
     DBuf<float2> hl;        // split weights (hi, lo) (format 1)
@@ -209,7 +210,7 @@ struct Blocked {
         int us;       // staging floats per field (allocation for the class)
         i64 begin, n; // range in block_ids
     };
-    bool built = false;
+    std::atomic<bool> built{false};  // set last, by matrix_prepare under Matrix::mu; read without it
     i64 n_blocks = 0;
     i64 n_src = 0;  // source cells of the matrix (bounds the last staged chunk)
     DBuf<int> brow, wbase, wlen, cstart, ccol, rstart, block_ids, fallback_slices;
@@ -248,7 +249,7 @@ struct Segmented {
         int usmax;     // staged-cell bucket of the launch
         i64 begin, n;  // range in gids
     };
-    bool built = false;
+    std::atomic<bool> built{false};  // set last, by matrix_prepare under Matrix::mu; read without it
     i64 n_groups = 0;
     DBuf<int4> grp;       // per group: (first cell in cellmap, cells, first entry pair, entry pairs)
     int max_ent = 0;      // entry pairs of the largest group
@@ -321,6 +322,10 @@ struct Matrix {
     std::vector<float> seg_xyz;    // the same for each 8-row segment (segmented layout)
     std::map<i64, SplitParams> tuned;  // nrhs -> best kernel choice
     std::mutex mu;
+    // Both layouts that a split apply reads are there. (The blocked one is
+    // complete before the sliced one, whose long rows the staged applies need:
+    // another thread's first apply may be between the two.)
+    bool split_ready() const { return blocked.built && sell32.built; }
 };
 
 constexpr int kGatherTile = 4096;  // new cells a block of the source gather takes

@@ -1,0 +1,75 @@
+"""First applies of a matrix, which build the layouts: in any order of the
+kernel variants, and from several host threads at once. Rows of more than 32
+entries, which the staged kernels leave to the sliced layout, are among them;
+every split kernel gives the same bits."""
+import threading
+
+import numpy as np
+import pytest
+
+from test_gpu_apply_shapes import LONG, SHORT, _check_split, _reference, _rows_matrix
+
+pytestmark = pytest.mark.gpu
+
+
+def _lens(seed):
+    return np.random.default_rng(seed).choice(LONG + 4 * SHORT, 700).astype(np.int64)
+
+
+@pytest.mark.parametrize("first", ["segmented", "prepare", "staged", "direct", "hilo"])
+def test_any_variant_first(gpu, oracle, first):
+    import torch
+    nf = 6
+    X = np.random.default_rng(2).standard_normal((nf, 4000)).astype(np.float32)
+    xs = torch.tensor(X, device="cuda")
+    M = _rows_matrix(gpu, _lens(1), 4000, 3)
+    if first == "prepare":
+        M.prepare(3)
+    elif first == "hilo":
+        gpu.apply_f32split_hilo(M, xs)
+    else:
+        v, u = {"segmented": (5, 32), "staged": (3, 4), "direct": (0, 4)}[first]
+        gpu.apply_f32split(M, xs, fields_per_pass=0, unroll=u, variant=v)
+    ys = {}
+    for v, u in ((3, 4), (1, 4), (2, 4), (0, 4), (4, 1), (5, 32)):
+        y = torch.full((nf, M.n_dst), float("nan"), device="cuda")
+        ys[v] = gpu.apply_f32split(M, xs, y, fields_per_pass=0, unroll=u, variant=v).cpu().numpy()
+    _check_split(ys[3], *_reference(M, oracle, X))
+    for v, y in ys.items():
+        assert np.array_equal(y, ys[3]), v
+
+
+@pytest.mark.parametrize("nf", [1, 6, 20])
+def test_first_applies_from_several_threads(gpu, nf):
+    """Eight threads, each on its own stream, start on a matrix without layouts:
+    default, staged, segmented and FP64 applies side by side."""
+    import torch
+    X = torch.randn((nf, 4000), device="cuda", generator=torch.Generator(device="cuda").manual_seed(4))
+    X64 = X.double()
+    calls = [lambda M, y: gpu.apply_f32split(M, X, y),
+             lambda M, y: gpu.apply_f32split(M, X, y, fields_per_pass=0, unroll=4, variant=3),
+             lambda M, y: gpu.apply_f32split(M, X, y, fields_per_pass=0, unroll=32, variant=5),
+             lambda M, y: gpu.apply_f64(M, X64, y)]
+    for seed in range(6):
+        M = _rows_matrix(gpu, _lens(10 + seed), 4000, 20 + seed)
+        out = [torch.full((nf, M.n_dst), float("nan"), device="cuda", dtype=torch.float64 if q % 4 == 3 else torch.float32)
+               for q in range(8)]
+        torch.cuda.synchronize()
+        start = threading.Barrier(8)
+
+        def work(q):
+            with torch.cuda.stream(torch.cuda.Stream()):
+                start.wait(30)
+                calls[q % 4](M, out[q])
+                torch.cuda.current_stream().synchronize()
+
+        th = [threading.Thread(target=work, args=(q,)) for q in range(8)]
+        for t in th:
+            t.start()
+        for t in th:
+            t.join()
+        want = gpu.apply_f32split(M, X, fields_per_pass=0, unroll=1, variant=4)
+        want64 = gpu.apply_f64(M, X64)
+        for q in range(8):
+            assert torch.equal(out[q], want64 if q % 4 == 3 else want), (seed, q)
+        assert M.device_status() == 0

@@ -526,9 +526,10 @@ int default_item_fields(const Matrix &m, i64 nrhs) {
 // for one or two fields always. Direct against staged: 16 fields of C96 -> 1
 // deg 10.4 against 17.5 us, 4 of C384 -> 0.25 deg 38.8 against 32.2; 16 of 0.5
 // deg -> C192 (ten launches) 31.8 against 44.3, 64 of it 117.8 against 113.7.
+// The matrix has its split layouts.
 SplitParams default_split_params(const Matrix &m, i64 nrhs) {
     SplitParams p;
-    const i64 launches = m.split_ready() ? split_launches(m) : 3;
+    const i64 launches = split_launches(m);
     if (nrhs <= 2 || m.nnz * nrhs <= i64(4000000) * launches) {
         p.variant = 4;
         p.fields_per_pass = 0;
@@ -1184,7 +1185,7 @@ int axgb_get_kernel_choice(int h, int64_t nrhs, int32_t *choice, int32_t *cached
     AXGB_TRY({
         auto m = Registry::get().find(Registry::get().mats, h, "matrix");
         AXGB_REQUIRE(choice && nrhs > 0, "get_kernel_choice: NULL choice or nrhs <= 0");
-        SplitParams p = default_split_params(*m, nrhs);
+        SplitParams p;
         int32_t c = 0;
         {
             std::lock_guard<std::mutex> lk(m->mu);
@@ -1194,6 +1195,7 @@ int axgb_get_kernel_choice(int h, int64_t nrhs, int32_t *choice, int32_t *cached
                 c = 1;
             }
         }
+        if (!c) p = pick_params(*m, nrhs, 0);
         choice[0] = p.variant;
         choice[1] = p.fields_per_pass;
         choice[2] = p.unroll;

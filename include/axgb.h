@@ -290,7 +290,9 @@ int axgb_set_autotune(int enable);
  * axgb_autotune_f32split returns
  * it. Seeding lets a caller reuse a choice tuned in an earlier process
  * without timing again. When nothing is cached for (matrix, nrhs), get
- * sets *cached = 0 and returns the default choice. */
+ * sets *cached = 0 and returns the default choice; it depends on the split
+ * layouts, which are then built if the matrix has none yet (as its first
+ * split apply would). */
 int axgb_set_kernel_choice(int matrix_handle, int64_t nrhs, const int32_t *choice);
 int axgb_get_kernel_choice(int matrix_handle, int64_t nrhs, int32_t *choice, int32_t *cached);
 

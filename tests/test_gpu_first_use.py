@@ -73,3 +73,19 @@ def test_first_applies_from_several_threads(gpu, nf):
         for q in range(8):
             assert torch.equal(out[q], want64 if q % 4 == 3 else want), (seed, q)
         assert M.device_status() == 0
+
+
+@pytest.mark.parametrize("nf,direct", [(3, True), (40, True), (400, False)])
+def test_default_choice_before_and_after_the_layouts(gpu, nf, direct):
+    """The default kernel choice read from a matrix without layouts is the one
+    its applies use: rows of every length class, 8 staged launches, 40 fields
+    of half a million entries (more than 12 and less than 32 million)."""
+    lens = np.repeat(np.arange(1, 33), 960)
+    rp = np.concatenate([[0], np.cumsum(lens)])
+    start = np.arange(len(lens)) // 4  # neighbouring rows share their sources: every block is staged
+    col = np.arange(rp[-1]) - np.repeat(rp[:-1] - start, lens)
+    M = gpu.Matrix.from_csr(int(col.max()) + 1, len(lens), rp, col, np.full(rp[-1], 0.5))
+    ch = gpu.get_kernel_choice(M, nf)
+    M.prepare(2)
+    assert gpu.get_kernel_choice(M, nf) == ch
+    assert ch["cached"] is False and (ch["variant"] == 4) is direct

@@ -8,6 +8,8 @@
 // regular/rectilinear detection (detail/regular_grid_detector.hpp:64-299)
 // runs on sorted node coordinates with a parallel sort. Everything after
 // that runs on the GPU.
+#include <cuda.h>
+
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -221,13 +223,16 @@ struct Downloader {
         bool widen;  // int32 on the device, int64 on the host
     };
     std::mutex mu;
-    int device = -1;
     char *slots = nullptr;
     cudaStream_t st[kThreads] = {};
 
+    // The current context's; those of ended contexts are not touched again.
     static Downloader &get() {
-        static Downloader d;
-        return d;
+        static std::mutex all_mu;
+        static std::map<unsigned long long, Downloader> all;
+        const unsigned long long id = context_id();
+        std::lock_guard<std::mutex> lk(all_mu);
+        return all[id];
     }
     void release() {
         for (auto &q : st) {
@@ -236,7 +241,6 @@ struct Downloader {
         }
         if (slots) cudaFreeHost(slots);
         slots = nullptr;
-        device = -1;
     }
     // size: bytes of an element on the device
     static void add(std::vector<Piece> &v, const void *dev, void *host, i64 n, size_t size, bool widen) {
@@ -274,13 +278,16 @@ struct Downloader {
         std::lock_guard<std::mutex> lk(mu);
         int dev = 0;
         AXGB_CUDA(cudaGetDevice(&dev));
-        if (dev != device) {
-            release();
-            void *h = nullptr;
-            AXGB_CUDA(cudaHostAlloc(&h, 2 * kThreads * kPiece, cudaHostAllocDefault));
-            slots = static_cast<char *>(h);
-            for (auto &q : st) AXGB_CUDA(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
-            device = dev;
+        if (!slots) {
+            try {
+                for (auto &q : st) AXGB_CUDA(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
+                void *h = nullptr;
+                AXGB_CUDA(cudaHostAlloc(&h, 2 * kThreads * kPiece, cudaHostAllocDefault));
+                slots = static_cast<char *>(h);
+            } catch (...) {
+                release();
+                throw;
+            }
         }
         std::atomic<int> failed{0};
         auto work = [&](int w) {
@@ -317,24 +324,29 @@ struct Downloader {
 
 struct ScratchPools {
     std::mutex mu;
-    std::map<int, cudaMemPool_t> of;  // by device
+    std::map<unsigned long long, cudaMemPool_t> of;  // by context; those of ended contexts are not touched again
     static ScratchPools &get() {
         static ScratchPools p;
         return p;
     }
 };
 
-// What the pools keep goes back to the device (blocks in use stay), the
-// downloads' pinned slots to the host.
+// What the current context's pool keeps goes back to the device (blocks in
+// use stay), the downloads' pinned slots to the host.
 void scratch_give_back() {
-    {
+    unsigned long long id = 0;
+    try {
+        id = context_id();
         auto &D = Downloader::get();
         std::lock_guard<std::mutex> lk(D.mu);
         D.release();
+    } catch (const Error &) {
+        return;  // no context: nothing is held
     }
     auto &P = ScratchPools::get();
     std::lock_guard<std::mutex> lk(P.mu);
-    for (auto &kv : P.of) cudaMemPoolTrimTo(kv.second, 0);
+    auto it = P.of.find(id);
+    if (it != P.of.end()) cudaMemPoolTrimTo(it->second, 0);
 }
 
 // Reusable device staging for the host-pointer entry points.
@@ -562,13 +574,32 @@ SplitParams pick_params(Matrix &m, i64 nrhs, cudaStream_t s) {
 
 }  // namespace
 
-cudaMemPool_t scratch_pool() {
-    int dev = 0;
+unsigned long long context_id() {
+    using GetId = CUresult (*)(CUcontext, unsigned long long *);
+    static const GetId get = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        AXGB_CUDA(cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &r));
+        if (!f) throw Error(AXGB_ERR_CUDA, "cuCtxGetId: not in this driver");
+        return reinterpret_cast<GetId>(f);
+    }();
+    unsigned long long id = 0;
+    if (get(nullptr, &id) == CUDA_SUCCESS) return id;
+    int dev = 0;  // a thread that has not used its device, or one after a reset
     AXGB_CUDA(cudaGetDevice(&dev));
+    AXGB_CUDA(cudaSetDevice(dev));
+    if (get(nullptr, &id) != CUDA_SUCCESS) throw Error(AXGB_ERR_CUDA, "no CUDA context");
+    return id;
+}
+
+cudaMemPool_t scratch_pool() {
+    const unsigned long long id = context_id();
     auto &P = ScratchPools::get();
     std::lock_guard<std::mutex> lk(P.mu);
-    auto it = P.of.find(dev);
+    auto it = P.of.find(id);
     if (it != P.of.end()) return it->second;
+    int dev = 0;
+    AXGB_CUDA(cudaGetDevice(&dev));
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
     props.handleTypes = cudaMemHandleTypeNone;
@@ -578,7 +609,7 @@ cudaMemPool_t scratch_pool() {
     AXGB_CUDA(cudaMemPoolCreate(&pool, &props));
     std::uint64_t keep = kScratchKept;
     AXGB_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-    P.of[dev] = pool;
+    P.of[id] = pool;
     return pool;
 }
 

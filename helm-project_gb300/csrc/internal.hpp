@@ -97,12 +97,20 @@ struct DBuf {
     }
 };
 
+// What the library keeps per process and device (scratch pool, kernels' shared-
+// memory limits, the export's streams and slots) belongs to a CUDA context and
+// goes with it: cudaDeviceReset ends the context, and the next call makes
+// another, at the same address. This is the id of the calling thread's current
+// context, which is never given out twice (about 10 ns).
+unsigned long long context_id();
+
 // Stream-ordered scratch: taken from and returned to the library's own
 // memory pool on one stream, which must be the one its users run on. The pool
-// (one per device, api.cpp) keeps at most kScratchKept bytes between calls
-// and gives them back when the last mesh, matrix and batch is destroyed. An
-// allocation costs about a microsecond where cudaMalloc and cudaFree take tens
-// and wait for the device.
+// (one per context, api.cpp) keeps at most kScratchKept bytes between calls
+// and gives them back when the last mesh, matrix and batch is destroyed; the
+// driver also takes them back for an allocation of this process that would
+// not fit otherwise. An allocation costs about a microsecond where cudaMalloc
+// and cudaFree take tens and wait for the device.
 constexpr size_t kScratchKept = size_t(512) << 20;
 cudaMemPool_t scratch_pool();
 template <class T>

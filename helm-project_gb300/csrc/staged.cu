@@ -1010,17 +1010,15 @@ int blocked_launches(const Matrix &m) {
 
 namespace {
 
-// Allows `kernel` its dynamic shared memory, once a device (the call costs
+// Allows `kernel` its dynamic shared memory, once a context (the call costs
 // about as much as a launch).
 template <auto kernel>
 void allow_smem(size_t bytes) {
-    static std::atomic<unsigned long long> done{0};  // bit per device
-    int dev = 0;
-    AXGB_CUDA(cudaGetDevice(&dev));
-    const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
-    if (done.load(std::memory_order_acquire) & bit) return;
+    static std::atomic<unsigned long long> done{0};  // the context it was last allowed in
+    const unsigned long long id = context_id();
+    if (done.load(std::memory_order_acquire) == id) return;
     AXGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
-    done.fetch_or(bit, std::memory_order_release);
+    done.store(id, std::memory_order_release);
 }
 
 template <int L, int T, int NS, int US>

@@ -17,7 +17,18 @@
  * (0 = the legacy default stream) and return once the work is enqueued;
  * host-pointer entry points are synchronous.
  * Nothing here allocates on the calling thread's behalf in the apply path
- * except the first use of a matrix in a given format (see axgb_matrix_prepare).
+ * except the first use of a matrix in a given format (see axgb_matrix_prepare)
+ * and the scratch of matrices whose sources are renumbered (axgb_matrix_stats).
+ *
+ * Scratch: weight generation, layout builds and that gather take device
+ * scratch from a memory pool of the library's own. While any mesh, matrix or
+ * batch handle lives the pool keeps up to 512 MiB of what was given back to
+ * it (other allocations of this process that need the memory get it, other
+ * processes do not); destroying the last handle returns all of it.
+ * Conservative generation takes up to 1 GiB of it for its candidate search
+ * (64 to 128 bytes a destination cell), besides what it takes for each
+ * candidate pair. CSR exports of more than a few MiB keep 8 MiB of pinned
+ * host memory in the same way.
  */
 #ifndef AXGB_H
 #define AXGB_H

@@ -9,6 +9,8 @@
 // runs on sorted node coordinates with a parallel sort. Everything after
 // that runs on the GPU.
 #include <cuda.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
@@ -204,119 +206,106 @@ void mesh_upload_impl(Mesh &m) {
     AXGB_CUDA(cudaDeviceSynchronize());
 }
 
-// Downloads into pageable host memory (a caller's fresh arrays): each of
-// kThreads host threads moves every kThreads-th piece of kPiece bytes through
-// two pinned slots of its own, so the copies from the device, the copies into
-// the arrays and, above all, the page faults of fresh memory run side by side
-// (one cudaMemcpy into pageable memory takes them one after another). int32
-// indices are widened to int64 on the way. The slots (8 MiB) and streams are
-// kept until the last handle is destroyed; one download at a time. Export of
-// the 0.25 deg -> C384 weights, 105 MB: 2.4 ms, against 22-33 ms.
-struct Downloader {
+// Downloads into pageable host memory (a caller's arrays). A copy into memory
+// that the process has touched runs at 150 GB/s; into fresh memory the page
+// faults take most of the time, one after another (8 MiB: 52 against 450 us).
+// So some host threads take piece after piece, touch its pages and copy it;
+// int32 indices are widened to int64 on the way.
+// Nothing is kept between downloads.
+// Starting a thread costs some 20 to 40 us, so there is one for every 2.5 MiB, and
+// none up to kResident where the arrays' pages are there. By MiB on the device,
+// into memory that was there / fresh memory, in us: one thread; this rule;
+// eight threads with two pinned slots each, kept between calls:
+//   1.5   134 / 958     159 / 250      433 / 419
+//   4.6   252 / 2040    233 / 348      391 / 434
+//   12.2  601 / 7550    428 / 630      592 / 627
+//   24.8  12700         823            664 / 882
+//   76    50700         1438 / 1945    1680 / 2007
+// Pieces of 1 MiB: 1898 / 2545 at 76 MiB (a copy's latency, some 20 us, is not
+// shared by the threads).
+struct Download {
     static constexpr int kThreads = 8;
-    static constexpr size_t kPiece = size_t(512) << 10;
-    static constexpr size_t kSmall = size_t(1) << 20;  // below: plain copies
+    static constexpr size_t kPiece = size_t(2) << 20;
+    static constexpr size_t kSmall = size_t(1) << 20;     // below: no threads
+    static constexpr size_t kResident = size_t(4) << 20;  // below: none if no page has to be made
+    static constexpr size_t kPerThread = size_t(5) << 19;
     struct Piece {
         const void *dev;
         void *host;
         size_t n;    // elements
         bool widen;  // int32 on the device, int64 on the host
     };
-    std::mutex mu;
-    char *slots = nullptr;
-    cudaStream_t st[kThreads] = {};
+    std::vector<Piece> pieces;
+    size_t total = 0;  // bytes on the device
 
-    // The current context's; those of ended contexts are not touched again.
-    static Downloader &get() {
-        static std::mutex all_mu;
-        static std::map<unsigned long long, Downloader> all;
-        const unsigned long long id = context_id();
-        std::lock_guard<std::mutex> lk(all_mu);
-        return all[id];
-    }
-    void release() {
-        for (auto &q : st) {
-            if (q) cudaStreamDestroy(q);
-            q = nullptr;
-        }
-        if (slots) cudaFreeHost(slots);
-        slots = nullptr;
-    }
     // size: bytes of an element on the device
-    static void add(std::vector<Piece> &v, const void *dev, void *host, i64 n, size_t size, bool widen) {
+    void add(const void *dev, void *host, i64 n, size_t size, bool widen) {
         if (!host || n <= 0) return;
         const size_t per = kPiece / size;
         for (size_t b = 0; b < static_cast<size_t>(n); b += per) {
             const size_t m = std::min(per, static_cast<size_t>(n) - b);
-            v.push_back({static_cast<const char *>(dev) + b * size,
-                         static_cast<char *>(host) + b * size * (widen ? 2 : 1), widen ? m : m * size, widen});
+            pieces.push_back({static_cast<const char *>(dev) + b * size,
+                              static_cast<char *>(host) + b * size * (widen ? 2 : 1), widen ? m : m * size, widen});
         }
+        total += static_cast<size_t>(n) * size;
     }
-    static void put(const Piece &p, const char *from) {
-        if (!p.widen) {
-            std::memcpy(p.host, from, p.n);
-            return;
-        }
-        const int32_t *a = reinterpret_cast<const int32_t *>(from);
-        int64_t *b = static_cast<int64_t *>(p.host);
-        for (size_t k = 0; k < p.n; ++k) b[k] = a[k];
-    }
-    static size_t dev_bytes(const Piece &p) { return p.widen ? p.n * sizeof(int32_t) : p.n; }
 
-    void run(const std::vector<Piece> &v) {
-        size_t total = 0;
-        for (auto &p : v) total += dev_bytes(p);
-        if (total <= kSmall) {
-            std::vector<char> buf(kPiece);
-            for (auto &p : v) {
-                char *to = p.widen ? buf.data() : static_cast<char *>(p.host);
-                AXGB_CUDA(cudaMemcpy(to, p.dev, dev_bytes(p), cudaMemcpyDeviceToHost));
-                if (p.widen) put(p, to);
-            }
-            return;
+    // A widened piece is copied into the upper half of its array and widened from
+    // there, block after block upwards: writing up to entry k reaches byte 8 k of
+    // the array, the entries from k on lie from byte 4 n + 4 k up. (A buffer of
+    // its own would be mapped and unmapped on each call, which costs more here.)
+    static cudaError_t copy(const Piece &p) {
+        char *to = static_cast<char *>(p.host) + (p.widen ? p.n * sizeof(int32_t) : 0);
+        const size_t bytes = p.widen ? p.n * sizeof(int32_t) : p.n;
+        for (size_t o = 0; o < bytes; o += 4096) static_cast<volatile char *>(to)[o] = 0;
+        const cudaError_t e = cudaMemcpy(to, p.dev, bytes, cudaMemcpyDeviceToHost);
+        if (!p.widen || e != cudaSuccess) return e;
+        int64_t *wide = static_cast<int64_t *>(p.host);
+        constexpr size_t kBlock = 2048;
+        int32_t in[kBlock];
+        for (size_t k = 0; k < p.n; k += kBlock) {
+            const size_t m = std::min(kBlock, p.n - k);
+            std::memcpy(in, to + k * sizeof(int32_t), m * sizeof(int32_t));
+            for (size_t q = 0; q < m; ++q) wide[k + q] = in[q];
         }
-        std::lock_guard<std::mutex> lk(mu);
+        return e;
+    }
+
+    // The process has the first, middle and last page of every piece's array.
+    bool resident() const {
+        const auto page = static_cast<std::uintptr_t>(sysconf(_SC_PAGESIZE));
+        for (const Piece &p : pieces) {
+            const auto a = reinterpret_cast<std::uintptr_t>(p.host);
+            const size_t bytes = p.widen ? p.n * sizeof(int64_t) : p.n;
+            for (size_t at : {size_t(0), bytes / 2, bytes - 1}) {
+                unsigned char there = 0;
+                if (mincore(reinterpret_cast<void *>((a + at) / page * page), 1, &there) != 0 || !(there & 1)) return false;
+            }
+        }
+        return true;
+    }
+    int threads() const {
+        if (total <= kSmall || (total <= kResident && resident())) return 1;
+        return static_cast<int>(std::clamp<size_t>(1 + total / kPerThread, 2, kThreads));
+    }
+
+    void run() const {
+        const int used = threads();
         int dev = 0;
         AXGB_CUDA(cudaGetDevice(&dev));
-        if (!slots) {
-            try {
-                for (auto &q : st) AXGB_CUDA(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
-                void *h = nullptr;
-                AXGB_CUDA(cudaHostAlloc(&h, 2 * kThreads * kPiece, cudaHostAllocDefault));
-                slots = static_cast<char *>(h);
-            } catch (...) {
-                release();
-                throw;
-            }
-        }
-        std::atomic<int> failed{0};
-        auto work = [&](int w) {
-            if (cudaSetDevice(dev) != cudaSuccess) {
-                failed = static_cast<int>(cudaErrorUnknown);
-                return;
-            }
-            char *slot[2] = {slots + 2 * w * kPiece, slots + (2 * w + 1) * kPiece};
-            auto load = [&](size_t i, int q) {
-                return cudaMemcpyAsync(slot[q], v[i].dev, dev_bytes(v[i]), cudaMemcpyDeviceToHost, st[w]);
-            };
-            cudaError_t e = static_cast<size_t>(w) < v.size() ? load(w, 0) : cudaSuccess;
-            int q = 0;
-            for (size_t i = w; i < v.size() && e == cudaSuccess && !failed; i += kThreads, q ^= 1) {
-                e = cudaStreamSynchronize(st[w]);
-                if (e == cudaSuccess && i + kThreads < v.size()) e = load(i + kThreads, q ^ 1);
-                if (e == cudaSuccess) put(v[i], slot[q]);
-            }
-            const cudaError_t f = cudaStreamSynchronize(st[w]);
-            if (e == cudaSuccess) e = f;
-            if (e != cudaSuccess) failed = static_cast<int>(e);
+        std::atomic<size_t> next{0};
+        std::atomic<int> failed{cudaSuccess};
+        auto work = [&](bool own) {
+            cudaError_t e = own ? cudaSuccess : cudaSetDevice(dev);
+            for (size_t i; e == cudaSuccess && !failed && (i = next++) < pieces.size();) e = copy(pieces[i]);
+            if (e != cudaSuccess) failed = e;
         };
         std::vector<std::thread> th;
         try {
-            for (int w = 1; w < kThreads; ++w) th.emplace_back(work, w);
-        } catch (...) {  // no more threads: this one takes the pieces left
-            for (int w = static_cast<int>(th.size()) + 1; w < kThreads; ++w) work(w);
+            for (int w = 1; w < used; ++w) th.emplace_back(work, false);
+        } catch (...) {  // no more threads: those there are take all pieces
         }
-        work(0);
+        work(true);
         for (auto &t : th) t.join();
         AXGB_CUDA(static_cast<cudaError_t>(failed.load()));
     }
@@ -332,14 +321,11 @@ struct ScratchPools {
 };
 
 // What the current context's pool keeps goes back to the device (blocks in
-// use stay), the downloads' pinned slots to the host.
+// use stay).
 void scratch_give_back() {
     unsigned long long id = 0;
     try {
         id = context_id();
-        auto &D = Downloader::get();
-        std::lock_guard<std::mutex> lk(D.mu);
-        D.release();
     } catch (const Error &) {
         return;  // no context: nothing is held
     }
@@ -878,15 +864,15 @@ int axgb_matrix_export_csr(int h, int64_t *row_ptr, int64_t *col_idx, double *va
     AXGB_TRY({
         auto m = Registry::get().find(Registry::get().mats, h, "matrix");
         AXGB_CUDA(cudaDeviceSynchronize());  // the matrix is complete before other streams read it
-        std::vector<Downloader::Piece> v;
-        Downloader::add(v, m->row_ptr.p, row_ptr, m->n_dst + 1, sizeof(int), true);
-        Downloader::add(v, m->col.p, col_idx, m->nnz, sizeof(int), true);
-        Downloader::add(v, m->val.p, values, m->nnz, sizeof(double), false);
-        Downloader::add(v, m->frac_a.p, frac_a, m->n_src, sizeof(double), false);
-        Downloader::add(v, m->frac_b.p, frac_b, m->n_dst, sizeof(double), false);
-        Downloader::add(v, m->area_a.p, area_a, m->n_src, sizeof(double), false);
-        Downloader::add(v, m->area_b.p, area_b, m->n_dst, sizeof(double), false);
-        Downloader::get().run(v);
+        Download d;
+        d.add(m->row_ptr.p, row_ptr, m->n_dst + 1, sizeof(int), true);
+        d.add(m->col.p, col_idx, m->nnz, sizeof(int), true);
+        d.add(m->val.p, values, m->nnz, sizeof(double), false);
+        d.add(m->frac_a.p, frac_a, m->n_src, sizeof(double), false);
+        d.add(m->frac_b.p, frac_b, m->n_dst, sizeof(double), false);
+        d.add(m->area_a.p, area_a, m->n_src, sizeof(double), false);
+        d.add(m->area_b.p, area_b, m->n_dst, sizeof(double), false);
+        d.run();
     });
 }
 

@@ -98,8 +98,7 @@ struct DBuf {
 };
 
 // What the library keeps per process and device (scratch pool, kernels' shared-
-// memory limits, the export's streams and slots) belongs to a CUDA context and
-// goes with it: cudaDeviceReset ends the context, and the next call makes
+// memory limits) belongs to a CUDA context and goes with it: cudaDeviceReset ends the context, and the next call makes
 // another, at the same address. This is the id of the calling thread's current
 // context, which is never given out twice (about 10 ns).
 unsigned long long context_id();

@@ -27,8 +27,7 @@
  * processes do not); destroying the last handle returns all of it.
  * Conservative generation takes up to 1 GiB of it for its candidate search
  * (64 to 128 bytes a destination cell), besides what it takes for each
- * candidate pair. CSR exports of more than a few MiB keep 8 MiB of pinned
- * host memory in the same way.
+ * candidate pair.
  */
 #ifndef AXGB_H
 #define AXGB_H

@@ -1,7 +1,6 @@
 """New handles after a context reset work as the first ones did: what the
-library keeps per process (scratch pool, kernels' shared-memory limits, the
-export's streams and slots) is not carried over from the ended context. Run in
-a child process."""
+library keeps per process (scratch pool, kernels' shared-memory limits) is not
+carried over from the ended context. Run in a child process."""
 import os
 import subprocess
 import sys

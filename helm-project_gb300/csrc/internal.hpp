@@ -216,6 +216,7 @@ struct Blocked {
         int L;        // row-length class (multiple of 4, <= 32)
         int us;       // staging floats per field (allocation for the class)
         i64 begin, n; // range in block_ids
+        bool in_order = false;  // most warps hold consecutive rows, so that their stores fill sectors
     };
     std::atomic<bool> built{false};  // set last, by matrix_prepare under Matrix::mu; read without it
     i64 n_blocks = 0;

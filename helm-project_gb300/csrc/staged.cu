@@ -66,6 +66,11 @@ const int kUsBuckets[] = {kUsSmall, kUsLarge};
 // tile costs whatever its rows, the waits and copies, is then shared by more
 // fields. 100 fields of C48 -> 0.25 deg: 168 -> 146 us. (A stride of 512 with 8
 // fields for C192 -> 0.5 deg: 380 us against 371 for 500 fields.)
+// Not with hi+lo outputs where the order by length scatters a warp's rows over
+// the block: its stores fill sectors only together with the other warps', which
+// are up to 32 fields apart with this form, times two arrays. 100 fields with hi+lo:
+// C192 -> 0.25 deg (rows of 1 to 4) 371 us with 16 fields a stage, 286 with 4;
+// 1 -> 0.25 deg (rows of 1) 163 and 224. One output: 174 and 204, 125 and 166.
 constexpr int kUsTiny = 256, kTinyT = 16, kTinyBatchT = 8;
 constexpr int kShortL = 8;
 // Zero floats staged after a block's chunks, one in every shared-memory bank:
@@ -969,6 +974,17 @@ void build_blocked(Matrix &m, cudaStream_t s) {
         l.begin = static_cast<i64>(ids.size());
         l.n = static_cast<i64>(kv.second.size());
         ids.insert(ids.end(), kv.second.begin(), kv.second.end());
+        i64 warps = 0, in_order = 0;
+        for (int b : kv.second)
+            for (int w = 0; w < kWarps; ++w) {
+                const int *r = hb[b].rows + 32 * w;
+                if (r[0] < 0) continue;
+                ++warps;
+                bool consecutive = true;
+                for (int t = 1; t < 32; ++t) consecutive &= r[t] < 0 || r[t] == r[0] + t;
+                in_order += consecutive;
+            }
+        l.in_order = 4 * in_order >= 3 * warps;
         B.launches.push_back(l);
     }
     B.order.resize(B.launches.size());
@@ -1069,11 +1085,12 @@ int ws_auto_stages() {
     return ns;
 }
 
+// in_order: most warps hold consecutive rows.
 template <int L, int T>
-void launch_ws(const BlkArgs &a, int us, int ns, i64 grid, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs,
-               cudaStream_t s) {
+void launch_ws(const BlkArgs &a, int us, bool in_order, int ns, i64 grid, const float *x, i64 ldx, float *y, i64 ldy,
+               i64 nrhs, cudaStream_t s) {
     if constexpr (L <= kShortL) {
-        if (us <= kUsTiny) {
+        if (us <= kUsTiny && (in_order || !a.ylo)) {
             BlkArgs b = a;
             b.fchunk = (a.fchunk + kTinyT - 1) / kTinyT * kTinyT;
             const i64 g = b.nbl * ((nrhs + b.fchunk - 1) / b.fchunk);
@@ -1117,7 +1134,7 @@ void launch_one(const Blocked &B, const Blocked::Launch &l, int kind, int ns, co
     a.status = B.status.p;
     a.n_src = B.n_src;
     if (kind == 3) {
-        if constexpr (T == 4) launch_ws<L, T>(a, l.us, ns, grid, x, ldx, y, ldy, nrhs, s);  // four fields per stage only
+        if constexpr (T == 4) launch_ws<L, T>(a, l.us, l.in_order, ns, grid, x, ldx, y, ldy, nrhs, s);  // four fields per stage only
     } else if (bulk) {
         size_t bytes = sizeof(float) * static_cast<size_t>(l.us) * 2 * T;
         AXGB_CUDA(cudaFuncSetAttribute(k_blk_bulk<L, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -1,0 +1,49 @@
+"""The staged kernels' forms for blocks of short rows that stage little, chosen
+by field count, row order and outputs: bit for bit against the direct kernel,
+the low parts of hi+lo outputs included."""
+import numpy as np
+import pytest
+
+from test_gpu_apply_shapes import _check_split, _reference
+
+pytestmark = pytest.mark.gpu
+
+
+def _fine(gpu, lens, n_src, seed):
+    """A destination much finer than the source: rows of the given lengths over neighbouring cells."""
+    rng = np.random.default_rng(seed)
+    n = len(lens)
+    rp = np.concatenate([[0], np.cumsum(lens)])
+    start = np.minimum(np.arange(n) * n_src // n, n_src - 9)
+    col = np.concatenate([s + np.sort(rng.choice(9, k, replace=False)) for s, k in zip(start, lens)])
+    return gpu.Matrix.from_csr(n_src, n, rp, col, rng.uniform(0.1, 1.0, rp[-1]))
+
+
+def _staged_and_direct(gpu, M, xs, fpp):
+    """(y, lo) of the hi+lo apply by the producer-warp kernel and by the direct one."""
+    nf, out = xs.shape[0], []
+    for v, u, st in ((3, 4, 0), (4, 1, 2)):
+        gpu.set_kernel_choice(M, nf, variant=v, fields_per_pass=fpp, unroll=u, stages=st)
+        out.append(gpu.apply_f32split_hilo(M, xs))
+    return out
+
+
+@pytest.mark.parametrize("rows", ["uniform", "mixed", "eight"])
+@pytest.mark.parametrize("nf,fpp", [(1, 0), (15, 0), (16, 0), (17, 0), (33, 16), (40, 20), (100, 0), (100, 52)])
+def test_hilo_of_blocks_that_stage_little(gpu, oracle, rows, nf, fpp):
+    """Rows of one length keep their order (16 fields a stage), rows of mixed
+    lengths do not (4 fields a stage with two outputs)."""
+    import torch
+    rng = np.random.default_rng(71)
+    lens = {"uniform": np.full(3001, 2), "mixed": rng.integers(1, 5, 3001), "eight": rng.integers(0, 9, 3001)}[rows]
+    M = _fine(gpu, lens, 500, 72)
+    X = rng.standard_normal((nf, 500)).astype(np.float32)
+    xs = torch.tensor(X, device="cuda")
+    (y, lo), (y2, lo2) = _staged_and_direct(gpu, M, xs, fpp)
+    assert torch.equal(y, y2) and torch.equal(lo, lo2)
+    ref, cond = _reference(M, oracle, X)
+    _check_split(y.cpu().numpy(), ref, cond)
+    # y + lo carries the sum to 2^-46 a term (as the module's note on tolerances has it)
+    assert np.all(np.abs(y.cpu().numpy().astype(np.float64) + lo.cpu().numpy() - ref) <= 1e-10 * cond)
+    assert torch.equal(gpu.apply_f32split(M, xs), y2)
+    assert M.device_status() == 0

@@ -226,7 +226,9 @@ struct Blocked {
     DBuf<unsigned short> lidx;
     DBuf<float> hi, lo;
     std::vector<Launch> launches;
-    std::vector<int> order;  // launches by size, largest first
+    // the launches, largest first; the same with the blocks that stage little
+    // in one launch with the others of their length class
+    std::vector<Launch> by_size, joined;
     i64 n_fallback = 0;
     DBuf<int> status;  // device status word: 1 = a bounded wait timed out
     // stream pool for concurrent class launches (fork/join on the caller's stream)

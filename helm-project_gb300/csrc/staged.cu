@@ -73,6 +73,11 @@ const int kUsBuckets[] = {kUsSmall, kUsLarge};
 // 1 -> 0.25 deg (rows of 1) 163 and 224. One output: 174 and 204, 125 and 166.
 constexpr int kUsTiny = 256, kTinyT = 16, kTinyBatchT = 8;
 constexpr int kShortL = 8;
+// Up to so many (entry, field) they are not launched apart from the others of
+// their length class, since a launch and its events cost 2 to 4 us: 8 fields of
+// C96 -> 0.5 deg bilinear 12.2 us, 14.4 apart; 12: 14.7 and 14.6. From there on they
+// gain (8 fields of C384 -> 0.25 deg, 34 million: 50 us joined, 47 apart).
+constexpr i64 kJoinWork = 12000000;
 // Zero floats staged after a block's chunks, one in every shared-memory bank:
 // a padding read can then take a bank no entry of its gather step uses. A
 // block whose chunks nearly fill its staging stride gets what is left (at
@@ -987,10 +992,21 @@ void build_blocked(Matrix &m, cudaStream_t s) {
         l.in_order = 4 * in_order >= 3 * warps;
         B.launches.push_back(l);
     }
-    B.order.resize(B.launches.size());
-    for (size_t q = 0; q < B.order.size(); ++q) B.order[q] = static_cast<int>(q);
-    std::stable_sort(B.order.begin(), B.order.end(),
-                     [&](int p1, int p2) { return B.launches[p1].n > B.launches[p2].n; });
+    auto sorted = [](std::vector<Blocked::Launch> v) {
+        std::stable_sort(v.begin(), v.end(), [](const auto &a, const auto &b) { return a.n > b.n; });
+        return v;
+    };
+    B.by_size = sorted(B.launches);
+    std::vector<Blocked::Launch> joined;  // (L, kUsTiny) comes right before (L, kUsSmall)
+    for (const Blocked::Launch &l : B.launches) {
+        if (!joined.empty() && joined.back().L == l.L && joined.back().us == kUsTiny && l.us == kUsSmall) {
+            joined.back().us = kUsSmall;
+            joined.back().n += l.n;
+        } else {
+            joined.push_back(l);
+        }
+    }
+    B.joined = sorted(std::move(joined));
     B.n_blocks = nb;
     B.n_src = m.n_src;
     B.brow.upload_vec(brow, s);
@@ -1361,12 +1377,13 @@ void apply_blocked(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, i64 nr
         }
         AXGB_CUDA(cudaEventCreateWithFlags(&B.fork, cudaEventDisableTiming));
     }
+    const std::vector<Blocked::Launch> &launches = m.nnz * nrhs <= kJoinWork ? B.joined : B.by_size;
     // the largest class stays on the caller's stream, the others go round the pool
-    const int used = static_cast<int>(std::min<size_t>(kPool, B.order.empty() ? 0 : B.order.size() - 1));
+    const int used = static_cast<int>(std::min<size_t>(kPool, launches.empty() ? 0 : launches.size() - 1));
     if (used > 0) AXGB_CUDA(cudaEventRecord(B.fork, s));
     for (int q = 0; q < used; ++q) AXGB_CUDA(cudaStreamWaitEvent(B.pool[q], B.fork, 0));
-    for (size_t i = 0; i < B.order.size(); ++i) {
-        const Blocked::Launch &l = B.launches[B.order[i]];
+    for (size_t i = 0; i < launches.size(); ++i) {
+        const Blocked::Launch &l = launches[i];
         const size_t slot = i % (kPool + 1);
         cudaStream_t st = slot == 0 ? s : B.pool[slot - 1];
         if (T >= 8)

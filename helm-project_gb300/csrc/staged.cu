@@ -1108,7 +1108,10 @@ void launch_ws(const BlkArgs &a, int us, bool in_order, int ns, i64 grid, const 
     if constexpr (L <= kShortL) {
         if (us <= kUsTiny && (in_order || !a.ylo)) {
             BlkArgs b = a;
-            b.fchunk = (a.fchunk + kTinyT - 1) / kTinyT * kTinyT;
+            // whole stages, and about 1800 items: a stage does more here than elsewhere. 24
+            // fields of C96 -> 0.5 deg bilinear: 19.9 us in one item, 22.8 in 16 + 8.
+            const i64 fc = std::max(a.fchunk, std::min<i64>(128, b.nbl * nrhs / 1800));
+            b.fchunk = (fc + kTinyT - 1) / kTinyT * kTinyT;
             const i64 g = b.nbl * ((nrhs + b.fchunk - 1) / b.fchunk);
             launch_ws_us<L, kTinyT, 2, kUsTiny>(b, g, x, ldx, y, ldy, nrhs, s);
             return;

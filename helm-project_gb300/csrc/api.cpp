@@ -509,11 +509,17 @@ void host_batch(Matrix &m, const T *src, T *dst, int64_t n_vars, F apply_fn) {
 // down to 16, in chunks of equal size. 64 fields of C192 -> 0.5 deg: 61 us with
 // 32, 71 with 64; 300 of C96 -> 1 deg: 68 us with 32, 85 with 128; 300 of C384 ->
 // 0.25 deg: 819 us with 128, 934 with 32.
+// Where all blocks are one launch, no other class fills its tail, and longer
+// items do better: about 2400, the last one what is left. 0.25 -> 0.5 deg: 150
+// fields in 128 + 22 131 us, in 2 x 76 136; 100 in 84 + 16 91, in 2 x 52 96; 24 in 20 + 4
+// 31.5, in 2 x 12 33.2.
 int default_item_fields(const Matrix &m, i64 nrhs) {
     const i64 blocks = std::max<i64>(1, (m.n_dst + 127) / 128);
-    const i64 most = std::min<i64>(128, std::max<i64>(16, blocks * nrhs / 3600));
+    const bool one = m.blocked.launches.size() == 1;
+    const i64 most = std::min<i64>(128, std::max<i64>(16, blocks * nrhs / (one ? 2400 : 3600)));
     const i64 chunks = (nrhs + most - 1) / most;
-    return static_cast<int>(((nrhs + chunks - 1) / chunks + 3) / 4 * 4);
+    const i64 fields = one ? most : std::max<i64>(16, (nrhs + chunks - 1) / chunks);
+    return static_cast<int>((fields + 3) / 4 * 4);
 }
 
 // The direct kernel, one launch that reads the sources from L1 and L2, or the

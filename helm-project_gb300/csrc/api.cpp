@@ -530,11 +530,13 @@ int default_item_fields(const Matrix &m, i64 nrhs) {
 // for one or two fields always. Direct against staged: 16 fields of C96 -> 1
 // deg 10.4 against 17.5 us, 4 of C384 -> 0.25 deg 38.8 against 32.2; 16 of 0.5
 // deg -> C192 (ten launches) 31.8 against 44.3, 64 of it 117.8 against 113.7.
+// The direct kernel walks fields eight at a time, so 10 count as 16 (C192 -> 0.5
+// deg: 24.8 us direct, 20.0 staged).
 // The matrix has its split layouts.
 SplitParams default_split_params(const Matrix &m, i64 nrhs) {
     SplitParams p;
-    const i64 launches = split_launches(m);
-    if (nrhs <= 2 || m.nnz * nrhs <= i64(4000000) * launches) {
+    const i64 walked = nrhs <= 4 ? nrhs : (nrhs + 7) / 8 * 8;
+    if (nrhs <= 2 || m.nnz * walked <= i64(4000000) * split_launches(m, nrhs)) {
         p.variant = 4;
         p.fields_per_pass = 0;
         p.unroll = 1;

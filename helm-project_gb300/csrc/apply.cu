@@ -1558,7 +1558,9 @@ void gather_source(const Matrix &m, const float *x, i64 ldx, i64 nrhs, float *xr
     AXGB_CUDA(cudaGetLastError());
 }
 
-int split_launches(const Matrix &m) { return blocked_launches(m) + (m.sell32.n_lrows > 0 ? 1 : 0); }
+int split_launches(const Matrix &m, i64 nrhs) {
+    return static_cast<int>(staged_launches(m, nrhs).size()) + (m.blocked.n_fallback > 0 ? 1 : 0) + (m.sell32.n_lrows > 0 ? 1 : 0);
+}
 
 void apply_split_layouts(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, const SplitParams &p,
                          cudaStream_t s, float *ylo, i64 ldylo);

@@ -402,7 +402,8 @@ void apply_segmented(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, i64 
 void apply_blocked(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, int kind, int T, int ns,
                    i64 fchunk, cudaStream_t s, float *ylo = nullptr, i64 ldylo = 0);
 int blocked_launches(const Matrix &m);
-int split_launches(const Matrix &m);  // launches of a staged apply, long rows included
+int split_launches(const Matrix &m, i64 nrhs);  // launches of a staged apply, long rows included
+const std::vector<Blocked::Launch> &staged_launches(const Matrix &m, i64 nrhs);  // its staged ones, in launch order
 // persistent staged kernels over the blocked layouts of several matrices
 // (batches); use[q] selects the matrices whose fields allow the staged kernels
 struct BlkBatch;

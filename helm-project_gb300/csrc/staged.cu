@@ -1364,6 +1364,10 @@ void blk_batch_launch(BlkBatch &bb, const cudaStream_t *streams, int n_streams) 
     AXGB_CUDA(cudaGetLastError());
 }
 
+const std::vector<Blocked::Launch> &staged_launches(const Matrix &m, i64 nrhs) {
+    return m.nnz * nrhs <= kJoinWork ? m.blocked.joined : m.blocked.by_size;
+}
+
 void apply_blocked(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, int kind, int T, int ns,
                    i64 fchunk, cudaStream_t s, float *ylo, i64 ldylo) {
     Blocked &B = m.blocked;
@@ -1380,7 +1384,7 @@ void apply_blocked(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, i64 nr
         }
         AXGB_CUDA(cudaEventCreateWithFlags(&B.fork, cudaEventDisableTiming));
     }
-    const std::vector<Blocked::Launch> &launches = m.nnz * nrhs <= kJoinWork ? B.joined : B.by_size;
+    const std::vector<Blocked::Launch> &launches = staged_launches(m, nrhs);
     // the largest class stays on the caller's stream, the others go round the pool
     const int used = static_cast<int>(std::min<size_t>(kPool, launches.empty() ? 0 : launches.size() - 1));
     if (used > 0) AXGB_CUDA(cudaEventRecord(B.fork, s));

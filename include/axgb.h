@@ -277,8 +277,9 @@ int axgb_apply_f32split_hilo(int matrix_handle, const float *x, int64_t ld_x, fl
  * to 3 need x 16-byte aligned and ld_x a multiple of 4 (variant 2 also n_src
  * a multiple of 4); otherwise the direct kernel runs. variant 4: the direct
  * kernel with its own tile and unroll (the default for one or two fields,
- * and while weights * fields is at most 4 million for each launch that the
- * staged form would take); the other knobs are unused. variant 5: segmented,
+ * and while weights * fields, counted in eights above four, is at most 4
+ * million for each launch that the staged form would take); the other knobs
+ * are unused. variant 5: segmented,
  * one lane per field: groups of 32 nearby rows stage their distinct source
  * cells (original numbering, any x alignment) for 32 fields at a time;
  * stages = staging slots (2 or 3). Every variant gives the same bits. */

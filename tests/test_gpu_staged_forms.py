@@ -47,3 +47,38 @@ def test_hilo_of_blocks_that_stage_little(gpu, oracle, rows, nf, fpp):
     assert np.all(np.abs(y.cpu().numpy().astype(np.float64) + lo.cpu().numpy() - ref) <= 1e-10 * cond)
     assert torch.equal(gpu.apply_f32split(M, xs), y2)
     assert M.device_status() == 0
+
+
+def _blocks(gpu, lens, seed):
+    """Neighbouring rows share their sources: every block is staged."""
+    rng = np.random.default_rng(seed)
+    rp = np.concatenate([[0], np.cumsum(lens)])
+    start = np.arange(len(lens)) // 4
+    col = np.arange(rp[-1]) - np.repeat(rp[:-1] - start, lens)
+    return gpu.Matrix.from_csr(int(col.max()) + 1, len(lens), rp, col, rng.uniform(0.1, 1.0, rp[-1]))
+
+
+@pytest.mark.parametrize("nf", [3, 5, 10, 24, 40, 100, 129, 150])
+@pytest.mark.parametrize("kind", ["one class", "little and much", "many classes"])
+def test_default_split_of_the_fields(gpu, oracle, kind, nf):
+    """The default choice's work items, staged (little and much staging joined
+    and apart) and direct, against one item for all fields."""
+    import torch
+    rng = np.random.default_rng(81)
+    lens = {"one class": np.full(120000, 4), "little and much": np.full(120000, 3),
+            "many classes": np.repeat(np.arange(1, 33), 1900)}[kind]
+    M = _blocks(gpu, lens, 82)
+    if kind == "little and much":  # some blocks' sources lie apart
+        c = M.to_csr()
+        col = c["col"].reshape(-1, 3)
+        far = (np.arange(120000) // 128) % 3 == 0
+        col[far, 2] = M.n_src + np.arange(far.sum())
+        M = gpu.Matrix.from_csr(M.n_src + int(far.sum()), M.n_dst, c["row_ptr"], col.reshape(-1), c["val"])
+    X = rng.standard_normal((nf, (M.n_src + 3) // 4 * 4)).astype(np.float32)
+    xs = torch.tensor(X, device="cuda")[:, :M.n_src]
+    y = gpu.apply_f32split(M, xs)
+    assert torch.equal(gpu.apply_f32split(M, xs, fields_per_pass=0, unroll=4, variant=3), y)
+    assert torch.equal(gpu.apply_f32split(M, xs, fields_per_pass=0, unroll=1, variant=4), y)
+    _check_split(y.cpu().numpy()[:3], *_reference(M, oracle, X[:3, :M.n_src]))
+    assert gpu.get_kernel_choice(M, nf)["variant"] in ((3, 4) if nf >= 8 else (1, 4))
+    assert M.device_status() == 0

@@ -1239,11 +1239,8 @@ void persist_launch(const BlkDesc *d, int nd, i64 total, unsigned long long *cou
     k<<<static_cast<unsigned>(grid), kRows, bytes, s>>>(d, nd, total, counter);
 }
 
-// Two fields a stage with the largest stride: 49 KB of staging, four CTAs an
-// SM, where four fields (two CTAs) leave it at eight row warps (17-pair batch
-// 1096 -> 1010 us; the producer-warp kernel is better off with four).
-template <int US, int T = US == kUsLarge ? 2 : kBatchT>
-void persist_dispatch(int L, const BlkDesc *d, int nd, i64 total, unsigned long long *counter, cudaStream_t s) {
+template <int US, int T>
+void persist_class(int L, const BlkDesc *d, int nd, i64 total, unsigned long long *counter, cudaStream_t s) {
     switch (L) {
         case 4: persist_launch<4, US, T>(d, nd, total, counter, s); break;
         case 8: persist_launch<8, US, T>(d, nd, total, counter, s); break;
@@ -1254,6 +1251,23 @@ void persist_dispatch(int L, const BlkDesc *d, int nd, i64 total, unsigned long 
         case 28: persist_launch<28, US, T>(d, nd, total, counter, s); break;
         default: persist_launch<32, US, T>(d, nd, total, counter, s); break;
     }
+}
+
+// With the largest stride two fields a stage, 49 KB of staging, let four CTAs on
+// an SM, where four fields (two CTAs) leave it at eight row warps (17-pair batch
+// 1096 -> 1010 us; the producer-warp kernel is better off with four). Where two
+// CTAs an SM hold all items, more of them would be idle, and four fields take
+// half the stages: 37 fields of 0.5 deg -> C48, about 220 items in two classes, 30 us
+// a class against 47.
+template <int US>
+void persist_dispatch(int L, const BlkDesc *d, int nd, i64 total, unsigned long long *counter, cudaStream_t s) {
+    if constexpr (US == kUsLarge) {
+        if (total > 2 * 152) {
+            persist_class<US, 2>(L, d, nd, total, counter, s);
+            return;
+        }
+    }
+    persist_class<US, kBatchT>(L, d, nd, total, counter, s);
 }
 
 }  // namespace

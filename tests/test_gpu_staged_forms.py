@@ -82,3 +82,27 @@ def test_default_split_of_the_fields(gpu, oracle, kind, nf):
     _check_split(y.cpu().numpy()[:3], *_reference(M, oracle, X[:3, :M.n_src]))
     assert gpu.get_kernel_choice(M, nf)["variant"] in ((3, 4) if nf >= 8 else (1, 4))
     assert M.device_status() == 0
+
+
+@pytest.mark.parametrize("nfs", [(1, 5, 30, 2), (33, 40, 64, 17), (3, 3, 4, 4)])
+def test_batches_of_small_and_large_groups(gpu, nfs):
+    """Batches whose classes of few blocks are joined across lengths and
+    strides, beside large ones that are not; bit for bit the single applies."""
+    import torch
+    rng = np.random.default_rng(91)
+    few = np.repeat(np.arange(1, 33), 300)  # three blocks a length
+    wide = rng.integers(1, 33, 5000)        # scattered rows: large strides, some left to the slices
+    rp = np.concatenate([[0], np.cumsum(wide)])
+    start = np.minimum(np.arange(5000) * 4, 20000)
+    col = np.concatenate([s + np.sort(rng.choice(120, k, replace=False)) for s, k in zip(start, wide)])
+    ms = [_blocks(gpu, few, 92), gpu.Matrix.from_csr(20120, 5000, rp, col, rng.uniform(0.1, 1.0, rp[-1])),
+          _blocks(gpu, np.full(60000, 4), 93), _fine(gpu, rng.integers(0, 9, 9001), 1000, 94)]
+    xs = [torch.randn((n, (m.n_src + 3) // 4 * 4), device="cuda")[:, :m.n_src] for n, m in zip(nfs, ms)]
+    ys = [torch.full((n, m.n_dst), float("nan"), device="cuda") for n, m in zip(nfs, ms)]
+    B = gpu.Batch(ms, list(nfs))
+    for _ in range(2):
+        B.apply(xs, ys)
+        for m, x, y in zip(ms, xs, ys):
+            assert torch.equal(y, gpu.apply_f32split(m, x, fields_per_pass=0, unroll=1, variant=4))
+            assert m.device_status() == 0
+            y.fill_(float("nan"))

@@ -782,6 +782,7 @@ void build_sell(Matrix &m, int fmt, cudaStream_t s) {
             }
         if (fmt == 0) S.ord.upload_vec(rows_by_length(rp, n_rows, n_slices * 32), s);
         S.n_lrows = static_cast<i64>(lrow.size());
+        S.n_lentries = lptr.back();
         S.lrow.upload_vec(lrow, s);
         S.lptr.upload_vec(lptr, s);
         const size_t ne = std::max<size_t>(1, lptr.back());
@@ -1120,6 +1121,7 @@ __global__ void __launch_bounds__(256, U == 1 ? 4 : 2)
                 wsh[lane] = w;
 #pragma unroll
                 for (int f = 0; f < kNanG; ++f) {
+                    if (f >= nf) break;  // what the lanes without a field add up is not stored
                     const unsigned nan_mask = __ballot_sync(0xffffffffu, nan_bits(xv[f]));
                     if ((lane & 15) == f) skip = nan_mask;
                     ps[wp][f][lane] = __dmul_rn(w, xv[f]);
@@ -1671,15 +1673,22 @@ void nan_batch_apply_f64(Matrix &m, const double *x, i64 ldx, double *y, i64 ldy
     const Sell &S = m.sell64;
     // One field alone: without others side by side, twice the blocks an SM (0.25
     // -> 0.5 deg: 35 -> 26 us; eight entries ahead instead of four 28).
-    const auto kernel = nrhs == 1 ? k_nan<1, kNanK> : k_nan<kNanU, kNanK>;
-    const int rows_w = nan_rows_w(nrhs);
-    const i64 warps = (S.n_lrows + rows_w - 1) / rows_w + S.n_slices;
-    for (i64 f = 0; f < nrhs; f += 65535 * kNanG) {
-        const i64 nf = std::min<i64>(nrhs - f, 65535 * kNanG);
+    auto launch = [&](const double *xf, double *yf, i64 nf) {
+        const auto kernel = nf == 1 ? k_nan<1, kNanK> : k_nan<kNanU, kNanK>;
+        const int rows_w = nan_rows_w(nf);
+        const i64 warps = (S.n_lrows + rows_w - 1) / rows_w + S.n_slices;
         const dim3 grid(nblk(warps, 8), nblk(nf, kNanG));
-        kernel<<<grid, 256, 0, s>>>(sell_args(m, S), long_rows(S), S.total.p, S.ord.p, S.n_slices, x + f * ldx, ldx,
-                                    y + f * ldy, ldy, nf, rows_w, na_thres);
-    }
+        kernel<<<grid, 256, 0, s>>>(sell_args(m, S), long_rows(S), S.total.p, S.ord.p, S.n_slices, xf, ldx, yf, ldy, nf,
+                                    rows_w, na_thres);
+    };
+    // 9 to 11 fields leave the 16 lanes that add up a long row half empty: where long
+    // rows are a good part of the rows and not much above 32 entries, eight fields
+    // (two rows a warp) and then the others (five rows and more) are faster. C384 ->
+    // 41 k Voronoi cells (rows of 35), 9 fields: 322 us, 370 in one launch. Longer rows
+    // are chains whose length counts: 0.25 deg -> C48 815 us in one launch, 1665 in two.
+    const bool split = nrhs > 8 && nrhs < 12 && S.n_lrows * 8 > m.n_dst && S.n_lentries <= 48 * S.n_lrows;
+    const i64 most = split ? 8 : 65535 * kNanG;
+    for (i64 f = 0; f < nrhs; f += most) launch(x + f * ldx, y + f * ldy, std::min<i64>(nrhs - f, most));
     AXGB_CUDA(cudaGetLastError());
 }
 

@@ -199,7 +199,7 @@ struct Sell {
     DBuf<int> ord;          // rows of every 128 by length, longest first, with kOrdPlain (format 0)
     // Rows of more than 32 entries, row-contiguous in the layout's entry
     // order (for the warp-per-row kernels): row ids, offsets, entries.
-    i64 n_lrows = 0;
+    i64 n_lrows = 0, n_lentries = 0;
     DBuf<int> lrow, lptr, lcol;
     DBuf<float2> lhl;       // format 1
     DBuf<double> lw64;      // format 0

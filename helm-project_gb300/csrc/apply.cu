@@ -735,6 +735,32 @@ std::vector<int> rows_by_length(const std::vector<int> &rp, i64 n_rows, i64 n_po
     return ord;
 }
 
+// Rows of more than 32 entries in the order their kernels take them. Rows of
+// hundreds to thousands of entries (polar cells) are the kernels' length where
+// they are begun in the last wave, and slow one another on one SM: they come
+// first, the longest at the front, with others between them (a block of k_nan
+// takes up to 80 rows). The others keep their order, as neighbours share
+// sources. 0.25 deg -> C48 (rows of 33 to 4300), in row order and in this one: one
+// field 18.8 and 14.7 us, FP64 24.5 and 21.0, NaN-aware 630 and 593 (679 with the heavy rows
+// next to one another), 8 fields 38.7 and 31.6.
+std::vector<int> long_row_order(const std::vector<int> &rp, i64 n_rows) {
+    std::vector<int> rows, heavy, out;
+    for (i64 r = 0; r < n_rows; ++r) {
+        const int n = rp[r + 1] - rp[r];
+        if (n > 32) (n > 256 ? heavy : rows).push_back(static_cast<int>(r));
+    }
+    std::stable_sort(heavy.begin(), heavy.end(),
+                     [&](int a, int b) { return rp[a + 1] - rp[a] > rp[b + 1] - rp[b]; });
+    const size_t gap = heavy.empty() ? 0 : std::min<size_t>(79, rows.size() / heavy.size());
+    size_t at = 0;
+    for (int h : heavy) {
+        out.push_back(h);
+        for (size_t k = 0; k < gap; ++k) out.push_back(rows[at++]);
+    }
+    out.insert(out.end(), rows.begin() + at, rows.end());
+    return out;
+}
+
 void build_sell(Matrix &m, int fmt, cudaStream_t s) {
     Sell &S = fmt == 0 ? m.sell64 : m.sell32;
     if (S.built) return;
@@ -774,12 +800,9 @@ void build_sell(Matrix &m, int fmt, cudaStream_t s) {
     {
         std::vector<int> rp(n_rows + 1);
         AXGB_CUDA(cudaMemcpy(rp.data(), m.row_ptr.p, sizeof(int) * (n_rows + 1), cudaMemcpyDeviceToHost));
-        std::vector<int> lrow, lptr(1, 0);
-        for (i64 r = 0; r < n_rows; ++r)
-            if (rp[r + 1] - rp[r] > 32) {
-                lrow.push_back(static_cast<int>(r));
-                lptr.push_back(lptr.back() + rp[r + 1] - rp[r]);
-            }
+        std::vector<int> lptr(1, 0);
+        const std::vector<int> lrow = long_row_order(rp, n_rows);
+        for (int r : lrow) lptr.push_back(lptr.back() + rp[r + 1] - rp[r]);
         if (fmt == 0) S.ord.upload_vec(rows_by_length(rp, n_rows, n_slices * 32), s);
         S.n_lrows = static_cast<i64>(lrow.size());
         S.n_lentries = lptr.back();

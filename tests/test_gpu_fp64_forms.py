@@ -3,7 +3,7 @@ against the oracle's sums (bit for bit for the NaN-aware apply)."""
 import numpy as np
 import pytest
 
-from test_gpu_apply_shapes import _check_f64, _reference, _rows_matrix
+from test_gpu_apply_shapes import _check_f64, _check_split, _reference, _rows_matrix
 
 pytestmark = pytest.mark.gpu
 
@@ -33,3 +33,23 @@ def test_nan_fields_beside_long_rows(gpu, oracle, nf, lens):
     """Field counts that leave part of a long row's lanes without a field; 9 to
     11 in one launch and in two."""
     _nan_check(gpu, oracle, lens, nf, 61)
+
+
+@pytest.mark.parametrize("heavy", [1, 7, 30, 120])
+def test_heavy_rows_between_others(gpu, oracle, heavy):
+    """Rows of more than 256 entries come first in the long rows' list, others
+    between them: few, as many as the others, and more than those."""
+    import torch
+    rng = np.random.default_rng(71)
+    lens = np.concatenate([rng.integers(257, 1200, heavy), rng.integers(33, 257, 60), rng.integers(0, 33, 200)])
+    rng.shuffle(lens)
+    M = _rows_matrix(gpu, lens, 4000, 72)
+    for nf in (1, 5, 20):
+        X = np.random.default_rng(73).standard_normal((nf, M.n_src)).astype(np.float32)
+        xs = torch.tensor(X, device="cuda")
+        ref, cond = _reference(M, oracle, X)
+        y = gpu.apply_f32split(M, xs)
+        _check_split(y.cpu().numpy(), ref, cond)
+        assert torch.equal(gpu.apply_f32split(M, xs, fields_per_pass=0, unroll=4, variant=3), y)
+        _check_f64(gpu.apply_f64(M, xs.double()).cpu().numpy(), ref, cond)
+    _nan_check(gpu, oracle, lens, 3, 74)

@@ -587,6 +587,31 @@ __global__ void __launch_bounds__(256, 4)
     const int n = a.rlen[row];
     if (n > 32) return;
     const int e0 = a.base[row >> 5] + static_cast<int>(row & 31);
+    if (!kAll && __all_sync(__activemask(), n <= 1)) {
+        // Rows of one entry (nearest neighbour, a destination within the source's
+        // cells): it is loaded once, eight fields side by side. 100 fields of 1 -> 0.25
+        // deg: 218 us, 389 with two entries' loads for every four fields.
+        constexpr int U = 8;
+        const int c = n == 1 ? a.col[e0] : 0;
+        const double w = n == 1 ? a.w64[e0] : 0.0;
+        for (i64 f = fa; f < fb; f += U) {
+            const int nf = static_cast<int>(min(static_cast<i64>(U), fb - f));
+            const double *xf = x + f * ldx + c;
+            double *yf = y + f * ldy + row;
+            double v[U];
+            if (n == 1) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) v[u] = fma(w, __ldg(xf + min(u, nf - 1) * ldx), 0.0);
+            } else {
+#pragma unroll
+                for (int u = 0; u < U; ++u) v[u] = 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (u < nf) yf[u * ldy] = v[u];
+        }
+        return;
+    }
     for (i64 f = fa; f < fb; f += F) {
         const int nf = kAll ? F : static_cast<int>(min(static_cast<i64>(F), fb - f));
         const double *xf = x + f * ldx;

@@ -53,3 +53,27 @@ def test_heavy_rows_between_others(gpu, oracle, heavy):
         assert torch.equal(gpu.apply_f32split(M, xs, fields_per_pass=0, unroll=4, variant=3), y)
         _check_f64(gpu.apply_f64(M, xs.double()).cpu().numpy(), ref, cond)
     _nan_check(gpu, oracle, lens, 3, 74)
+
+
+@pytest.mark.parametrize("nf", [2, 3, 4, 7, 8, 9, 16, 65, 70])
+@pytest.mark.parametrize("lens", ["ones", "ones and none", "a warp of ones"])
+def test_rows_of_one_entry(gpu, oracle, nf, lens):
+    """Warps whose rows have one entry or none take eight fields at a time; the
+    others of the matrix do not."""
+    import torch
+    rng = np.random.default_rng(81)
+    n = 3001
+    l = {"ones": np.ones(n), "ones and none": rng.integers(0, 2, n),
+         "a warp of ones": np.where(np.arange(n) // 128 % 2, 1, rng.integers(0, 7, n))}[lens].astype(np.int64)
+    M = _rows_matrix(gpu, l, 900, 82)
+    X = rng.standard_normal((nf, M.n_src))
+    X[0, :5] = [np.inf, -np.inf, np.nan, -0.0, 0.0]
+    xs = torch.tensor(X, device="cuda")
+    d = gpu.apply_f64(M, xs).cpu().numpy()
+    X0 = X.copy()
+    X0[0, :3] = 1.0
+    _check_f64(d[1:], *(v[1:] for v in _reference(M, oracle, X0)))
+    for f in range(0, nf, max(1, nf // 6)):
+        one = gpu.apply_f64(M, xs[f:f + 1]).cpu().numpy()[0]
+        assert np.array_equal(one, d[f], equal_nan=True)
+        assert np.array_equal(np.signbit(one), np.signbit(d[f]))

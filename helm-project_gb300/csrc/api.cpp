@@ -398,8 +398,8 @@ void check_apply(const Matrix &m, const void *x, i64 ldx, const void *y, i64 ldy
 // cp.async staging; 2 or 3 buffers), 2 (blocked, bulk copies; 2 buffers),
 // 1 and 2 with 2, 4 or 8 fields per stage, 3 (blocked, producer warp and
 // mbarrier ring of 2 or 3 slots, or 0: per row-length class the depth that
-// lets more CTAs fit; 4 fields per stage); 4 (one fused launch
-// for few fields; the other knobs unused); 5 (segmented, lane = field, 32
+// lets more CTAs fit; 4 fields per stage); 4 (the direct kernel
+// with its own tile and up to eight fields side by side; the other knobs unused); 5 (segmented, lane = field, 32
 // fields per stage, 2 or 3 staging slots).
 void check_split_params(const SplitParams &p, const char *who) {
     const std::string w(who);
@@ -437,7 +437,7 @@ SplitParams tune_split(Matrix &m, const float *x, i64 ldx, float *y, i64 ldy, i6
         for (int u : {2, 4})
             if (u <= std::max<i64>(1, nrhs)) cands.push_back({0, static_cast<int>(t), u});
     if (nrhs == 1) cands.push_back({0, 1, 1});
-    if (nrhs <= 8) cands.push_back({4, 0, 1, 2});
+    cands.push_back({4, 0, 1, 2});
     cudaEvent_t e0, e1;
     AXGB_CUDA(cudaEventCreate(&e0));
     AXGB_CUDA(cudaEventCreate(&e1));

@@ -89,3 +89,70 @@ def test_default_choice_before_and_after_the_layouts(gpu, nf, direct):
     M.prepare(2)
     assert gpu.get_kernel_choice(M, nf) == ch
     assert ch["cached"] is False and (ch["variant"] == 4) is direct
+
+
+@pytest.mark.parametrize("nf", [1, 5, 40])
+def test_renumbered_apply_under_capture(gpu, nf):
+    """A split apply whose sources are gathered into scratch first, captured in a
+    graph (the scratch is then the graph's) and replayed on new fields."""
+    import torch
+    n_src, n_dst = 20003, 9000
+    rng = np.random.default_rng(61)
+    perm = rng.permutation(n_src)
+    lens = rng.integers(1, 8, n_dst)
+    rp = np.concatenate([[0], np.cumsum(lens)])
+    start = np.minimum(np.arange(n_dst) * n_src // n_dst, n_src - 8)
+    col = np.concatenate([np.sort(perm[s:s + n]) for s, n in zip(start, lens)])
+    M = gpu.Matrix.from_csr(n_src, n_dst, rp, col, rng.uniform(0.1, 1.0, rp[-1]))
+    M.prepare(2)
+    assert M.stats()["source_renumbered"]
+    x = torch.zeros((nf, n_src), device="cuda")
+    y = torch.empty((nf, n_dst), device="cuda")
+    for v, u in ((None, None), (3, 4)):
+        kw = {} if v is None else dict(fields_per_pass=0, unroll=u, variant=v)
+        gpu.apply_f32split(M, x, y, **kw)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            gpu.apply_f32split(M, x, y, **kw)
+        for k in range(3):
+            x.copy_(torch.randn((nf, n_src), device="cuda", generator=torch.Generator(device="cuda").manual_seed(k)))
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(y, gpu.apply_f32split(M, x))
+
+
+@pytest.mark.parametrize("nf", [6, 30])
+def test_one_matrix_on_two_streams(gpu, nf):
+    """Staged applies of one matrix, their largest class on the caller's stream and the
+    others on shared ones, from two streams in turn."""
+    import torch
+    M = _rows_matrix(gpu, _lens(30), 4000, 31)
+    M.prepare(2)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    xs = [torch.randn((nf, 4000), device="cuda") for _ in range(2)]
+    want = [gpu.apply_f32split(M, x, fields_per_pass=0, unroll=1, variant=4) for x in xs]
+    torch.cuda.synchronize()
+    ys = [[torch.full((nf, M.n_dst), float("nan"), device="cuda") for _ in range(8)] for _ in range(2)]
+    torch.cuda.synchronize()
+    for k in range(8):
+        for q, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                gpu.apply_f32split(M, xs[q], ys[q][k], fields_per_pass=0, unroll=4, variant=3 if k % 2 else 1)
+    torch.cuda.synchronize()
+    for q in range(2):
+        for y in ys[q]:
+            assert torch.equal(y, want[q])
+
+
+def test_autotuned_choice_of_small_work(gpu):
+    """Small work of more than eight fields: whatever is chosen (the direct kernel's own
+    form is among the candidates) gives the same bits and is kept."""
+    import torch
+    M = _rows_matrix(gpu, np.random.default_rng(40).choice(SHORT, 1000), 900, 41)
+    x = torch.randn((12, 900), device="cuda")
+    want = gpu.apply_f32split(M, x)
+    y = torch.empty_like(want)
+    best = gpu.autotune_f32split(M, x, y)
+    assert torch.equal(gpu.apply_f32split(M, x), want)
+    assert gpu.get_kernel_choice(M, 12)["cached"] is True and best is not None

@@ -77,3 +77,17 @@ def test_rows_of_one_entry(gpu, oracle, nf, lens):
         one = gpu.apply_f64(M, xs[f:f + 1]).cpu().numpy()[0]
         assert np.array_equal(one, d[f], equal_nan=True)
         assert np.array_equal(np.signbit(one), np.signbit(d[f]))
+
+
+@pytest.mark.parametrize("nf,rows", [(21, 64000), (29, 50001), (65, 64000)])
+def test_field_tiles_of_eight_and_more(gpu, oracle, nf, rows):
+    """Work for which a warp takes tiles of 8 fields, several of them and the last in part
+    (at least 38,912 slices times fields), and of 16."""
+    import torch
+    M = _rows_matrix(gpu, np.random.default_rng(91).integers(0, 9, rows), 900, 92)
+    X = np.random.default_rng(93).standard_normal((nf, M.n_src))
+    xs = torch.tensor(X, device="cuda")
+    d = gpu.apply_f64(M, xs).cpu().numpy()
+    _check_f64(d, *_reference(M, oracle, X))
+    for f in (0, 7, 8, 16, nf - 1):
+        assert np.array_equal(gpu.apply_f64(M, xs[f:f + 1]).cpu().numpy()[0], d[f])

@@ -206,48 +206,147 @@ void mesh_upload_impl(Mesh &m) {
     AXGB_CUDA(cudaDeviceSynchronize());
 }
 
-// Downloads into pageable host memory (a caller's arrays). A copy into memory
-// that the process has touched runs at 150 GB/s; into fresh memory the page
-// faults take most of the time, one after another (8 MiB: 52 against 450 us).
-// So some host threads take piece after piece, touch its pages and copy it;
-// int32 indices are widened to int64 on the way.
-// Nothing is kept between downloads.
-// Starting a thread costs some 20 to 40 us, so there is one for every 2.5 MiB, and
-// none up to kResident where the arrays' pages are there. By MiB on the device,
-// into memory that was there / fresh memory, in us: one thread; this rule;
-// eight threads with two pinned slots each, kept between calls:
+// CSR export: downloads into pageable host memory (a caller's arrays). What
+// takes the time is making the pages of fresh memory, one after another (8 MiB:
+// 450 us, 52 into memory that is there), so host threads share the work. int32
+// indices are widened to int64 on the way.
+struct Piece {
+    const void *dev;
+    void *host;
+    size_t n;    // elements
+    bool widen;  // int32 on the device, int64 on the host
+    size_t dev_bytes() const { return widen ? n * sizeof(int32_t) : n; }
+};
+
+// Large exports: each of kThreads host threads moves every kThreads-th piece
+// through two pinned slots of its own. The slots (8 MiB) and streams are kept
+// until the last handle is destroyed; one download at a time. Export of the 0.25
+// deg -> C384 weights, 105 MB: 1.7 ms (2.5 the first time), against 22-33 ms with
+// plain copies. (Copying straight into the arrays, as below, takes as long as a
+// rule and 6 to 11 ms now and then.)
+struct PinnedRing {
+    static constexpr int kThreads = 8;
+    static constexpr size_t kPiece = size_t(512) << 10;
+    std::mutex mu;
+    char *slots = nullptr;
+    cudaStream_t st[kThreads] = {};
+
+    // The current context's; those of ended contexts are not touched again.
+    static PinnedRing &get() {
+        static std::mutex all_mu;
+        static std::map<unsigned long long, PinnedRing> all;
+        const unsigned long long id = context_id();
+        std::lock_guard<std::mutex> lk(all_mu);
+        return all[id];
+    }
+    void release() {
+        for (auto &q : st) {
+            if (q) cudaStreamDestroy(q);
+            q = nullptr;
+        }
+        if (slots) cudaFreeHost(slots);
+        slots = nullptr;
+    }
+    static void put(const Piece &p, const char *from) {
+        if (!p.widen) {
+            std::memcpy(p.host, from, p.n);
+            return;
+        }
+        const int32_t *a = reinterpret_cast<const int32_t *>(from);
+        int64_t *b = static_cast<int64_t *>(p.host);
+        for (size_t k = 0; k < p.n; ++k) b[k] = a[k];
+    }
+    void run(const std::vector<Piece> &v) {
+        std::lock_guard<std::mutex> lk(mu);
+        int dev = 0;
+        AXGB_CUDA(cudaGetDevice(&dev));
+        if (!slots) {
+            try {
+                for (auto &q : st) AXGB_CUDA(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
+                void *h = nullptr;
+                AXGB_CUDA(cudaHostAlloc(&h, 2 * kThreads * kPiece, cudaHostAllocDefault));
+                slots = static_cast<char *>(h);
+            } catch (...) {
+                release();
+                throw;
+            }
+        }
+        std::atomic<int> failed{0};
+        auto work = [&](int w) {
+            if (cudaSetDevice(dev) != cudaSuccess) {
+                failed = static_cast<int>(cudaErrorUnknown);
+                return;
+            }
+            char *slot[2] = {slots + 2 * w * kPiece, slots + (2 * w + 1) * kPiece};
+            auto load = [&](size_t i, int q) {
+                return cudaMemcpyAsync(slot[q], v[i].dev, v[i].dev_bytes(), cudaMemcpyDeviceToHost, st[w]);
+            };
+            cudaError_t e = static_cast<size_t>(w) < v.size() ? load(w, 0) : cudaSuccess;
+            int q = 0;
+            for (size_t i = w; i < v.size() && e == cudaSuccess && !failed; i += kThreads, q ^= 1) {
+                e = cudaStreamSynchronize(st[w]);
+                if (e == cudaSuccess && i + kThreads < v.size()) e = load(i + kThreads, q ^ 1);
+                if (e == cudaSuccess) put(v[i], slot[q]);
+            }
+            const cudaError_t f = cudaStreamSynchronize(st[w]);
+            if (e == cudaSuccess) e = f;
+            if (e != cudaSuccess) failed = static_cast<int>(e);
+        };
+        std::vector<std::thread> th;
+        try {
+            for (int w = 1; w < kThreads; ++w) th.emplace_back(work, w);
+        } catch (...) {  // no more threads: this one takes the pieces left
+            for (int w = static_cast<int>(th.size()) + 1; w < kThreads; ++w) work(w);
+        }
+        work(0);
+        for (auto &t : th) t.join();
+        AXGB_CUDA(static_cast<cudaError_t>(failed.load()));
+    }
+};
+
+// Smaller ones keep nothing: some threads take piece after piece, touch its
+// pages and copy straight into the array. Starting a thread costs some 20 to 40 us,
+// so there is one for every 2.5 MiB, and none up to kResident where the arrays'
+// pages are there. By MiB on the device, into memory that was there / fresh
+// memory, in us: one thread without touching; this; eight threads with the ring:
 //   1.5   134 / 958     159 / 250      433 / 419
 //   4.6   252 / 2040    233 / 348      391 / 434
 //   12.2  601 / 7550    428 / 630      592 / 627
 //   24.8  12700         823            664 / 882
-//   76    50700         1438 / 1945    1680 / 2007
-// Pieces of 1 MiB: 1898 / 2545 at 76 MiB (a copy's latency, some 20 us, is not
-// shared by the threads).
 struct Download {
     static constexpr int kThreads = 8;
     static constexpr size_t kPiece = size_t(2) << 20;
     static constexpr size_t kSmall = size_t(1) << 20;     // below: no threads
     static constexpr size_t kResident = size_t(4) << 20;  // below: none if no page has to be made
     static constexpr size_t kPerThread = size_t(5) << 19;
-    struct Piece {
+    static constexpr size_t kRing = size_t(16) << 20;     // from here on: PinnedRing
+    struct Span {
         const void *dev;
         void *host;
-        size_t n;    // elements
-        bool widen;  // int32 on the device, int64 on the host
+        size_t n, size;  // elements, bytes of one on the device
+        bool widen;
     };
-    std::vector<Piece> pieces;
+    std::vector<Span> spans;
     size_t total = 0;  // bytes on the device
 
     // size: bytes of an element on the device
     void add(const void *dev, void *host, i64 n, size_t size, bool widen) {
         if (!host || n <= 0) return;
-        const size_t per = kPiece / size;
-        for (size_t b = 0; b < static_cast<size_t>(n); b += per) {
-            const size_t m = std::min(per, static_cast<size_t>(n) - b);
-            pieces.push_back({static_cast<const char *>(dev) + b * size,
-                              static_cast<char *>(host) + b * size * (widen ? 2 : 1), widen ? m : m * size, widen});
-        }
+        spans.push_back({dev, host, static_cast<size_t>(n), size, widen});
         total += static_cast<size_t>(n) * size;
+    }
+    std::vector<Piece> cut(size_t piece) const {
+        std::vector<Piece> v;
+        for (const Span &s : spans) {
+            const size_t per = piece / s.size;
+            for (size_t b = 0; b < s.n; b += per) {
+                const size_t m = std::min(per, s.n - b);
+                v.push_back({static_cast<const char *>(s.dev) + b * s.size,
+                             static_cast<char *>(s.host) + b * s.size * (s.widen ? 2 : 1), s.widen ? m : m * s.size,
+                             s.widen});
+            }
+        }
+        return v;
     }
 
     // A widened piece is copied into the upper half of its array and widened from
@@ -272,7 +371,7 @@ struct Download {
     }
 
     // The process has the first, middle and last page of every piece's array.
-    bool resident() const {
+    static bool resident(const std::vector<Piece> &pieces) {
         const auto page = static_cast<std::uintptr_t>(sysconf(_SC_PAGESIZE));
         for (const Piece &p : pieces) {
             const auto a = reinterpret_cast<std::uintptr_t>(p.host);
@@ -284,13 +383,18 @@ struct Download {
         }
         return true;
     }
-    int threads() const {
-        if (total <= kSmall || (total <= kResident && resident())) return 1;
+    int threads(const std::vector<Piece> &pieces) const {
+        if (total <= kSmall || (total <= kResident && resident(pieces))) return 1;
         return static_cast<int>(std::clamp<size_t>(1 + total / kPerThread, 2, kThreads));
     }
 
     void run() const {
-        const int used = threads();
+        if (total >= kRing) {
+            PinnedRing::get().run(cut(PinnedRing::kPiece));
+            return;
+        }
+        const std::vector<Piece> pieces = cut(kPiece);
+        const int used = threads(pieces);
         int dev = 0;
         AXGB_CUDA(cudaGetDevice(&dev));
         std::atomic<size_t> next{0};
@@ -321,11 +425,14 @@ struct ScratchPools {
 };
 
 // What the current context's pool keeps goes back to the device (blocks in
-// use stay).
+// use stay), the export's pinned slots to the host.
 void scratch_give_back() {
     unsigned long long id = 0;
     try {
         id = context_id();
+        auto &R = PinnedRing::get();
+        std::lock_guard<std::mutex> lk(R.mu);
+        R.release();
     } catch (const Error &) {
         return;  // no context: nothing is held
     }

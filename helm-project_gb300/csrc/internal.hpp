@@ -98,7 +98,7 @@ struct DBuf {
 };
 
 // What the library keeps per process and device (scratch pool, kernels' shared-
-// memory limits) belongs to a CUDA context and goes with it: cudaDeviceReset ends the context, and the next call makes
+// memory limits, the export's slots) belongs to a CUDA context and goes with it: cudaDeviceReset ends the context, and the next call makes
 // another, at the same address. This is the id of the calling thread's current
 // context, which is never given out twice (about 10 ns).
 unsigned long long context_id();
@@ -293,7 +293,7 @@ struct Segmented {
 struct SplitParams {
     int variant = 1;          // 0 direct gathers, 1 blocked + cp.async chunk staging,
                               // 2 blocked + bulk-copy (TMA) staging, 3 blocked + producer
-                              // warp and mbarrier ring, 4 one fused launch (few fields)
+                              // warp and mbarrier ring, 4 direct with its own tile and fields side by side
     int fields_per_pass = 0;  // direct: RHS tile width; blocked: fields per work item (0 = all)
     int unroll = 4;           // direct: fields per thread iteration; staged: fields per stage
     int stages = 2;           // blocked: staging buffers (variants 1 and 3: 2-3, 2: 2)

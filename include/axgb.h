@@ -27,7 +27,8 @@
  * processes do not); destroying the last handle returns all of it.
  * Conservative generation takes up to 1 GiB of it for its candidate search
  * (64 to 128 bytes a destination cell), besides what it takes for each
- * candidate pair.
+ * candidate pair. CSR exports of 16 MiB and more keep 8 MiB of pinned host
+ * memory in the same way.
  */
 #ifndef AXGB_H
 #define AXGB_H

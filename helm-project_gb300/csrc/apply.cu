@@ -3,13 +3,11 @@
 // batch_apply, libs/axis/include/axis/solver/apply.hpp:275-343).
 //
 // Layout: 32-row sliced ELL built once per matrix from the CSR. One warp
-// owns one slice (one row per lane): it loads its row's entries (column,
-// FP64 weight or FP32 hi+lo pair) once into registers, then streams the
-// fields of its work item through them, so the matrix is read once per
-// item while the gathers of x are the only per-field traffic. Slices are
-// grouped by length class (<=8, <=16, <=32, <=64 entries) so each class
-// runs a kernel with a fixed register array; longer slices take a kernel
-// that re-reads its entries from global memory.
+// owns one slice (one row per lane) and a tile of fields, several of them side
+// by side; it reads the row's entries (column, FP64 weight or FP32 hi+lo pair)
+// a few ahead, and again (from L1) for the tile's next fields. Rows of more
+// than 32 entries are taken by a warp each, from a row-contiguous copy, in the
+// same launch, first in the grid.
 //
 // Split FP32 path: weights w = hi + lo (hi = fp32(w), lo = fp32(w - hi));
 // per entry the product hi*x is split exactly (fma), lo*x is added to the
@@ -17,10 +15,8 @@
 // output is the compensated sum rounded once to FP32. Two fields are
 // processed together with packed f32x2 instructions.
 //
-// Work items are (field tile, slice), tile-major: all warps sweep the same
-// tile of fields at once, so the source values they gather stay in L2
-// between neighbouring slices. The tile width and the number of fields per
-// thread iteration are the tuning knobs (see the autotuner in api.cpp).
+// Tiles come one after another: all warps sweep the same tile of fields at once,
+// so the source values they gather stay in L2 between neighbouring slices.
 #include <algorithm>
 #include <type_traits>
 
@@ -129,7 +125,7 @@ __device__ __forceinline__ float ldg_f(const float *p) { return __ldg(p); }
 // Rows of more than 32 entries (coarse destination cells over a fine source,
 // e.g. polar cells over a lat-lon source): one warp per (row, F fields), lane =
 // leaf of the order in fp32x2.cuh, the F fields carried side by side, entries
-// read row-contiguous (Sell::lcol/lhi/llo), shuffle tree at the end.
+// read row-contiguous (Sell::lcol/lhl), shuffle tree at the end.
 constexpr int kF64F = 4;          // fields an FP64 row carries side by side
 constexpr int kOrdGain = 16;       // twentieths, see rows_by_length
 constexpr int kOrdPlain = static_cast<int>(0x80000000u);  // in Sell::ord: the group gains little
@@ -367,21 +363,9 @@ __device__ __forceinline__ void f64_long_row(const LongRows &L, i64 i, i64 fc, c
 }
 
 // ─── direct split kernel: one launch over the whole matrix ───────────────
-// blockIdx.y: a tile of fields. Warps [0, n_long): a row of more than 32
-// entries (split_long_row; the chunks of F fields shared out over blockIdx.y);
-// the others: lane per row of one slice (of ids, or all), rows of at most 32
-// entries, F fields side by side: K entries' loads, then their gathers, then the compensated steps in
-// entry order (two memory round trips a chunk instead of two an entry). The
-// entries are read again for the tile's next F fields, from L1. Nothing is
-// asked of the fields' alignment. Bound by the latency of its dependent round
-// trips and by instruction issue: it is the kernel for few fields, small
-// matrices (the rule is default_split_params in api.cpp) and unaligned
-// fields. 45 unaligned fields of a 361 x 271 ocean grid -> 1 deg: 30 us, against
-// 184 us for a launch per length class whose warps walked all fields; 7 fields
-// of C192 -> 0.5 deg with hi+lo outputs 16.4 us, against 20 staged.
-// The same for one field. There is too little work in a row to hide its chain
-// of dependent loads (length, entries, source values) behind other warps: the
-// short rows' warps stay and take slice after slice, with the lengths read
+// One field (k_split_fused is the form for several). There is too little work in
+// a row to hide its chain of dependent loads (length, entries, source values)
+// behind other warps: the short rows' warps stay and take slice after slice, with the lengths read
 // two slices ahead and the first kOneK entries one slice ahead, so that only
 // the gathers are waited for. The first blocks take the long rows, a warp
 // each. 0.25 deg -> C384: 16.7 us, against 23 us with a warp a slice.
@@ -473,6 +457,8 @@ __global__ void __launch_bounds__(256, kOneBlocks) k_split_one(SellArgs a, LongR
     }
 }
 
+// A lane's row of at most 32 entries for fields f .. f + nf - 1, F side by side: K
+// entries' loads, then their gathers, then the compensated steps in entry order.
 template <int F, int K, bool ALL>
 __device__ __forceinline__ void short_rows(const SellArgs &a, int n, int e0, i64 row, const float *__restrict__ x,
                                            i64 ldx, float *__restrict__ y, i64 ldy, i64 f, int nf) {
@@ -522,6 +508,17 @@ __device__ __forceinline__ void short_rows(const SellArgs &a, int n, int e0, i64
     }
 }
 
+// blockIdx.y: a tile of fields. Warps [0, n_long): a row of more than 32
+// entries (split_long_row; the chunks of F fields shared out over blockIdx.y);
+// the others: lane per row of one slice (of ids, or all), rows of at most 32
+// entries, F fields side by side (short_rows: two memory round trips for K
+// entries instead of two an entry). The entries are read again for the tile's next F fields, from L1. Nothing is
+// asked of the fields' alignment. Bound by the latency of its dependent round
+// trips and by instruction issue: it is the kernel for few fields, small
+// matrices (the rule is default_split_params in api.cpp) and unaligned
+// fields. 45 unaligned fields of a 361 x 271 ocean grid -> 1 deg: 30 us, against
+// 184 us for a launch per length class whose warps walked all fields; 7 fields
+// of C192 -> 0.5 deg with hi+lo outputs 16.4 us, against 20 staged.
 template <int F, int K>
 __global__ void __launch_bounds__(256, F <= 4 ? 4 : 3) k_split_fused(SellArgs a, LongRows L, int n_long, int n_slices,
                                                                     const float *__restrict__ x, i64 ldx,
@@ -886,8 +883,7 @@ dim3 long_grid(i64 rows, i64 nrhs) {
     return dim3(nblk(rows * 32, 256), static_cast<unsigned>(std::min<i64>(65535, (nrhs + kLongF - 1) / kLongF)));
 }
 
-// Slices of the long classes: their short rows (k_*_rows), then every row
-// of more than 32 entries (k_*_long).
+// Every row of more than 32 entries (the staged applies leave them out).
 void launch_split_long(const Sell &S, const float *x, i64 ldx, float *y, i64 ldy, i64 nrhs, cudaStream_t s,
                        float *ylo = nullptr, i64 ldylo = 0) {
     if (S.n_lrows == 0 || nrhs == 0) return;
@@ -1053,7 +1049,7 @@ struct NanRow {
 // rows_w is one from nine fields up and more with fewer, so that the additions,
 // which cost the same with any number of lanes, have lanes to serve (one
 // field of C384 -> 41 k Voronoi cells, most rows long: 249 -> 42 us; 5
-// fields: 324 -> 187).
+// fields: 324 -> 183).
 // The warps after them: lane per row (Sell::ord), U fields side by side and K
 // entries ahead, loads past a row's end or the last field repeated, not left
 // out (k_f64_fused). blockIdx.y: 16 fields. The long rows come
@@ -1467,7 +1463,8 @@ double *noalloc_scratch() {
 // ROWS: the long-row items, else the slice items, with the row functions of
 // the direct kernel: eight fields side by side in 80 registers, three blocks
 // an SM (17-pair batch 1043 us, against 1096 us with four fields a long row in
-// 64 registers).
+// 64 registers). The long rows' form spills at 80 registers (32 bytes stored, 40
+// loaded a thread).
 constexpr int kBatchTile = 8;  // fields of a slice item
 template <bool ROWS>
 __global__ void __launch_bounds__(256, ROWS ? 3 : 2) k_batch(const Batch::Desc *__restrict__ desc, int n_desc, i64 total,
@@ -1591,7 +1588,7 @@ __global__ void __launch_bounds__(kGatherT) k_gather_desc(const GatherDesc *__re
 }
 
 // Blocks of a gather: the tiles, and so many of the fields side by side that
-// there are about four blocks an SM and a block keeps its indices for several
+// there are about eight blocks an SM and a block keeps its indices for several
 // fields.
 dim3 gather_grid(i64 n, i64 nrhs) {
     const i64 tiles = (n + kGatherTile - 1) / kGatherTile;

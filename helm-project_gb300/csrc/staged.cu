@@ -9,8 +9,8 @@
 //     order; without a hint, 4 consecutive slices;
 //   * rows of more than 32 entries are left out (a warp each, k_split_long);
 //     the block keeps its other rows. (Leaving out a whole block with a long
-//     row sent C384 -> 1 deg, rows of 24 entries and up to 43, to the lane =
-//     field gathers of k_split_rows: a 32-byte sector for every 4-byte value.)
+//     row sent C384 -> 1 deg, rows of 24 entries and up to 43, to gathers with
+//     lane = field: a 32-byte sector for every 4-byte value.)
 //   * inside a block the rows are sorted by entry count (longest first), so
 //     warp w holds rows of similar length and loops only to its own maximum;
 //   * the block's distinct source columns are rounded out to 16-byte chunks;
